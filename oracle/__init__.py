@@ -28,7 +28,7 @@ def build(with_reference: bool | None = None) -> None:
     """Compile the oracle (and the reference bridge when the tree exists)."""
     targets = ["oracle"]
     if with_reference is None:
-        with_reference = REFERENCE_TREE.exists()
+        with_reference = (REFERENCE_TREE / "code").is_dir()  # an empty mount point is no tree
     if with_reference:
         targets.append("ref")
     subprocess.run(["make", "-s", "-C", str(HERE), f"OLAP_REFERENCE_TREE={REFERENCE_TREE}", *targets], check=True)
