@@ -247,6 +247,168 @@ __global__ void __launch_bounds__(kCompactThreads) compact_kernel(const Op op_in
   }
 }
 
+// ---- compaction in two kernels: marks, then expansion ------------------------
+// An op whose evaluation is long or latency-bound (probes), or that streams at
+// full DRAM rate (select), does not wait for its output offsets: a mark kernel
+// writes one bit per item, the selected items' values packed at the start of
+// their mark tile, and each tile's count; expand_kernel then turns the marks
+// into positions.  No look-back, so no block waits for another, and a warp
+// works alone on its tile, so that tiles are sized to give every warp of the
+// device the same number of them (and a short input reaches every SM).  The
+// marks stay in L2 between the two kernels; an input whose marks do not fit
+// the arena runs in chunks, the running total kept on the device.
+constexpr int kExpandThreads = 1024;
+constexpr int kExpandDirect = 256;  // selected items of a step up to which its lanes write their own
+constexpr int kMarkRounds = 4;  // tiles per warp of a mark kernel on a long input
+
+struct Marks {
+  uint32_t* bits;    // bit i % 32 of word i / 32: item i of the chunk is selected
+  uint32_t* counts;  // selected items per mark tile
+  void* vals;        // their values: those of tile t from element t * tile on
+  int64_t n;         // items of the chunk
+  int32_t tile;      // items per mark tile, a multiple of 128
+  int32_t n_tiles;
+};
+
+// Emit: constexpr bool kVals; void emit(int64_t pos, int64_t item, int64_t v)
+// writes item `item` (of the whole input) at output position pos; v is the
+// index of its value in Marks::vals.  A warp takes a run of whole tiles, 1,024
+// items (a word per lane) at a step; only the first sum over the tiles before
+// a block's needs the whole block.  Bound by instructions: where few items of
+// a step are selected, each lane writes its own word's (neighbouring lanes
+// write neighbouring positions, so a store still covers few lines); where
+// many are, they are listed in shared memory first and written from there,
+// one line per store.
+template <class Emit>
+__global__ void __launch_bounds__(kExpandThreads, 2) expand_kernel(const Emit em, const Marks mk, int64_t first_item,
+                                                                   const unsigned long long* __restrict__ run_in,
+                                                                   unsigned long long* __restrict__ run_out,
+                                                                   unsigned long long* __restrict__ total) {
+  constexpr int W = kExpandThreads / 32;
+  extern __shared__ uint16_t s_list[];  // [W][1024]
+  __shared__ unsigned long long s_sum[W];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int per = (mk.n_tiles + gridDim.x * W - 1) / (gridDim.x * W);  // tiles per warp
+  const int b0 = min(static_cast<int>(blockIdx.x) * W * per, mk.n_tiles);
+  unsigned long long s = 0;
+  for (int i = tid; i < (b0 >> 2); i += kExpandThreads) {
+    const uint4 c = __ldg(reinterpret_cast<const uint4*>(mk.counts) + i);
+    s += static_cast<unsigned long long>(c.x) + c.y + c.z + c.w;
+  }
+  if (tid < (b0 & 3)) s += __ldg(mk.counts + (b0 & ~3) + tid);
+  const int t0 = min(b0 + warp * per, mk.n_tiles), t1 = min(t0 + per, mk.n_tiles);
+  s = static_cast<unsigned long long>(warp_sum_i64(static_cast<int64_t>(s)));
+  if (lane == 0) s_sum[warp] = s;
+  __syncthreads();
+  // this warp's first position: every tile before its own
+  s = s_sum[lane] + (run_in && lane == 0 ? *run_in : 0ull);
+  for (int t = b0 + lane; t < t0; t += 32) s += __ldg(mk.counts + t);
+  int64_t base = warp_sum_i64(static_cast<int64_t>(s));
+  uint16_t* list = s_list + warp * 1024;
+  for (int t = t0; t < t1; ++t) {
+    const int64_t tb = static_cast<int64_t>(t) * mk.tile;
+    const int len = static_cast<int>(tb + mk.tile < mk.n ? mk.tile : mk.n - tb);
+    int64_t v = tb;
+    for (int r = 0; r < len; r += 1024) {
+      uint32_t word = r + 32 * lane < len ? __ldg(mk.bits + ((tb + r) >> 5) + lane) : 0u;
+      const uint32_t c = __popc(word);
+      uint32_t inc = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+      }
+      uint32_t at = inc - c;
+      const int all = static_cast<int>(__shfl_sync(0xffffffffu, inc, 31));
+      if (all <= kExpandDirect) {
+        const int64_t i0 = first_item + tb + r + 32 * lane - 1;
+        while (word) {
+          em.emit(base + at, i0 + __ffs(word), Emit::kVals ? v + at : 0);
+          ++at;
+          word &= word - 1;
+        }
+      } else {
+        while (word) {
+          list[at++] = static_cast<uint16_t>(32 * lane + __ffs(word) - 1);
+          word &= word - 1;
+        }
+        __syncwarp();
+        for (int i = lane; i < all; i += 32) em.emit(base + i, first_item + tb + r + list[i], Emit::kVals ? v + i : 0);
+        __syncwarp();
+      }
+      base += all;
+      v += all;
+    }
+  }
+  if (t1 == mk.n_tiles && t0 < t1 && lane == 0) {
+    if (run_out) *run_out = static_cast<unsigned long long>(base);
+    if (total) *total = static_cast<unsigned long long>(base);
+  }
+}
+
+// Items per warp tile for n items on `warps` resident warps: kMarkRounds
+// tiles per warp, the same number for each, down to one step of 128 items.
+inline int64_t mark_tile(int64_t n, int64_t warps) {
+  const int64_t t = (n + kMarkRounds * warps - 1) / (kMarkRounds * warps);
+  return (t + 127) & ~int64_t(127);
+}
+
+// Grid and block of a mark kernel whose warps take tiles in turn: blocks of
+// `threads` while the tiles fill every SM, smaller ones for a short input.
+inline void mark_grid(const olap_ctx* ctx, int64_t n_tiles, int threads, int blocks_per_sm, unsigned* grid,
+                      unsigned* block) {
+  const int64_t cap = static_cast<int64_t>(ctx->sm_count) * blocks_per_sm;
+  int t = threads;
+  while (t > 64 && n_tiles < cap * (t / 32)) t >>= 1;
+  const int64_t g = (n_tiles + t / 32 - 1) / (t / 32);
+  *grid = static_cast<unsigned>(g < cap ? g : cap);
+  *block = static_cast<unsigned>(t);
+}
+
+// Runs mark(marks, first_item, emit) and the expansion over n items with
+// val_bytes per value, in chunks whose marks fit the arena; *total gets the
+// count.  `warps`: resident warps of the mark kernel.
+template <class Emit, class Mark>
+int mark_and_expand(olap_ctx* ctx, Arena& ar, int64_t n, size_t val_bytes, int64_t warps, Emit em,
+                    unsigned long long* total, Mark&& mark) {
+  if (n == 0) {
+    OLAP_CUDA_TRY(ctx, cudaMemsetAsync(total, 0, sizeof(unsigned long long), ctx->stream));
+    return OLAP_OK;
+  }
+  const char* small = "scratch arena too small for the compaction state";
+  unsigned long long* run = ar.take<unsigned long long>(2);
+  uint32_t* counts = ar.take<uint32_t>(static_cast<size_t>(kMarkRounds * warps));
+  if (!run || !counts) return set_error(ctx, OLAP_ERR_CAPACITY, small);
+  // items per chunk: 1/8 byte of marks and val_bytes of values each
+  const int64_t left = static_cast<int64_t>(ar.cap - ar.off) - 1024;
+  int64_t chunk = left > 0 ? left * 8 / (1 + 8 * static_cast<int64_t>(val_bytes)) & ~int64_t(127) : 0;
+  if (chunk < 128) return set_error(ctx, OLAP_ERR_CAPACITY, small);
+  // equal chunks, and tiles addressed by 32 bits
+  const int64_t n_chunks = (n + chunk - 1) / chunk;
+  chunk = ((n + n_chunks - 1) / n_chunks + 127) & ~int64_t(127);
+  Marks mk;
+  mk.bits = ar.take<uint32_t>(static_cast<size_t>(chunk / 32));
+  mk.vals = val_bytes ? ar.take<char>(static_cast<size_t>(chunk) * val_bytes) : nullptr;
+  mk.counts = counts;
+  if (!mk.bits || (val_bytes && !mk.vals)) return set_error(ctx, OLAP_ERR_CAPACITY, small);
+  mk.tile = static_cast<int32_t>(mark_tile(chunk, warps));
+  constexpr int smem = kExpandThreads / 32 * 1024 * static_cast<int>(sizeof(uint16_t));
+  OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(expand_kernel<Emit>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  int which = 0;
+  for (int64_t first = 0; first < n; first += chunk, which ^= 1) {
+    mk.n = chunk < n - first ? chunk : n - first;
+    mk.n_tiles = static_cast<int32_t>((mk.n + mk.tile - 1) / mk.tile);
+    const int rc = mark(mk, first, em);
+    if (rc != OLAP_OK) return rc;
+    const int64_t blocks = (mk.n_tiles + kExpandThreads / 32 - 1) / (kExpandThreads / 32);
+    const int64_t cap = static_cast<int64_t>(ctx->sm_count) * 2;
+    expand_kernel<Emit><<<static_cast<unsigned>(blocks < cap ? blocks : cap), kExpandThreads, smem, ctx->stream>>>(
+        em, mk, first, first ? run + which : nullptr, run + (which ^ 1), first + mk.n == n ? total : nullptr);
+    OLAP_CUDA_TRY(ctx, cudaGetLastError());
+  }
+  return OLAP_OK;
+}
+
 // Host helper: scan-tile state for n_items in tiles of tile_items
 // (compact_tile_items<Op>()) from the arena; zeroes it on the stream.
 inline int make_scan_tiles(olap_ctx* ctx, Arena& ar, int64_t n_items, unsigned long long* total,

@@ -4,89 +4,105 @@
 // every sel_lt_T_* primitive, :28-440; the 3-predicate driver selalgo_rowwise
 // :450-467) and code/project/test_project_option.cpp (pairs (Ra, Rc) of the
 // rows where Ra <= c and Rc <= c, :34-864).  Selection vectors are int32 row
-// ids in ascending order, produced in one pass by the order-preserving
-// compaction of compact.cuh; bitmaps hold bit i of row i at byte i/8, bit
+// ids in ascending order, produced from a bitmap by the mark and expansion
+// kernels of compact.cuh; bitmaps hold bit i of row i at byte i/8, bit
 // i%8 (the storage order of a little-endian std::vector<bool>).
+#include <algorithm>
 #include <cstring>
 
 #include "compact.cuh"
 
 namespace olap {
 
-__device__ __forceinline__ bool cmp_pass(int32_t v, int32_t val, int cmp) {
-  return cmp == OLAP_CMP_LT ? v < val : v <= val;
-}
+// cmp(col, val) as col <= val: col < val is col <= val - 1, and nothing is
+// below INT32_MIN.
+struct LePred {
+  int32_t val;
+  int none;
+  LePred(int32_t v, int cmp) : val(cmp == OLAP_CMP_LT && v != INT32_MIN ? v - 1 : v), none(cmp == OLAP_CMP_LT && v == INT32_MIN) {}
+};
 
 __device__ __forceinline__ int32_t lane4(const int4& v, int k) {
   return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w;
 }
 
-// Items are rows (kRid false) or positions of an input selection vector.
-// The plain column case caches nothing between flags() and emit(), so it
-// takes 16 groups per thread and 4 rounds per tile (256 KB tiles); with row
-// ids, 8 groups and one round.
+// Marks of cmp(col[r], val) over the column (kRid false) or over the rows of an
+// input selection vector; a warp takes whole tiles.  Bound by the column read:
+// full tiles of an aligned column take four 16-byte loads per lane at a time,
+// and two lanes' 4-bit results make one byte of the bitmap (row order, no
+// ballots).  With a selection vector or unaligned, 32 rows at a time, lane =
+// row, one ballot per word.  The predicate is col <= val (the caller turns <
+// into it), none when `none`.  counts may be null (the bitmap alone).
 template <bool kRid>
-struct SelectOp {
-  static constexpr int kGroups = kRid ? 8 : 16;
-  static constexpr int kRounds = kRid ? 1 : 4;  // emit() of a plain column needs nothing cached
-  const int32_t* col;
-  const int32_t* in_rowids;  // optional input selection vector
-  int32_t* out;
-  unsigned long long* range_err;
-  int64_t col_len;
-  int32_t val;
-  int32_t cmp;
-  int32_t vec;               // col (or in_rowids) 16-byte aligned
-  int4 rid[kGroups];  // values (or row ids) of each group, loaded by prefetch()
-
-  __device__ __forceinline__ bool vec_ok() const { return vec != 0; }
-  __device__ __forceinline__ void prefetch(int u, int64_t first) {
-    rid[u] = ld_stream_v4_ordered((kRid ? in_rowids : col) + first, policy_evict_first());
-  }
-  template <bool kFull>
-  __device__ __forceinline__ uint32_t flags(int u, int64_t first, int nv) {
-    const uint64_t pol = policy_evict_first();
-    uint32_t m = 0;
-    if constexpr (!kRid) {
-      if (kFull) {
-        const int4 v = rid[u];
+__global__ void __launch_bounds__(512) select_mark_kernel(const int32_t* __restrict__ col, int64_t col_len,
+                                                          const int32_t* __restrict__ in_rowids, int64_t n,
+                                                          int32_t val, int none, int vec, uint32_t* __restrict__ bits,
+                                                          uint32_t* __restrict__ counts, int32_t tile,
+                                                          int64_t n_tiles, unsigned long long* range_err) {
+  const int lane = threadIdx.x & 31;
+  const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  const uint64_t pol = policy_evict_first();
+  const uint32_t keep = none ? 0u : 15u;
+  unsigned int bad = 0;
+  for (int64_t t = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; t < n_tiles; t += n_warps) {
+    const int64_t first = t * tile;
+    const int64_t end = first + tile < n ? first + tile : n;
+    uint32_t c = 0;
+    if (!kRid && vec && first + tile <= n) {
+      const int32_t* src = col + first + 4 * lane;
+      unsigned char* dst = reinterpret_cast<unsigned char*>(bits) + (first >> 3) + (lane >> 1);
+      auto put = [&](const int4 v, int at) {
+        uint32_t m = static_cast<uint32_t>(v.x <= val) | static_cast<uint32_t>(v.y <= val) << 1 |
+                     static_cast<uint32_t>(v.z <= val) << 2 | static_cast<uint32_t>(v.w <= val) << 3;
+        m &= keep;
+        c += __popc(m);
+        m |= __shfl_down_sync(0xffffffffu, m, 1) << 4;
+        if (!(lane & 1)) dst[at >> 3] = static_cast<unsigned char>(m);
+      };
+      int at = 0;
+      for (; at + 512 <= tile; at += 512) {
+        int4 v[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) m |= static_cast<uint32_t>(cmp_pass(lane4(v, k), val, cmp)) << k;
-      } else if (vec && nv == 4) {
-        const int4 v = ld_stream_v4(col + first, pol);
+        for (int u = 0; u < 4; ++u) v[u] = ld_stream_v4_ordered(src + at + 128 * u, pol);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) m |= static_cast<uint32_t>(cmp_pass(lane4(v, k), val, cmp)) << k;
-      } else {
-        for (int k = 0; k < nv; ++k) m |= static_cast<uint32_t>(cmp_pass(col[first + k], val, cmp)) << k;
+        for (int u = 0; u < 4; ++u) put(v[u], at + 128 * u);
       }
+      for (; at < tile; at += 128) put(ld_stream_v4_ordered(src + at, pol), at);
     } else {
-      int4 r = make_int4(0, 0, 0, 0);
-      if (kFull) {
-        r = rid[u];
-      } else if (vec && nv == 4) {
-        r = ld_stream_v4(in_rowids + first, pol);
-      } else {
-        int32_t t[4] = {0, 0, 0, 0};
-        for (int k = 0; k < nv; ++k) t[k] = in_rowids[first + k];
-        r = make_int4(t[0], t[1], t[2], t[3]);
-      }
-      rid[u] = r;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (k >= nv) continue;
-        const int32_t row = lane4(r, k);
-        if (row < 0 || row >= col_len) {  // not a row of col: dropped and counted
-          atomicAdd(range_err, 1ull);
-          continue;
+      for (int64_t r0 = first; r0 < end; r0 += 32) {
+        const int64_t r = r0 + lane;
+        bool pass = false;
+        if (r < end) {
+          if (kRid) {
+            const int32_t row = __ldg(in_rowids + r);
+            if (row < 0 || row >= col_len) ++bad;  // not a row of col: dropped and counted
+            else pass = __ldg(col + row) <= val && !none;
+          } else {
+            pass = __ldg(col + r) <= val && !none;
+          }
         }
-        m |= static_cast<uint32_t>(cmp_pass(__ldg(col + row), val, cmp)) << k;
+        const uint32_t word = __ballot_sync(0xffffffffu, pass);
+        if (lane == 0) {
+          bits[r0 >> 5] = word;
+          c += __popc(word);
+        }
       }
     }
-    return m;
+    if (counts) {
+      c = __reduce_add_sync(0xffffffffu, c);
+      if (lane == 0) counts[t] = c;
+    }
   }
-  __device__ __forceinline__ void emit(int u, int k, int64_t item, int64_t pos) {
-    if constexpr (kRid) out[pos] = lane4(rid[u], k);
-    else out[pos] = static_cast<int32_t>(item);
+  if (kRid && bad) atomicAdd(range_err, static_cast<unsigned long long>(bad));
+}
+
+// Selected rows: their ids, or the entries of the input selection vector.
+struct SelectEmit {
+  static constexpr bool kVals = false;
+  const int32_t* in_rowids;
+  int32_t* out;
+  __device__ __forceinline__ void emit(int64_t pos, int64_t item, int64_t) const {
+    out[pos] = in_rowids ? __ldg(in_rowids + item) : static_cast<int32_t>(item);
   }
 };
 
@@ -175,22 +191,6 @@ struct ProjectRowsOp {
     out_c[pos] = lane4(c[u], k);
   }
 };
-
-// One 32-bit word of the bitmap per warp step: lane l tests row 32w + l.
-__global__ void select_bitmap_kernel(const int32_t* __restrict__ col, int64_t n, int32_t val, int cmp,
-                                     uint32_t* __restrict__ bits) {
-  const int64_t nwords = (n + 31) >> 5;
-  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const uint64_t pol = policy_evict_first();
-  for (int64_t w = warp; w < nwords; w += nwarps) {
-    const int64_t r = (w << 5) + lane;
-    const bool pass = r < n && cmp_pass(ld_stream_s32_if(r < n, col + r, pol, 0), val, cmp);
-    const uint32_t word = __ballot_sync(0xffffffffu, pass);
-    if (lane == 0) bits[w] = word;
-  }
-}
 
 // SUM(Rd) and COUNT over rows with Ra, Rb, Rc all <= condition.
 __global__ void __launch_bounds__(512) selalgo_kernel(int32_t cond, int64_t n, const int32_t* __restrict__ ra,
@@ -337,25 +337,28 @@ int olap_select_rowids(olap_ctx* ctx, const int32_t* col, int64_t col_len, int32
                "lengths must be in [0, 2^31)");
   OLAP_REQUIRE(ctx, cmp == OLAP_CMP_LE || cmp == OLAP_CMP_LT, "cmp must be OLAP_CMP_LE or OLAP_CMP_LT");
   OLAP_REQUIRE(ctx, n == 0 || (col && out_rowids), "null column or output");
-  auto fill = [&](auto& op) {
-    std::memset(&op, 0, sizeof(op));
-    op.col = col;
-    op.in_rowids = in_rowids;
-    op.out = out_rowids;
-    op.range_err = &ctx->counters->range_errors;
-    op.col_len = col_len;
-    op.val = val;
-    op.cmp = cmp;
-    op.vec = in_rowids ? olap::al16(in_rowids) : olap::al16(col);
-  };
-  if (in_rowids) {
-    olap::SelectOp<true> op;
-    fill(op);
-    return olap::run_compaction(ctx, op, n, d_count);
-  }
-  olap::SelectOp<false> op;
-  fill(op);
-  return olap::run_compaction(ctx, op, n, d_count);
+  olap::Arena ar(ctx);
+  unsigned long long* total = d_count ? reinterpret_cast<unsigned long long*>(d_count)
+                                      : ar.take<unsigned long long>(1);
+  if (!total) return olap::set_error(ctx, OLAP_ERR_CAPACITY, "scratch arena exhausted");
+  const olap::SelectEmit em{in_rowids, out_rowids};
+  const olap::LePred le(val, cmp);
+  return olap::mark_and_expand(
+      ctx, ar, n, 0, ctx->sm_count * int64_t(64), em, total,
+      [&](const olap::Marks& mk, int64_t first, const olap::SelectEmit&) {
+        unsigned grid, block;
+        olap::mark_grid(ctx, mk.n_tiles, 512, 4, &grid, &block);
+        if (in_rowids)
+          olap::select_mark_kernel<true><<<grid, block, 0, ctx->stream>>>(
+              col, col_len, in_rowids + first, mk.n, le.val, le.none, 0, mk.bits, mk.counts, mk.tile, mk.n_tiles,
+              &ctx->counters->range_errors);
+        else
+          olap::select_mark_kernel<false><<<grid, block, 0, ctx->stream>>>(
+              col + first, col_len, nullptr, mk.n, le.val, le.none, olap::al16(col), mk.bits, mk.counts, mk.tile,
+              mk.n_tiles, nullptr);
+        OLAP_CUDA_TRY(ctx, cudaGetLastError());
+        return OLAP_OK;
+      });
 }
 
 int olap_debug_wait_timeout(olap_ctx* ctx, uint32_t spin_limit) {
@@ -383,7 +386,15 @@ int olap_select_bitmap(olap_ctx* ctx, const int32_t* col, int64_t n, int32_t val
   OLAP_REQUIRE(ctx, cmp == OLAP_CMP_LE || cmp == OLAP_CMP_LT, "cmp must be OLAP_CMP_LE or OLAP_CMP_LT");
   if (n == 0) return OLAP_OK;
   OLAP_REQUIRE(ctx, col && bitmap, "null column or bitmap");
-  olap::select_bitmap_kernel<<<olap::stream_grid(ctx, n, 256), 256, 0, ctx->stream>>>(col, n, val, cmp, bitmap);
+  const olap::LePred le(val, cmp);
+  // a bitmap has no tile counts to add up: short tiles, balanced over the warps
+  const int64_t tile = std::min<int64_t>(olap::mark_tile(n, ctx->sm_count * int64_t(64)), 1 << 20);
+  const int64_t n_tiles = (n + tile - 1) / tile;
+  unsigned grid, block;
+  olap::mark_grid(ctx, n_tiles, 512, 4, &grid, &block);
+  olap::select_mark_kernel<false><<<grid, block, 0, ctx->stream>>>(col, n, nullptr, n, le.val, le.none, olap::al16(col),
+                                                                  bitmap, nullptr, static_cast<int32_t>(tile), n_tiles,
+                                                                  nullptr);
   OLAP_CUDA_TRY(ctx, cudaGetLastError());
   return OLAP_OK;
 }
