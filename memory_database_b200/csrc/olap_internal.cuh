@@ -248,6 +248,14 @@ __device__ __forceinline__ int32_t ld_probe_s8_if(bool pred, const int8_t* p, ui
   return v;
 }
 
+// A gathered value whose line holds few others of the gather: on a miss L2
+// fetches 64 bytes of it.  volatile keeps the load inside its guard.
+__device__ __forceinline__ int32_t ld_gather_64(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.global.nc.L2::64B.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
 // Exact 64-bit accumulation into shared memory with 32-bit atomics: the low
 // word is added atomically and its carry-out is forwarded to the high word.
 // Addition mod 2^64 is commutative, so the final pair is exact whatever the

@@ -67,3 +67,21 @@ def test_select_in_chunks(small_ctx):
     d = dev(col)
     for t in (0, 30, 999):
         assert np.array_equal(ops.select_rowids(d, t, ctx=small_ctx).cpu().numpy(), np.flatnonzero(col <= t))
+
+
+@pytest.mark.parametrize("apart", [1, 5, 7, 40])
+@pytest.mark.parametrize("k", [1, 5, 1023, 1025, 70_001])
+def test_gather_densities(ctx, k, apart):
+    """Both gathers (up to 6 rows apart, and farther), ids out of range among them."""
+    from memory_database_b200 import operators as ops
+    rng = np.random.default_rng(k)
+    n = k * apart
+    cols = [rng.integers(-2**31, 2**31, n).astype(np.int32) for _ in range(3)]
+    ids = np.sort(rng.integers(0, n, k)).astype(np.int32)
+    bad = rng.random(k) < 0.1
+    ids[bad] = rng.choice([-1, n, 2**31 - 1], bad.sum())
+    for put in (dev, unaligned):
+        got = ops.gather(put(ids), [dev(c) for c in cols], ctx=ctx)
+        for c, g in zip(cols, got):
+            assert np.array_equal(g.cpu().numpy(), np.where(bad, 0, c[np.where(bad, 0, ids)]))
+        assert ctx.take_range_errors() == bad.sum()
