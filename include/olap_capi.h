@@ -353,8 +353,9 @@ OLAP_API int olap_gather_i32(olap_ctx* ctx, const int32_t* rowids, int64_t k, in
 /* ---- joins (code/join) -------------------------------------------------------
  * Hash table: capacity 64-bit slots (a multiple of 8 in (n, 2^32]; use
  * olap_hashtable_capacity(n), about 2n slots: load <= 1/2), 16-byte
- * aligned, caller-allocated.  A key's home slot is its hash scaled onto the
- * capacity (linear probing from there).  A duplicate build key keeps the payload of its last
+ * aligned, caller-allocated.  A key's home bucket is the aligned four slots
+ * that its hash scaled onto the capacity falls in (linear probing by buckets
+ * from there, the slots of a bucket filled in order).  A duplicate build key keeps the payload of its last
  * row, as the reference's sequential build does.  Key INT32_MIN marks empty
  * slots and cannot be built (counted as a range error). */
 OLAP_API int64_t olap_hashtable_capacity(int64_t n_build);

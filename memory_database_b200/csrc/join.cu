@@ -7,9 +7,9 @@
 // contribute 0.  With duplicate build keys the sequential build keeps the last
 // row's payload; both builds here keep exactly that row.
 //
-// Hash table (a format of this library): 2^k 64-bit slots, open addressing
-// with linear probing over 32-byte buckets of 4 slots (one DRAM sector per
-// probe step).  During the build a slot holds (key << 32 | row) so that a
+// Hash table (a format of this library): 64-bit slots, open addressing with
+// linear probing over 32-byte buckets of 4 slots (one DRAM sector per probe
+// step).  During the build a slot holds (key << 32 | row) so that a
 // duplicate key keeps the largest row with one 64-bit atomicMax; a finishing
 // pass replaces the row by that row's payload, so a probe reads key and
 // payload in one load.  The key INT32_MIN marks an empty slot and cannot be
@@ -21,6 +21,7 @@
 namespace olap {
 
 constexpr uint64_t kEmptySlot = 0x80000000FFFFFFFFull;  // key INT32_MIN, row 0xffffffff
+constexpr uint32_t kEmptyKey = 0x80000000u;              // INT32_MIN, the reserved empty key
 
 __host__ __device__ __forceinline__ uint32_t hash32(uint32_t x) {  // murmur3 finaliser
   x ^= x >> 16;
@@ -33,12 +34,19 @@ __host__ __device__ __forceinline__ uint32_t hash32(uint32_t x) {  // murmur3 fi
 
 // Home slot of key k in a table of `cap` slots: the hash scaled onto
 // [0, cap) by a multiply and shift, so the capacity need not be a power of
-// two (a caller sizes the table to its build side, any multiple of 8).
-// Linear probing moves forward and wraps at the end.
+// two (a caller sizes the table to its build side, any multiple of 8).  A key
+// lies in the bucket of four slots that holds its home slot, else in the next
+// one that had a free slot (linear probing by buckets, wrapping at the end),
+// at the first slot that was free: the slots of a bucket fill in order, so a
+// free last slot ends a run.  Starting at the bucket's first slot instead of
+// the home slot itself, a lookup reads on past its first 32 bytes for 8 % of
+// the absent keys and 3 % of the present ones at load 1/2 (about 25 %
+// before).
 __host__ __device__ __forceinline__ uint64_t home_slot(uint32_t k, uint64_t cap) {
   return (static_cast<uint64_t>(hash32(k)) * cap) >> 32;
 }
-__host__ __device__ __forceinline__ uint64_t next_slot(uint64_t h, uint64_t cap) { return h + 1 == cap ? 0 : h + 1; }
+// The same as a bucket of a table of nb = cap / 4 buckets (at most 2^30).
+__device__ __forceinline__ uint32_t home_bucket(uint32_t k, uint32_t nb) { return __umulhi(hash32(k), nb); }
 
 // Blocked Bloom filter of the build keys (a format of this library, built
 // beside the table): 2^w 64-bit words, about 8 bits per build key; a key sets
@@ -119,8 +127,37 @@ __global__ void fill_u64_kernel(uint64_t* p, int64_t n, uint64_t v) {
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = v;
 }
 
+// Inserts `mine` = (key << 32 | row) into the table of nb buckets from bucket b
+// on; a key already present keeps its largest row.  A bucket of four slots is
+// read at once and only its first slot that is free or holds the key is tried,
+// so a run costs one round trip per bucket instead of one CAS per slot (keys
+// are never removed: a slot read as another key stays that key's).  False when
+// the table has no free slot.
+__device__ __forceinline__ bool insert_from(uint64_t* __restrict__ slots, uint32_t nb, uint32_t b, uint64_t mine) {
+  const uint32_t k = static_cast<uint32_t>(mine >> 32);
+  for (uint32_t step = 0; step < nb; ++step) {
+    uint64_t* q = slots + 4 * static_cast<uint64_t>(b);
+    uint64_t s[4];
+    asm volatile("ld.volatile.global.v2.u64 {%0,%1}, [%2];" : "=l"(s[0]), "=l"(s[1]) : "l"(q) : "memory");
+    asm volatile("ld.volatile.global.v2.u64 {%0,%1}, [%2];" : "=l"(s[2]), "=l"(s[3]) : "l"(q + 2) : "memory");
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+      if (s[j] != kEmptySlot && static_cast<uint32_t>(s[j] >> 32) != k) continue;
+      unsigned long long* at = reinterpret_cast<unsigned long long*>(q + j);
+      const unsigned long long prev = s[j] == kEmptySlot ? atomicCAS(at, kEmptySlot, mine) : s[j];
+      if (prev == kEmptySlot) return true;
+      if (static_cast<uint32_t>(prev >> 32) == k) {
+        atomicMax(at, mine);  // same key in the high word: keeps the largest row
+        return true;
+      }
+    }
+    b = b + 1 == nb ? 0u : b + 1;
+  }
+  return false;
+}
+
 __global__ void hash_build_kernel(const int32_t* __restrict__ keys, int64_t n, uint64_t* __restrict__ slots,
-                                  uint64_t cap, unsigned long long* range_err, unsigned long long* overflow) {
+                                  uint32_t nb, unsigned long long* range_err, unsigned long long* overflow) {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += stride) {
     const int32_t k = keys[r];
@@ -129,21 +166,7 @@ __global__ void hash_build_kernel(const int32_t* __restrict__ keys, int64_t n, u
       continue;
     }
     const uint64_t mine = (static_cast<uint64_t>(static_cast<uint32_t>(k)) << 32) | static_cast<uint32_t>(r);
-    uint64_t h = home_slot(static_cast<uint32_t>(k), cap);
-    bool done = false;
-    for (uint64_t step = 0; step < cap && !done; ++step) {
-      unsigned long long* s = reinterpret_cast<unsigned long long*>(slots + h);
-      const unsigned long long prev = atomicCAS(s, kEmptySlot, mine);
-      if (prev == kEmptySlot) {
-        done = true;
-      } else if ((prev >> 32) == static_cast<uint32_t>(k)) {
-        atomicMax(s, mine);  // same key in the high word: keeps the largest row
-        done = true;
-      } else {
-        h = next_slot(h, cap);
-      }
-    }
-    if (!done) atomicAdd(overflow, 1ull);
+    if (!insert_from(slots, nb, home_bucket(static_cast<uint32_t>(k), nb), mine)) atomicAdd(overflow, 1ull);
   }
 }
 
@@ -313,36 +336,17 @@ __global__ void __launch_bounds__(kBuildPartThreads) build_scatter_kernel(BuildP
   }
 }
 
-// Inserts `mine` = (key << 32 | row) into the table from slot h on (linear
-// probing); a key already present keeps its largest row.  False when the
-// table has no free slot.
-__device__ __forceinline__ bool insert_from(uint64_t* __restrict__ slots, uint64_t cap, uint64_t h,
-                                            uint64_t mine) {
-  const uint32_t k = static_cast<uint32_t>(mine >> 32);
-  for (uint64_t step = 0; step < cap; ++step) {
-    unsigned long long* s = reinterpret_cast<unsigned long long*>(slots + h);
-    const unsigned long long prev = atomicCAS(s, kEmptySlot, mine);
-    if (prev == kEmptySlot) return true;
-    if ((prev >> 32) == k) {
-      atomicMax(s, mine);  // same key in the high word: keeps the largest row
-      return true;
-    }
-    h = next_slot(h, cap);
-  }
-  return false;
-}
-
 // Inserts region p's rows (tuples [region_begin[p], region_begin[p+1])): the
 // region's 32 MB of slots are read from DRAM once, and every later CAS on
 // them is an L2 round trip.
 __global__ void build_insert_kernel(const uint64_t* __restrict__ tuples, const long long* __restrict__ region_begin,
-                                    int p, uint64_t* __restrict__ slots, uint64_t cap,
+                                    int p, uint64_t* __restrict__ slots, uint32_t nb,
                                     unsigned long long* overflow) {
   const int64_t b = region_begin[p], e = region_begin[p + 1];
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = b + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < e; i += stride) {
     const uint64_t mine = tuples[i];
-    if (!insert_from(slots, cap, home_slot(static_cast<uint32_t>(mine >> 32), cap), mine)) atomicAdd(overflow, 1ull);
+    if (!insert_from(slots, nb, home_bucket(static_cast<uint32_t>(mine >> 32), nb), mine)) atomicAdd(overflow, 1ull);
   }
 }
 
@@ -587,7 +591,6 @@ __global__ void __launch_bounds__(kSmemRegionThreads, 1) smem_region_scatter_ker
 // high halves apart, for 32-bit atomics) and stored whole; the run's first
 // and last words may be shared with the neighbouring regions and are ORed
 // into the (zeroed) filter instead.
-constexpr uint32_t kEmptyKey = 0x80000000u;  // INT32_MIN, the reserved empty key
 constexpr int kSmemFilterWords = 2064;  // a region's run with olap_hashjoin_filter_words is at most 2050
 
 __global__ void __launch_bounds__(kSmemRegionThreads, 1) smem_region_build_kernel(
@@ -641,7 +644,7 @@ __global__ void __launch_bounds__(kSmemRegionThreads, 1) smem_region_build_kerne
         if (bits >> 32) atomicOr(&s_fhi[w], static_cast<uint32_t>(bits >> 32));
       }
       bool done = false;
-      for (uint32_t j = __umulhi(h, cap32) - base; j < len; ++j) {
+      for (uint32_t j = (__umulhi(h, cap32) - base) & ~3u; j < len; ++j) {
         const uint32_t prev = atomicCAS(&s_key[j], kEmptyKey, k);
         if (prev == kEmptyKey) {
           atomicMax(&s_row[j], row);
@@ -664,7 +667,7 @@ __global__ void __launch_bounds__(kSmemRegionThreads, 1) smem_region_build_kerne
     for (int64_t t = b + threadIdx.x; t < e; t += blockDim.x) {
       const uint64_t mine = tuples[t];
       const uint32_t k = static_cast<uint32_t>(mine >> 32), row = static_cast<uint32_t>(mine);
-      for (uint32_t j = home32(k, cap32) - base; j < len; ++j) {
+      for (uint32_t j = (home32(k, cap32) - base) & ~3u; j < len; ++j) {
         if (s_key[j] != k) continue;
         if (s_row[j] == row) s_val[j] = pays[t];
         break;
@@ -755,106 +758,75 @@ __global__ void smem_region_taken_kernel(const uint64_t* __restrict__ taken, con
   }
 }
 
-// Half a bucket (two slots) of the hash table, marked evict-last in L2: every
-// probe re-reads the table at random while the probe keys stream past it once,
-// so the part of the table that L2 holds should stay there.  The 64-byte
-// prefetch size asks L2 to fetch only the 64 bytes around the bucket on a
-// miss: 36 instead of 57 bytes of DRAM per probe (2^24 probes, 256 MB
-// table), for about 5 % more time per probe.  The address is always inside
-// the table (the callers' guards may be moved past this load).
-__device__ __forceinline__ ulonglong2 ld_bucket_half(const uint64_t* p) {
-  ulonglong2 v;
-  asm("ld.global.nc.L2::cache_hint.L2::64B.v2.u64 {%0,%1}, [%2], %3;"
-      : "=l"(v.x), "=l"(v.y)
-      : "l"(p), "l"(policy_evict_last()));
-  return v;
-}
-
-// Probe: SUM of matched payloads and the match count; optionally the matches
-// (probe row, payload) compacted in probe-row order by the caller's second
-// pass (see ProbeOp).
-__device__ __forceinline__ bool hash_lookup_from(const uint64_t* __restrict__ slots, uint64_t cap, uint64_t h,
-                                                 uint32_t uk, int32_t* payload) {
-  for (uint64_t step = 0; step < cap; step += 4) {
-    // the 4-slot bucket holding h (one 32-byte sector), starting at h
-    const uint64_t b = h & ~3ull;
-    const ulonglong2 lo = ld_bucket_half(slots + b);
-    const ulonglong2 hi = ld_bucket_half(slots + b + 2);
-    const uint64_t s[4] = {lo.x, lo.y, hi.x, hi.y};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (j < static_cast<int>(h & 3)) continue;  // linear probing starts at h
-      if (s[j] == kEmptySlot) return false;
-      if ((s[j] >> 32) == uk) {
-        *payload = static_cast<int32_t>(static_cast<uint32_t>(s[j]));
-        return true;
-      }
-    }
-    h = b + 4 == cap ? 0 : b + 4;
+// A bucket (four slots, 32 bytes) of the hash table, marked evict-last in L2:
+// every probe re-reads the table at random while the probe keys stream past
+// it once, so the part of the table that L2 holds should stay there.  The
+// 64-byte prefetch size asks L2 to fetch only the 64 bytes around the bucket
+// on a miss: 36 instead of 57 bytes of DRAM per probe (2^24 probes, 256 MB
+// table), for about 5 % more time per probe.  kWide: one 32-byte load (the
+// table is 32-byte aligned); a random load costs L1 a cycle per lane, so two
+// 16-byte ones cost twice that.  The address is always inside the table (the
+// callers' guards may be moved past this load).
+template <bool kWide>
+__device__ __forceinline__ void ld_bucket(const uint64_t* p, uint64_t (&s)[4]) {
+  if (kWide) {
+    asm("ld.global.nc.L2::cache_hint.L2::64B.v4.u64 {%0,%1,%2,%3}, [%4], %5;"
+        : "=l"(s[0]), "=l"(s[1]), "=l"(s[2]), "=l"(s[3])
+        : "l"(p), "l"(policy_evict_last()));
+  } else {
+    asm("ld.global.nc.L2::cache_hint.L2::64B.v2.u64 {%0,%1}, [%2], %3;"
+        : "=l"(s[0]), "=l"(s[1])
+        : "l"(p), "l"(policy_evict_last()));
+    asm("ld.global.nc.L2::cache_hint.L2::64B.v2.u64 {%0,%1}, [%2], %3;"
+        : "=l"(s[2]), "=l"(s[3])
+        : "l"(p + 2), "l"(policy_evict_last()));
   }
-  return false;
 }
 
-__device__ __forceinline__ bool hash_lookup(const uint64_t* __restrict__ slots, uint64_t cap, int32_t k,
-                                            int32_t* payload) {
-  return hash_lookup_from(slots, cap, home_slot(static_cast<uint32_t>(k), cap), static_cast<uint32_t>(k), payload);
-}
-
-// Four lookups with their first buckets read together (8 x 16-byte loads in
-// flight) before any is resolved; a key whose run continues past its first
-// bucket (rare at load <= 1/2) falls back to hash_lookup from the next one.
-// Returns the 4-bit mask of matches; pay[j] holds the matched payloads.
-// Only the keys in `want` are looked up (the others count as absent).
-__device__ __forceinline__ uint32_t hash_lookup4(const uint64_t* __restrict__ slots, uint64_t cap, const int4 k4,
-                                                 int32_t pay[4], uint32_t want = 0xFu) {
-  const int32_t k[4] = {k4.x, k4.y, k4.z, k4.w};
-  uint64_t h[4];
-  ulonglong2 lo[4], hi[4];
-  const ulonglong2 none = make_ulonglong2(kEmptySlot, kEmptySlot);
+// Up to four lookups, the buckets of each round read together before any is
+// resolved; a key whose bucket is full of other keys goes on to the next one in
+// the next round.  Returns the 4-bit mask of matches; pay[j] holds the matched
+// payloads, 0 elsewhere.  Only the keys in `want` are looked up (the others
+// count as absent).
+template <bool kWide>
+__device__ __forceinline__ uint32_t hash_lookup4(const uint64_t* __restrict__ slots, uint32_t nb, const int4 k4,
+                                                 int32_t pay[4], uint32_t want) {
+  const uint32_t k[4] = {static_cast<uint32_t>(k4.x), static_cast<uint32_t>(k4.y), static_cast<uint32_t>(k4.z),
+                         static_cast<uint32_t>(k4.w)};
+  uint32_t b[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    h[j] = home_slot(static_cast<uint32_t>(k[j]), cap);
-    const uint64_t b = h[j] & ~3ull;
-    const bool w = (want >> j) & 1u;
-    lo[j] = w ? ld_bucket_half(slots + b) : none;
-    hi[j] = w ? ld_bucket_half(slots + b + 2) : none;
+    b[j] = home_bucket(k[j], nb);
+    pay[j] = 0;
+    if (k[j] == kEmptyKey) want &= ~(1u << j);  // marks the free slots: never in the table
   }
   uint32_t found = 0;
+  for (uint32_t step = 0; want && step < nb; ++step) {
+    uint64_t s[4][4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint64_t s[4] = {lo[j].x, lo[j].y, hi[j].x, hi[j].y};
-    const uint32_t uk = static_cast<uint32_t>(k[j]);
-    int state = ((want >> j) & 1u) ? 0 : 2;  // 0 go on, 1 found, 2 absent
-    pay[j] = 0;
+    for (int j = 0; j < 4; ++j)
+      if ((want >> j) & 1u) ld_bucket<kWide>(slots + 4 * static_cast<uint64_t>(b[j]), s[j]);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (state != 0 || q < static_cast<int>(h[j] & 3)) continue;
-      if (s[q] == kEmptySlot) {
-        state = 2;
-      } else if ((s[q] >> 32) == uk) {
-        pay[j] = static_cast<int32_t>(static_cast<uint32_t>(s[q]));
-        state = 1;
-      }
+    for (int j = 0; j < 4; ++j) {
+      if (!((want >> j) & 1u)) continue;
+      bool eq = false;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (static_cast<uint32_t>(s[j][q] >> 32) == k[j]) {
+          eq = true;
+          pay[j] = static_cast<int32_t>(static_cast<uint32_t>(s[j][q]));
+        }
+      if (eq) found |= 1u << j;
+      if (eq || static_cast<uint32_t>(s[j][3] >> 32) == kEmptyKey) want &= ~(1u << j);
+      b[j] = b[j] + 1 == nb ? 0u : b[j] + 1;
     }
-    if (state == 0) {
-      int32_t p = 0;
-      const uint64_t b4 = (h[j] & ~3ull) + 4;
-      const uint64_t next = b4 == cap ? 0 : b4;
-      // continue the run from the next bucket: a key whose home slot is
-      // `next` has the same probe sequence from there on
-      if (hash_lookup_from(slots, cap, next, uk, &p)) {
-        pay[j] = p;
-        state = 1;
-      }
-    }
-    if (state == 1) found |= 1u << j;
   }
   return found;
 }
 
-template <bool kFilter>
+template <bool kFilter, bool kWide>
 __global__ void __launch_bounds__(512, 2) hash_probe_sum_kernel(const int32_t* __restrict__ keys, int64_t n,
-                                                                const uint64_t* __restrict__ slots, uint64_t cap,
+                                                                const uint64_t* __restrict__ slots, uint32_t nb,
                                                                 Bloom filter, int vec, unsigned long long* sum,
                                                                 unsigned long long* matches) {
   __shared__ long long s_red[16][2];
@@ -867,16 +839,15 @@ __global__ void __launch_bounds__(512, 2) hash_probe_sum_kernel(const int32_t* _
   for (int64_t i = tid; i < n4; i += stride) {
     const int4 k = ld_stream_v4(keys + 4 * i, pol);
     int32_t p[4];
-    const uint32_t f = hash_lookup4(slots, cap, k, p, bloom_pass4<kFilter>(filter, k, keep));
+    const uint32_t f = hash_lookup4<kWide>(slots, nb, k, p, bloom_pass4<kFilter>(filter, k, keep));
     s += static_cast<int64_t>(p[0]) + p[1] + static_cast<int64_t>(p[2]) + p[3];  // 0 where absent
     c += __popc(f);
   }
   for (int64_t r = 4 * n4 + tid; r < n; r += stride) {
-    int32_t p = 0;
-    if (bloom_pass<kFilter>(filter, keys[r]) && hash_lookup(slots, cap, keys[r], &p)) {
-      s += p;
-      ++c;
-    }
+    int32_t p[4];
+    if (!bloom_pass<kFilter>(filter, keys[r])) continue;
+    c += hash_lookup4<kWide>(slots, nb, make_int4(keys[r], 0, 0, 0), p, 1u);
+    s += p[0];
   }
   s = warp_sum_i64(s);
   c = warp_sum_i64(c);
@@ -898,50 +869,58 @@ __global__ void __launch_bounds__(512, 2) hash_probe_sum_kernel(const int32_t* _
   }
 }
 
-// Matches (probe row, payload) in probe-row order.
-template <bool kFilter>
-struct ProbeOp {
-  static constexpr int kGroups = kCompactGroups;
-  const int32_t* keys;
-  const uint64_t* slots;
-  uint64_t cap;
-  Bloom filter;
+// Marks of the probe rows that match, with their payloads (compact.cuh): a
+// warp takes whole tiles, 128 rows at a step, lane l the rows 32 u + l, so a
+// ballot is a word of the bitmap and the payloads of a step go out as one
+// run.  Bound by the latency of the bucket reads: the four lookups of a lane
+// are in flight together, and 32 warps of 64 registers fit an SM.
+template <bool kFilter, bool kWide>
+__global__ void __launch_bounds__(512, 2) hash_probe_mark_kernel(const int32_t* __restrict__ keys,
+                                                                 const uint64_t* __restrict__ slots, uint32_t nb,
+                                                                 Bloom filter, Marks mk) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint64_t pol = policy_evict_first();
+  const uint64_t keep = policy_evict_last();
+  const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t t = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; t < mk.n_tiles; t += n_warps) {
+    const int64_t first = t * mk.tile;
+    const int64_t end = first + mk.tile < mk.n ? first + mk.tile : mk.n;
+    int32_t* vals = static_cast<int32_t*>(mk.vals) + first;
+    uint32_t c = 0;
+    for (int64_t r0 = first; r0 < end; r0 += 128) {
+      int32_t k[4], p[4];
+      uint32_t in = 0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool ok = r0 + 32 * u + lane < end;
+        in |= static_cast<uint32_t>(ok) << u;
+        k[u] = ld_stream_s32_if(ok, keys + r0 + 32 * u + lane, pol, 0);
+      }
+      const int4 k4 = make_int4(k[0], k[1], k[2], k[3]);
+      const uint32_t m = hash_lookup4<kWide>(slots, nb, k4, p, in & bloom_pass4<kFilter>(filter, k4, keep));
+      uint32_t w[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        w[u] = __ballot_sync(0xffffffffu, (m >> u) & 1u);
+        if ((m >> u) & 1u) vals[c + __popc(w[u] & lt)] = p[u];
+        c += __popc(w[u]);
+      }
+      // the chunk's bitmap holds whole 128-item steps
+      if (lane == 0) reinterpret_cast<uint4*>(mk.bits)[r0 >> 7] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    if (lane == 0) mk.counts[t] = c;
+  }
+}
+
+struct ProbeEmit {
+  static constexpr bool kVals = true;
+  const int32_t* vals;
   int32_t* out_rows;
   int32_t* out_payload;
-  int32_t vec;
-  int4 pay[kCompactGroups];
-
-  __device__ __forceinline__ bool vec_ok() const { return vec != 0; }
-  __device__ __forceinline__ void prefetch(int u, int64_t first) {
-    pay[u] = ld_stream_v4_ordered(keys + first, policy_evict_first());  // the keys, until flags() replaces them
-  }
-  template <bool kFull>
-  __device__ __forceinline__ uint32_t flags(int u, int64_t first, int nv) {
-    int32_t k[4] = {0, 0, 0, 0};
-    if (kFull) {
-      k[0] = pay[u].x; k[1] = pay[u].y; k[2] = pay[u].z; k[3] = pay[u].w;
-    } else if (vec && nv == 4) {
-      const int4 v = ld_stream_v4(keys + first, policy_evict_first());
-      k[0] = v.x; k[1] = v.y; k[2] = v.z; k[3] = v.w;
-    } else {
-      for (int j = 0; j < nv; ++j) k[j] = keys[first + j];
-    }
-    int32_t p[4] = {0, 0, 0, 0};
-    uint32_t m = 0;
-    if (nv == 4) {
-      const int4 k4 = make_int4(k[0], k[1], k[2], k[3]);
-      m = hash_lookup4(slots, cap, k4, p, bloom_pass4<kFilter>(filter, k4, policy_evict_last()));
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (j < nv && bloom_pass<kFilter>(filter, k[j]) && hash_lookup(slots, cap, k[j], &p[j])) m |= 1u << j;
-    }
-    pay[u] = make_int4(p[0], p[1], p[2], p[3]);
-    return m;
-  }
-  __device__ __forceinline__ void emit(int u, int k, int64_t item, int64_t pos) {
+  __device__ __forceinline__ void emit(int64_t pos, int64_t item, int64_t v) const {
     out_rows[pos] = static_cast<int32_t>(item);
-    out_payload[pos] = k == 0 ? pay[u].x : k == 1 ? pay[u].y : k == 2 ? pay[u].z : pay[u].w;
+    out_payload[pos] = __ldg(vals + v);
   }
 };
 
@@ -1009,33 +988,51 @@ __global__ void __launch_bounds__(512) vec_probe_kernel(const int32_t* __restric
 
 static bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// Matched pairs of n probe keys through the order-preserving compaction.
-template <bool kFilter>
-int probe_pairs(olap_ctx* ctx, Arena& ar, const uint64_t* table, uint64_t cap, const Bloom& bloom,
-                const int32_t* keys, int64_t n, unsigned long long* total, int32_t* out_rows,
-                int32_t* out_payload) {
-  ProbeOp<kFilter> op;
-  std::memset(&op, 0, sizeof(op));
-  op.keys = keys;
-  op.slots = table;
-  op.cap = cap;
-  op.filter = bloom;
-  op.out_rows = out_rows;
-  op.out_payload = out_payload;
-  op.vec = al16(keys);
-  ScanTiles st;
-  const int rc = make_scan_tiles(ctx, ar, n, total, ctx->stream, &st, compact_tile_items<ProbeOp<kFilter>>());
-  if (rc != OLAP_OK) return rc;
-  compact_kernel<ProbeOp<kFilter>><<<compact_grid(ctx, st.n_tiles), kCompactThreads, 0, ctx->stream>>>(op, n, st);
-  OLAP_CUDA_TRY(ctx, cudaGetLastError());
-  return OLAP_OK;
-}
-
 static unsigned grid_for(const olap_ctx* ctx, int64_t items, int threads) {
   int64_t g = (items + threads - 1) / threads;
   const int64_t cap = static_cast<int64_t>(ctx->sm_count) * (2048 / threads);
   if (g > cap) g = cap;
   return static_cast<unsigned>(g < 1 ? 1 : g);
+}
+
+// The probe of n keys: with out_rows the matched pairs in probe-row order and
+// their number in *total, else the sum and the match count.
+template <bool kFilter, bool kWide>
+int launch_hash_probe(olap_ctx* ctx, Arena& ar, const uint64_t* table, uint32_t nb, const Bloom& bloom,
+                      const int32_t* keys, int64_t n, unsigned long long* sum, unsigned long long* total,
+                      int32_t* out_rows, int32_t* out_payload) {
+  if (!out_rows) {
+    hash_probe_sum_kernel<kFilter, kWide><<<grid_for(ctx, (n + 3) / 4, 512), 512, 0, ctx->stream>>>(
+        keys, n, table, nb, bloom, al16(keys), sum, total);
+    OLAP_CUDA_TRY(ctx, cudaGetLastError());
+    return OLAP_OK;
+  }
+  const ProbeEmit em{nullptr, out_rows, out_payload};
+  return mark_and_expand(ctx, ar, n, sizeof(int32_t), ctx->sm_count * int64_t(32), em, total,
+                         [&](const Marks& mk, int64_t first, ProbeEmit& e) {
+                           e.vals = static_cast<const int32_t*>(mk.vals);
+                           unsigned grid, block;
+                           mark_grid(ctx, mk.n_tiles, 512, 2, &grid, &block);
+                           hash_probe_mark_kernel<kFilter, kWide><<<grid, block, 0, ctx->stream>>>(
+                               keys + first, table, nb, bloom, mk);
+                           OLAP_CUDA_TRY(ctx, cudaGetLastError());
+                           return OLAP_OK;
+                         });
+}
+
+// A probe through the filter reads a filter word for every key and a bucket
+// only for the keys that pass; while L2 holds the table both cost the same,
+// and the filter's read is saved by not using it.
+constexpr int64_t kProbeFilterSlots = int64_t(1) << 22;  // 32 MB
+
+static int hash_probe(olap_ctx* ctx, Arena& ar, const uint64_t* table, uint64_t cap, const Bloom& bloom,
+                      const int32_t* keys, int64_t n, unsigned long long* sum, unsigned long long* total,
+                      int32_t* out_rows, int32_t* out_payload) {
+  const bool filter = bloom.words && static_cast<int64_t>(cap) > kProbeFilterSlots;
+  const bool wide = (reinterpret_cast<uintptr_t>(table) & 31) == 0;
+  auto* f = filter ? (wide ? launch_hash_probe<true, true> : launch_hash_probe<true, false>)
+                   : (wide ? launch_hash_probe<false, true> : launch_hash_probe<false, false>);
+  return f(ctx, ar, table, static_cast<uint32_t>(cap >> 2), bloom, keys, n, sum, total, out_rows, out_payload);
 }
 
 // Plan of the region passes over a table of `capacity` slots for n rows.
@@ -1180,7 +1177,7 @@ int hashjoin_build_locked(olap_ctx* ctx, const int32_t* keys, const int32_t* pay
                                                                                           tuples);
     const unsigned ig = static_cast<unsigned>(ctx->sm_count) * 8;
     for (int p = 0; p < bp.n_regions; ++p)
-      olap::build_insert_kernel<<<ig, 256, 0, ctx->stream>>>(tuples, rbegin, p, table, bp.cap, overflow);
+      olap::build_insert_kernel<<<ig, 256, 0, ctx->stream>>>(tuples, rbegin, p, table, static_cast<uint32_t>(bp.cap >> 2), overflow);
     olap::hash_finish_kernel<<<olap::grid_for(ctx, capacity, 256), 256, 0, ctx->stream>>>(table, capacity, payload);
   } else {
     olap::fill_u64_kernel<<<olap::grid_for(ctx, capacity, 256), 256, 0, ctx->stream>>>(table, capacity,
@@ -1188,7 +1185,7 @@ int hashjoin_build_locked(olap_ctx* ctx, const int32_t* keys, const int32_t* pay
   }
   if (n && !smem_regions && !partitioned) {
     olap::hash_build_kernel<<<olap::grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(
-        keys, n, table, static_cast<uint64_t>(capacity), &ctx->counters->range_errors, overflow);
+        keys, n, table, static_cast<uint32_t>(capacity >> 2), &ctx->counters->range_errors, overflow);
     olap::hash_finish_kernel<<<olap::grid_for(ctx, capacity, 256), 256, 0, ctx->stream>>>(table, capacity, payload);
   }
   if (filter && !fused_filter && n)
@@ -1278,26 +1275,17 @@ int olap_hashjoin_probe_filtered(olap_ctx* ctx, const uint64_t* table, int64_t c
     if (!m) return olap::set_error(ctx, OLAP_ERR_CAPACITY, "scratch arena exhausted");
     OLAP_CUDA_TRY(ctx, cudaMemsetAsync(d_sum, 0, sizeof(int64_t), ctx->stream));
     OLAP_CUDA_TRY(ctx, cudaMemsetAsync(m, 0, sizeof(int64_t), ctx->stream));
-    auto* ds = reinterpret_cast<unsigned long long*>(d_sum);
     if (n) {
-      const dim3 grid(olap::grid_for(ctx, (n + 3) / 4, 512));
-      if (filter)
-        olap::hash_probe_sum_kernel<true><<<grid, 512, 0, ctx->stream>>>(keys, n, table, cap, bloom,
-                                                                        olap::al16(keys), ds, m);
-      else
-        olap::hash_probe_sum_kernel<false><<<grid, 512, 0, ctx->stream>>>(keys, n, table, cap, bloom,
-                                                                         olap::al16(keys), ds, m);
+      const int rc = olap::hash_probe(ctx, ar, table, cap, bloom, keys, n, reinterpret_cast<unsigned long long*>(d_sum),
+                                      m, nullptr, nullptr);
+      if (rc != OLAP_OK) return rc;
     }
-    OLAP_CUDA_TRY(ctx, cudaGetLastError());
   }
   if (out_rows && out_payload) {
     unsigned long long* total = (!d_sum && d_matches) ? reinterpret_cast<unsigned long long*>(d_matches)
                                                       : ar.take<unsigned long long>(1);
     if (!total) return olap::set_error(ctx, OLAP_ERR_CAPACITY, "scratch arena exhausted");
-    const int rc = filter ? olap::probe_pairs<true>(ctx, ar, table, cap, bloom, keys, n, total, out_rows, out_payload)
-                          : olap::probe_pairs<false>(ctx, ar, table, cap, bloom, keys, n, total, out_rows,
-                                                     out_payload);
-    if (rc != OLAP_OK) return rc;
+    return olap::hash_probe(ctx, ar, table, cap, bloom, keys, n, nullptr, total, out_rows, out_payload);
   }
   return OLAP_OK;
 }
