@@ -16,8 +16,9 @@
 // every distinct key fits one table, else per partition of the key hash
 // (see the plans below).
 #include <algorithm>
-#include <vector>
 #include <cstring>
+#include <type_traits>
+#include <vector>
 
 #include "compact.cuh"
 
@@ -129,33 +130,49 @@ __device__ __forceinline__ void global_add(const HashAgg& t, int32_t k, uint64_t
 //    least `capacity` slots, so each distinct key stays in shared memory; blocks
 //    flush their tables into the global table once, and the occupied slots
 //    are compacted into the outputs.  One read of the columns.
-//  * larger: the rows are partitioned by high bits of the key hash into P
-//    partitions of at most capacity / (2P) <= kAggSlots / 2 distinct keys (a
-//    histogram pass, a scan of the partition offsets, a scatter pass), then
-//    one block per partition aggregates it in a kAggSlots-slot shared table
-//    and writes its groups straight to the outputs.
+//  * larger: the rows are partitioned by the key hash into P partitions, whole
+//    waves of one block per SM, with so few distinct keys each that they fill
+//    at most about a quarter of a shared table (a histogram pass, a scan of
+//    the partition offsets, a scatter pass); then one block per partition
+//    aggregates it in a shared table of 8,192 or 14,336 slots and writes its
+//    groups straight to the outputs.
 // Optionally (OLAP_TUNE_GROUP_COMBINE) a warp first combines its rows that
 // share a key (match_any plus two 32-bit reductions of the split values), so
 // each distinct key of a warp costs one shared-table update.
 
 constexpr int kAggThreads = 1024;
 constexpr int kAggSlots = 8192;  // 16 B per slot: 128 KB of shared memory
+constexpr int kAggMaxSlots = 14336;  // 224 KB: the partitions' tables of many groups
 
 struct SmemAgg {
   int32_t* key;
   unsigned int* cnt;
-  uint32_t* lo;     // low words of the 64-bit sums; the high words follow at lo + slots
+  uint32_t* lo;     // low words of the 64-bit sums (signed); the high words follow at lo + slots
   uint32_t slots;   // a multiple of 4
   uint32_t nb;      // buckets of 4 slots (any count, so a table can fill the shared memory)
 
   // Home bucket of key k: the low 16 hash bits scaled to [0, nb) (plan 2's
   // partitions take the high bits); probing wraps after the last bucket.
   __device__ __forceinline__ uint32_t home(int32_t k) const {
-    return ((mix32(static_cast<uint32_t>(k)) & 0xFFFFu) * nb) >> 16;
+    return __umulhi(mix32(static_cast<uint32_t>(k)) << 16, nb);
   }
   __device__ __forceinline__ uint32_t next(uint32_t b) const { return b + 1 == nb ? 0u : b + 1; }
-  __device__ __forceinline__ uint64_t sum(uint32_t i) const { return smem_split_get(lo, slots, i); }
+  __device__ __forceinline__ uint64_t sum(uint32_t i) const {
+    return (static_cast<uint64_t>(lo[slots + i]) << 32) + static_cast<uint64_t>(static_cast<int64_t>(static_cast<int32_t>(lo[i])));
+  }
 };
+
+// What adding v to a slot's signed low word adds to its high word: v's own
+// high part, and one for a signed overflow of the low word (rare, so values of
+// both signs seldom touch the high word).
+__device__ __forceinline__ int32_t agg_high(uint32_t old, int32_t v) {
+  const int32_t o = static_cast<int32_t>(old), r = static_cast<int32_t>(old + static_cast<uint32_t>(v));
+  return ((o ^ r) & (v ^ r)) < 0 ? (v < 0 ? -1 : 1) : 0;
+}
+__device__ __forceinline__ int32_t agg_high(uint32_t old, int64_t v) {
+  const int32_t l = static_cast<int32_t>(v);
+  return static_cast<int32_t>((v - l) >> 32) + agg_high(old, l);
+}
 
 __device__ __forceinline__ SmemAgg smem_agg(unsigned char* base, uint32_t slots) {
   SmemAgg t;
@@ -196,9 +213,14 @@ __device__ __forceinline__ int smem_find_insert(const SmemAgg& t, int32_t k, uin
     const int4 q = lds_volatile_v4(t.key + 4 * b);
     int slot = q.x == k ? 0 : q.y == k ? 1 : q.z == k ? 2 : q.w == k ? 3 : -1;
     if (slot < 0 && (q.x == kEmptyKey || q.y == kEmptyKey || q.z == kEmptyKey || q.w == kEmptyKey)) {
-      // k is new to this bucket and it has room: claim the first free slot
+      // k is new to this bucket and it has room: claim the first free slot,
+      // starting at another slot every 8 buckets.  Most buckets hold one or
+      // two keys; with all of those in their first slots the sums and counts
+      // of a warp's rows fell on 8 to 16 of the 32 banks (5.3 passes per
+      // atomic instead of 3.5).
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int i = 0; i < 4; ++i) {
+        const int j = i ^ static_cast<int>((b >> 3) & 3u);
         const int32_t cur = j == 0 ? q.x : j == 1 ? q.y : j == 2 ? q.z : q.w;
         if (slot < 0 && cur == kEmptyKey) {
           const int32_t prev = atomicCAS(t.key + 4 * b + j, kEmptyKey, k);
@@ -216,7 +238,9 @@ __device__ __forceinline__ int smem_find_insert(const SmemAgg& t, int32_t k, uin
 __device__ __forceinline__ bool smem_agg_add(const SmemAgg& t, int32_t k, uint64_t s, uint32_t c) {
   const int i = smem_find_insert(t, k, t.home(k));
   if (i < 0) return false;
-  smem_add_split(t.lo, t.slots, i, s);
+  const uint32_t old = atomicAdd(t.lo + i, static_cast<uint32_t>(s));
+  const int32_t h = agg_high(old, static_cast<int64_t>(s));
+  if (h) atomicAdd(t.lo + t.slots + i, static_cast<uint32_t>(h));
   atomicAdd(t.cnt + i, c);
   return true;
 }
@@ -339,36 +363,41 @@ __global__ void __launch_bounds__(kAggThreads) group_hash_smem_kernel(int64_t n,
 // R rows (count 1 each) into the shared table, with every step of the R rows
 // issued together: the R home buckets are read first (plain loads: a stale
 // read can only miss a key, since keys are never removed, and a miss takes
-// the volatile insert path), then the R low-word adds whose old values give
-// the carries, the R count adds, and the high words where a carry or a
-// negative value needs one.  Only 32-bit shared atomics: on B200 a 64-bit
-// shared atomicAdd runs several times slower than a 32-bit one.  `sync`: the
-// lanes of the warp that call together (0 when the callers are not
-// warp-uniform); they are brought back together after the insert path, whose
-// probe loop ends at a different step on each lane (left diverged, the warp
-// would run all later steps once per lane group).  Returns the mask of the
-// rows that found no room (the caller adds them elsewhere).
-template <int R>
-__device__ __forceinline__ uint32_t smem_agg_rows(const SmemAgg& t, const int32_t (&k)[R], const int64_t (&v)[R],
+// the volatile insert path), then the R low-word adds whose old values tell
+// an overflow, the R count adds, and the high words where one is needed.  Only
+// 32-bit shared atomics: on B200 a 64-bit shared atomicAdd runs several times
+// slower than a 32-bit one.  V: int32_t, or int64_t for values of 33 bits.
+// kAll: every row is valid.  `sync`: the lanes of the warp that call together
+// (0 when the callers are not warp-uniform); they are brought back together
+// after the insert path, whose probe loop ends at a different step on each
+// lane (left diverged, the warp would run all later steps once per lane
+// group).  Returns the mask of the rows that found no room (the caller adds
+// them elsewhere).
+template <int R, bool kAll, class V>
+__device__ __forceinline__ uint32_t smem_agg_rows(const SmemAgg& t, const int32_t (&k)[R], const V (&v)[R],
                                                   uint32_t valid, uint32_t sync) {
   uint32_t b[R];
   int4 q[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    b[r] = t.home(k[r]);
-    q[r] = ((valid >> r) & 1u) ? *reinterpret_cast<const int4*>(t.key + 4 * b[r]) : make_int4(0, 0, 0, 0);
+    b[r] = 4 * t.home(k[r]);
+    q[r] = *reinterpret_cast<const int4*>(t.key + b[r]);
   }
   int s[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    s[r] = -1;
+    if (q[r].x == k[r]) s[r] = b[r];
+    if (q[r].y == k[r]) s[r] = b[r] + 1;
+    if (q[r].z == k[r]) s[r] = b[r] + 2;
+    if (q[r].w == k[r]) s[r] = b[r] + 3;
+    if (!kAll && !((valid >> r) & 1u)) s[r] = -2;
+  }
   uint32_t lost = 0;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int j = q[r].x == k[r] ? 0 : q[r].y == k[r] ? 1 : q[r].z == k[r] ? 2 : q[r].w == k[r] ? 3 : -1;
-    s[r] = ((valid >> r) & 1u) && j >= 0 ? static_cast<int>(4 * b[r]) + j : -1;
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    if (((valid >> r) & 1u) && s[r] < 0) {
-      s[r] = smem_find_insert(t, k[r], b[r]);
+    if (s[r] == -1) {
+      s[r] = smem_find_insert(t, k[r], b[r] >> 2);
       if (s[r] < 0) lost |= 1u << r;
     }
   }
@@ -382,10 +411,8 @@ __device__ __forceinline__ uint32_t smem_agg_rows(const SmemAgg& t, const int32_
     if (s[r] >= 0) atomicAdd(t.cnt + s[r], 1u);
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    if (s[r] < 0) continue;
-    const uint32_t lo = static_cast<uint32_t>(v[r]);
-    const uint32_t hi = static_cast<uint32_t>(static_cast<uint64_t>(v[r]) >> 32) + ((old[r] + lo) < old[r] ? 1u : 0u);
-    if (hi) atomicAdd(t.lo + t.slots + s[r], hi);
+    const int32_t h = agg_high(old[r], v[r]);
+    if (h && s[r] >= 0) atomicAdd(t.lo + t.slots + s[r], static_cast<uint32_t>(h));
   }
   return lost;
 }
@@ -415,28 +442,40 @@ __global__ void __launch_bounds__(kRowsThreads) group_hash_rows_kernel(int64_t n
   const int64_t e = b + per < n ? b + per : n;
   const uint64_t pol = policy_evict_first();
   unsigned int bad = 0;
-  auto rows = [&](const int4 kk, const int4 a, const int4 c, uint32_t valid, uint32_t sync) {
+  using V = std::conditional_t<HAS2, int64_t, int32_t>;
+  auto rows = [&](auto all, const int4 kk, const int4 a, const int4 c, uint32_t valid, uint32_t sync) {
     const int32_t kr[4] = {kk.x, kk.y, kk.z, kk.w}, ar[4] = {a.x, a.y, a.z, a.w}, cr[4] = {c.x, c.y, c.z, c.w};
     int32_t k[4];
-    int64_t v[4];
+    V v[4];
+    bool none = false;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       k[u] = agg_key(kr[u], key_offset);
-      v[u] = static_cast<int64_t>(ar[u]) + (HAS2 ? cr[u] : 0);
-      if (((valid >> u) & 1u) && k[u] == kEmptyKey) {  // reserved as the empty marker
-        ++bad;
-        valid &= ~(1u << u);
+      v[u] = static_cast<V>(ar[u]) + (HAS2 ? cr[u] : 0);
+      none |= k[u] == kEmptyKey;
+    }
+    // reserved as the empty marker (rare): not valid rows
+    if (none) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (((valid >> u) & 1u) && k[u] == kEmptyKey) {
+          ++bad;
+          valid &= ~(1u << u);
+        }
       }
     }
-    const uint32_t lost = smem_agg_rows<4>(t, k, v, valid, sync);
+    const uint32_t lost = (decltype(all)::value && __all_sync(0xffffffffu, valid == 0xFu))
+                              ? smem_agg_rows<4, true>(t, k, v, 0xFu, sync)
+                              : smem_agg_rows<4, false>(t, k, v, valid, sync);
     if (lost) {  // rare: keys that found no room in the table
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if ((lost >> u) & 1u) global_add(g, k[u], static_cast<uint64_t>(v[u]), 1);
+        if ((lost >> u) & 1u) global_add(g, k[u], static_cast<uint64_t>(static_cast<int64_t>(v[u])), 1);
     }
   };
   auto one = [&](int64_t r) {
-    rows(make_int4(keys[r], 0, 0, 0), make_int4(vals[r], 0, 0, 0), make_int4(HAS2 ? vals2[r] : 0, 0, 0, 0), 1u, 0u);
+    rows(std::false_type{}, make_int4(keys[r], 0, 0, 0), make_int4(vals[r], 0, 0, 0),
+         make_int4(HAS2 ? vals2[r] : 0, 0, 0, 0), 1u, 0u);
   };
   if (b < e) {
     const int64_t b4 = (b + 3) & ~int64_t(3);
@@ -467,7 +506,7 @@ __global__ void __launch_bounds__(kRowsThreads) group_hash_rows_kernel(int64_t n
         an = ld_stream_v4(ap + 4 * nx, pol);
         if (HAS2) cn = ld_stream_v4(cp + 4 * nx, pol);
       }
-      rows(kk, a, c, i < n4 ? 0xFu : 0u, 0xffffffffu);
+      rows(std::true_type{}, kk, a, c, i < n4 ? 0xFu : 0u, 0xffffffffu);
       kk = kn;
       a = an;
       c = cn;
@@ -481,18 +520,18 @@ __global__ void __launch_bounds__(kRowsThreads) group_hash_rows_kernel(int64_t n
     if (t.key[i] != kEmptyKey && t.cnt[i]) global_add(g, t.key[i], t.sum(i), t.cnt[i]);
 }
 
-// Plan 2.  Partition of a key: the top bits of its hash (the shared tables
-// index with the low bits).
-__device__ __forceinline__ uint32_t agg_part(int32_t k, int part_shift) {
-  return part_shift >= 32 ? 0u : mix32(static_cast<uint32_t>(k)) >> part_shift;
+// Plan 2.  Partition of a key: its hash scaled onto the partitions (the shared
+// tables index with the low bits).
+__device__ __forceinline__ uint32_t agg_part(int32_t k, int n_parts) {
+  return __umulhi(mix32(static_cast<uint32_t>(k)), static_cast<uint32_t>(n_parts));
 }
 
 struct PartPlan {
   int64_t n;
   int64_t per;        // rows per block of the histogram and scatter passes (multiple of 4)
   int32_t n_blocks;   // blocks of those passes
-  int32_t n_parts;    // P (power of two)
-  int32_t part_shift; // 32 - log2(P)
+  int32_t n_parts;    // P
+  uint32_t slots;     // slots of a partition's shared table
   int32_t key_offset;
 };
 
@@ -516,20 +555,25 @@ __global__ void __launch_bounds__(1024) group_part_hist_kernel(PartPlan pp, cons
       ++bad;
       return;
     }
-    atomicAdd(&s_hist[agg_part(k, pp.part_shift)], 1u);
+    atomicAdd(&s_hist[agg_part(k, pp.n_parts)], 1u);
   };
+  int64_t done = b;  // four 16-byte loads per thread in flight
   if (vec) {
-    for (int64_t r = b + 4 * threadIdx.x; r < e; r += 4 * blockDim.x) {
-      if (r + 4 <= e) {
-        const int4 k = ld_stream_v4(keys + r, pol);
-        one(k.x); one(k.y); one(k.z); one(k.w);
-      } else {
-        for (int64_t q = r; q < e; ++q) one(keys[q]);
+    const int64_t step = 16 * static_cast<int64_t>(blockDim.x);
+    for (; done + step <= e; done += step) {
+      int4 k[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) k[u] = ld_stream_v4_ordered(keys + done + 4 * (threadIdx.x + u * static_cast<int64_t>(blockDim.x)), pol);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        one(k[u].x);
+        one(k[u].y);
+        one(k[u].z);
+        one(k[u].w);
       }
     }
-  } else {
-    for (int64_t r = b + threadIdx.x; r < e; r += blockDim.x) one(keys[r]);
   }
+  for (int64_t r = done + threadIdx.x; r < e; r += blockDim.x) one(keys[r]);
   const unsigned int wbad = __reduce_add_sync(0xffffffffu, bad);
   if ((threadIdx.x & 31) == 0 && wbad) atomicAdd(range_err, static_cast<unsigned long long>(wbad));
   __syncthreads();
@@ -611,7 +655,7 @@ __global__ void __launch_bounds__(1024) group_part_scatter_kernel(PartPlan pp, c
   auto one = [&](int32_t key, int32_t a, int32_t c) {
     const int32_t k = agg_key(key, pp.key_offset);
     if (k == kEmptyKey) return;
-    const unsigned int pos = atomicAdd(&s_cur[agg_part(k, pp.part_shift)], 1u);
+    const unsigned int pos = atomicAdd(&s_cur[agg_part(k, pp.n_parts)], 1u);
     rows[pos] = PartRow<HAS2>::make(k, a, c);
   };
   if (vec) {
@@ -625,7 +669,7 @@ __global__ void __launch_bounds__(1024) group_part_scatter_kernel(PartPlan pp, c
         unsigned int pos[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-          pos[u] = k[u] != kEmptyKey ? atomicAdd(&s_cur[agg_part(k[u], pp.part_shift)], 1u) : 0u;
+          pos[u] = k[u] != kEmptyKey ? atomicAdd(&s_cur[agg_part(k[u], pp.n_parts)], 1u) : 0u;
         const int32_t av[4] = {a.x, a.y, a.z, a.w}, cv[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
         for (int u = 0; u < 4; ++u)
@@ -639,101 +683,122 @@ __global__ void __launch_bounds__(1024) group_part_scatter_kernel(PartPlan pp, c
   }
 }
 
-// The same scatter with coalesced writes (P <= kTiledParts): each tile of
-// kScatterTile rows (8 per thread) is counting-sorted by partition in shared
-// memory, then written out so that consecutive threads write consecutive
-// rows of a partition's run.  A row's partition is hashed once and kept
-// beside it in the sorted tile, and each partition's destination base is
-// worked out once per tile, so the write-out looks up one word per row.
-// Shared memory: the sorted rows and their partitions, then per partition
-// the tile count, the tile offset, the block's cursor and the destination
-// base.  The next tile's columns are prefetched into L2 while the current
-// one is sorted and written.  (4,096-row tiles of 4 rows per thread with the
-// partition hashed three times took 4.2 warp-instructions per row; now 2.8.)
-constexpr int kScatterTile = 8192;
-constexpr int kMaxPartials = 256;  // partial tables of split partitions (128 KB each)
-constexpr int kTiledParts = 4096;
+// The same scatter with coalesced writes: each tile of 8,192 rows (16 per
+// thread) is counting-sorted by partition in shared
+// memory, then written out so that consecutive threads write consecutive rows
+// of a partition's run.  A run ends at a whole 32-byte sector; the rows past
+// it (at most kCarry per partition) are carried into the next tile, because a
+// sector written in two pieces costs L2 a read-modify-write when it is evicted
+// in between (writing every row at once took 778 us for 2^27 rows in 444
+// partitions, the same rows in input order 519 us, no rows 472 us).  The rest
+// is the shared-memory pipe and the tile's chain of dependent phases: so two
+// blocks fit an SM, the next tile's keys load while the current tile is
+// written out and are ranked right after (one phase between barriers), and a
+// sorted row's partition is hashed again instead of kept beside it.  Shared
+// memory: the sorted rows, the carried rows, then per partition the tile
+// count, the tile offset of the new rows, the block's cursor, the destination
+// base, the tile index its write ends at, and the carried count.
+constexpr int kScatterThreads = 512;
+constexpr int kScatterBlocks = 2;
+constexpr int kMaxPartials = 256;  // partial tables of split partitions
 
 template <bool HAS2>
-__global__ void __launch_bounds__(1024, 1) group_part_scatter_tiled_kernel(
+constexpr int scatter_carry() {  // rows a sector holds, less one
+  return 32 / static_cast<int>(sizeof(typename PartRow<HAS2>::T)) - 1;
+}
+// G: 16-byte loads of a column per thread and tile (4, or 2 where the
+// partitions leave no room for the longer tile).
+template <bool HAS2, int G>
+constexpr size_t scatter_smem(int64_t parts) {
+  return sizeof(typename PartRow<HAS2>::T) * (4 * G * kScatterThreads + 2 * scatter_carry<HAS2>() * parts) + 6 * 4 * parts;
+}
+
+template <bool HAS2, int G>
+__global__ void __launch_bounds__(kScatterThreads, kScatterBlocks) group_part_scatter_tiled_kernel(
     PartPlan pp, const int32_t* __restrict__ keys, const int32_t* __restrict__ vals,
     const int32_t* __restrict__ vals2, const unsigned int* __restrict__ hist, unsigned long long* __restrict__ cursor,
     typename PartRow<HAS2>::T* __restrict__ rows) {
   using Row = typename PartRow<HAS2>::T;
+  constexpr int W = kScatterThreads / 32;
+  constexpr int R = 4 * G;
+  constexpr int kTile = R * kScatterThreads;
+  constexpr int C = scatter_carry<HAS2>();
   extern __shared__ __align__(16) unsigned char sc_smem[];
-  Row* s_rows = reinterpret_cast<Row*>(sc_smem);
-  uint16_t* s_part = reinterpret_cast<uint16_t*>(s_rows + kScatterTile);
-  unsigned int* s_cnt = reinterpret_cast<unsigned int*>(s_part + kScatterTile);
-  unsigned int* s_off = s_cnt + pp.n_parts;
-  unsigned int* s_cur = s_off + pp.n_parts;
-  unsigned int* s_dst = s_cur + pp.n_parts;
-  __shared__ unsigned int s_warp[32];
   const int P = pp.n_parts;
+  Row* s_rows = reinterpret_cast<Row*>(sc_smem);
+  Row* s_carry = s_rows + kTile + C * P;
+  unsigned int* s_cnt = reinterpret_cast<unsigned int*>(s_carry + C * P);
+  unsigned int* s_off = s_cnt + P;
+  unsigned int* s_cur = s_off + P;
+  unsigned int* s_dst = s_cur + P;
+  unsigned int* s_end = s_dst + P;
+  unsigned int* s_left = s_end + P;
+  __shared__ unsigned int s_warp[W];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int p = tid; p < P; p += blockDim.x) {
+  const int64_t b = static_cast<int64_t>(blockIdx.x) * pp.per;
+  const int64_t e = b + pp.per < pp.n ? b + pp.per : pp.n;
+  if (b >= e) return;
+  for (int p = tid; p < P; p += kScatterThreads) {
     const unsigned int c = hist[static_cast<int64_t>(blockIdx.x) * P + p];
     s_cur[p] = c ? static_cast<unsigned int>(atomicAdd(&cursor[p], static_cast<unsigned long long>(c))) : 0u;
     s_cnt[p] = 0;
+    s_left[p] = 0;
   }
-  const int64_t b = static_cast<int64_t>(blockIdx.x) * pp.per;
-  const int64_t e = b + pp.per < pp.n ? b + pp.per : pp.n;
   const uint64_t pol = policy_evict_first();
   const bool vec = ((reinterpret_cast<uintptr_t>(keys) | reinterpret_cast<uintptr_t>(vals) |
                      reinterpret_cast<uintptr_t>(vals2)) & 15) == 0;
-  const int per_thread = (P + blockDim.x - 1) / blockDim.x;  // partitions per thread in the scan
+  const int per_thread = (P + kScatterThreads - 1) / kScatterThreads;  // partitions per thread in the scan
   auto prefetch_tile = [&](int64_t t0) {  // the tile's columns into L2, ahead of its loads
     if (tid != 0 || t0 >= e) return;
-    const int64_t m = e - t0 < kScatterTile ? e - t0 : kScatterTile;
+    const int64_t m = e - t0 < kTile ? e - t0 : kTile;
     prefetch_l2_range(keys + t0, 4 * m);
     prefetch_l2_range(vals + t0, 4 * m);
     if (HAS2) prefetch_l2_range(vals2 + t0, 4 * m);
   };
-  prefetch_tile(b);
-  __syncthreads();
-  for (int64_t t0 = b; t0 < e; t0 += kScatterTile) {
-    prefetch_tile(t0 + kScatterTile);
-    // 1. this thread's 8 rows (4 at t0 + 4 tid, 4 at t0 + 4 (tid + 1024)):
-    //    key, partition and rank inside the tile
-    int32_t k[8], a[8], c[8];
-    uint32_t slot[8];  // partition << 13 | rank, or ~0u for no row
+  // this thread's 16 rows of a tile: 4 at t0 + 4 (tid + 512 h) for each h
+  auto row0 = [&](int64_t t0, int h) { return t0 + 4 * (tid + h * static_cast<int64_t>(kScatterThreads)); };
+  int32_t k[R];
+  uint32_t slot[R];  // partition << 13 | rank, or ~0u for no row
+  // what the key column would hold for the reserved key: no row
+  const int32_t no_key = static_cast<int32_t>(static_cast<uint32_t>(kEmptyKey) - static_cast<uint32_t>(pp.key_offset));
+  auto load_keys = [&](int64_t t0) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int64_t r0 = t0 + 4 * (tid + h * static_cast<int64_t>(blockDim.x));
+    for (int h = 0; h < G; ++h) {
+      const int64_t r0 = row0(t0, h);
       if (vec && r0 + 4 <= e) {
-        const int4 kk = ld_stream_v4(keys + r0, pol), av = ld_stream_v4(vals + r0, pol);
-        const int4 cv = HAS2 ? ld_stream_v4(vals2 + r0, pol) : make_int4(0, 0, 0, 0);
+        const int4 kk = ld_stream_v4_ordered(keys + r0, pol);
         k[4 * h] = kk.x; k[4 * h + 1] = kk.y; k[4 * h + 2] = kk.z; k[4 * h + 3] = kk.w;
-        a[4 * h] = av.x; a[4 * h + 1] = av.y; a[4 * h + 2] = av.z; a[4 * h + 3] = av.w;
-        c[4 * h] = cv.x; c[4 * h + 1] = cv.y; c[4 * h + 2] = cv.z; c[4 * h + 3] = cv.w;
       } else {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const bool ok = r0 + u < e;
-          k[4 * h + u] = ok ? keys[r0 + u] : kEmptyKey;
-          a[4 * h + u] = ok ? vals[r0 + u] : 0;
-          c[4 * h + u] = ok && HAS2 ? vals2[r0 + u] : 0;
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int q = 4 * h + u;
-        slot[q] = ~0u;
-        if (r0 + u < e) {
-          k[q] = agg_key(k[q], pp.key_offset);
-          if (k[q] != kEmptyKey) {
-            const uint32_t part = agg_part(k[q], pp.part_shift);
-            slot[q] = (part << 13) | atomicAdd(&s_cnt[part], 1u);
-          }
-        }
+        for (int u = 0; u < 4; ++u) k[4 * h + u] = r0 + u < e ? keys[r0 + u] : no_key;
       }
     }
+  };
+  auto rank_keys = [&]() {
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      k[q] = agg_key(k[q], pp.key_offset);
+      slot[q] = ~0u;
+      if (k[q] != kEmptyKey) {
+        const uint32_t part = agg_part(k[q], P);
+        slot[q] = (part << 13) | atomicAdd(&s_cnt[part], 1u);
+      }
+    }
+  };
+  prefetch_tile(b + kTile);
+  load_keys(b);
+  __syncthreads();  // the counts are zero
+  rank_keys();
+  for (int64_t t0 = b; t0 < e; t0 += kTile) {
+    const bool more = t0 + kTile < e;
+    prefetch_tile(t0 + 2 * kTile);
     __syncthreads();
-    // 2. exclusive scan of the tile counts (each thread a run of partitions);
-    //    destination bases, and the block's cursors moved past the tile
+    // exclusive scan of the tile's rows per partition, carried ones first
+    // (each thread a run of partitions)
     unsigned int run = 0;
     for (int j = 0; j < per_thread; ++j) {
       const int p = tid * per_thread + j;
-      if (p < P) run += s_cnt[p];
+      if (p < P) run += s_cnt[p] + s_left[p];
     }
     unsigned int inc = run;
 #pragma unroll
@@ -743,42 +808,66 @@ __global__ void __launch_bounds__(1024, 1) group_part_scatter_tiled_kernel(
     }
     if (lane == 31) s_warp[warp] = inc;
     __syncthreads();
-    if (warp == 0) {
-      unsigned int w = lane < static_cast<int>(blockDim.x >> 5) ? s_warp[lane] : 0u;
+    unsigned int off = inc - run, n_valid = 0;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned int y = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += y;
-      }
-      s_warp[lane] = w;  // inclusive over warps
+    for (int w = 0; w < W; ++w) {
+      const unsigned int x = s_warp[w];
+      if (w < warp) off += x;
+      n_valid += x;
     }
-    __syncthreads();
-    unsigned int off = (warp > 0 ? s_warp[warp - 1] : 0u) + inc - run;
-    const unsigned int n_valid = s_warp[(blockDim.x >> 5) - 1];
     for (int j = 0; j < per_thread; ++j) {
       const int p = tid * per_thread + j;
       if (p < P) {
-        const unsigned int cnt = s_cnt[p];
-        s_off[p] = off;
-        s_dst[p] = s_cur[p] - off;
-        s_cur[p] += cnt;
+        const unsigned int old = s_left[p], all = s_cnt[p] + old, cur = s_cur[p];
+        // written up to the last whole sector, all of it at the end
+        const unsigned int left = more ? min(all, (cur + all) & static_cast<unsigned int>(C)) : 0u;
+        for (unsigned int c = 0; c < old; ++c) s_rows[off + c] = s_carry[C * p + c];
+        s_off[p] = off + old;
+        s_dst[p] = cur - off;
+        s_end[p] = off + all - left;
+        s_cur[p] = cur + all - left;
+        s_left[p] = left;
         s_cnt[p] = 0;
-        off += cnt;
+        off += all;
       }
     }
     __syncthreads();
-    // 3. rows into their sorted places
+    // rows into their sorted places (the values are read only now: 16 of them
+    // beside the keys would not fit a thread's registers)
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      if (slot[q] == ~0u) continue;
-      const unsigned int at = s_off[slot[q] >> 13] + (slot[q] & 8191u);
-      s_rows[at] = PartRow<HAS2>::make(k[q], a[q], c[q]);
-      s_part[at] = static_cast<uint16_t>(slot[q] >> 13);
+    for (int h = 0; h < G; ++h) {
+      const int64_t r0 = row0(t0, h);
+      int32_t a[4], c[4];
+      if (vec && r0 + 4 <= e) {
+        const int4 av = ld_stream_v4(vals + r0, pol);
+        const int4 cv = HAS2 ? ld_stream_v4(vals2 + r0, pol) : make_int4(0, 0, 0, 0);
+        a[0] = av.x; a[1] = av.y; a[2] = av.z; a[3] = av.w;
+        c[0] = cv.x; c[1] = cv.y; c[2] = cv.z; c[3] = cv.w;
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          a[u] = r0 + u < e ? vals[r0 + u] : 0;
+          c[u] = HAS2 && r0 + u < e ? vals2[r0 + u] : 0;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t sl = slot[4 * h + u];
+        if (sl != ~0u) s_rows[s_off[sl >> 13] + (sl & 8191u)] = PartRow<HAS2>::make(k[4 * h + u], a[u], c[u]);
+      }
     }
     __syncthreads();
-    // 4. coalesced writes: sorted row i goes to its partition's run
-    for (unsigned int i = tid; i < n_valid; i += blockDim.x) rows[s_dst[s_part[i]] + i] = s_rows[i];
-    __syncthreads();
+    // coalesced writes (sorted row i goes to its partition's run, or is
+    // carried), while the next tile's keys load
+    if (more) load_keys(t0 + kTile);
+    for (unsigned int i = tid; i < n_valid; i += kScatterThreads) {
+      const Row x = s_rows[i];
+      const uint32_t p = agg_part(PartRow<HAS2>::key(x), P);
+      const unsigned int end = s_end[p];
+      if (i < end) rows[s_dst[p] + i] = x;
+      else s_carry[C * p + (i - end)] = x;
+    }
+    if (more) rank_keys();
   }
 }
 
@@ -792,12 +881,12 @@ __device__ __forceinline__ void append_groups(const SmemAgg& st, int64_t capacit
   __shared__ unsigned long long s_base;
   if (threadIdx.x == 0) s_n = 0;
   __syncthreads();
-  constexpr int kPer = kAggSlots / kAggThreads;
+  constexpr int kPer = kAggMaxSlots / kAggThreads;
   unsigned int pos[kPer];
 #pragma unroll
   for (int j = 0; j < kPer; ++j) {
-    const int i = j * kAggThreads + threadIdx.x;
-    pos[j] = st.key[i] != kEmptyKey ? atomicAdd(&s_n, 1u) : ~0u;
+    const uint32_t i = j * kAggThreads + threadIdx.x;
+    pos[j] = i < st.slots && st.key[i] != kEmptyKey ? atomicAdd(&s_n, 1u) : ~0u;
   }
   __syncthreads();
   if (threadIdx.x == 0) s_base = s_n ? atomicAdd(d_groups, static_cast<unsigned long long>(s_n)) : 0ull;
@@ -805,7 +894,7 @@ __device__ __forceinline__ void append_groups(const SmemAgg& st, int64_t capacit
 #pragma unroll
   for (int j = 0; j < kPer; ++j) {
     if (pos[j] == ~0u) continue;
-    const int i = j * kAggThreads + threadIdx.x;
+    const uint32_t i = j * kAggThreads + threadIdx.x;
     const unsigned long long o = s_base + pos[j];
     if (o >= static_cast<unsigned long long>(capacity)) {  // more groups than the outputs hold
       atomicAdd(overflow, 1ull);
@@ -832,11 +921,13 @@ struct AggUnit {
 template <bool HAS2>
 __global__ void __launch_bounds__(kAggThreads) group_part_agg_kernel(
     const long long* __restrict__ part_begin, const AggUnit* __restrict__ units,
-    const typename PartRow<HAS2>::T* __restrict__ rows, int combine, int64_t capacity,
+    const typename PartRow<HAS2>::T* __restrict__ rows, uint32_t slots, int combine, int64_t capacity,
     int32_t* __restrict__ out_keys, int64_t* __restrict__ out_sums, int64_t* __restrict__ out_counts,
     unsigned long long* d_groups, unsigned long long* overflow, int4* __restrict__ partials) {
   extern __shared__ __align__(16) unsigned char agg_smem[];
-  const SmemAgg st = smem_agg(agg_smem, kAggSlots);
+  using V = std::conditional_t<HAS2, int64_t, int32_t>;
+  using Row = typename PartRow<HAS2>::T;
+  const SmemAgg st = smem_agg(agg_smem, slots);
   smem_agg_clear(st);
   __syncthreads();
   int64_t b, e;
@@ -851,51 +942,61 @@ __global__ void __launch_bounds__(kAggThreads) group_part_agg_kernel(
     e = part_begin[blockIdx.x + 1];
   }
   unsigned int lost = 0;
-  // rows of the partition, 8 per thread in flight
-  for (int64_t base = b; base < e; base += 8 * static_cast<int64_t>(blockDim.x)) {
-    if (!combine) {  // two batches of 4 rows
+  const Row* p = rows + b + threadIdx.x;
+  int64_t left = e - b;
+  // whole steps of 8 rows per thread, in two batches; the step after next is
+  // on its way into L2
+  constexpr int64_t kStep = 8 * kAggThreads;
+  if (!combine) {
+    for (; left >= kStep; left -= kStep, p += kStep) {
+      if (threadIdx.x == 0 && left >= 3 * kStep) prefetch_l2_range(p + 2 * kStep, kStep * sizeof(Row));
+      Row x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = p[u * kAggThreads];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         int32_t k[4];
-        int64_t v[4];
-        uint32_t valid = 0;
+        V v[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const int64_t i = base + (4 * h + u) * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-          const bool ok = i < e;
-          typename PartRow<HAS2>::T x{};
-          if (ok) x = rows[i];
-          k[u] = ok ? PartRow<HAS2>::key(x) : 0;
-          v[u] = ok ? PartRow<HAS2>::val(x) : 0;
-          valid |= static_cast<uint32_t>(ok) << u;
+          k[u] = PartRow<HAS2>::key(x[4 * h + u]);
+          v[u] = static_cast<V>(PartRow<HAS2>::val(x[4 * h + u]));
         }
-        lost += __popc(smem_agg_rows<4>(st, k, v, valid, 0xffffffffu));  // the loop is block-uniform
+        lost += __popc(smem_agg_rows<4, true>(st, k, v, 0xFu, 0xffffffffu));  // the loop is block-uniform
       }
+    }
+  }
+  for (; left > 0; left -= 4 * kAggThreads, p += 4 * kAggThreads) {
+    int32_t k[4];
+    V v[4];
+    uint32_t valid = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool ok = u * kAggThreads + static_cast<int64_t>(threadIdx.x) < left;
+      Row x{};
+      if (ok) x = p[u * kAggThreads];
+      k[u] = ok ? PartRow<HAS2>::key(x) : 0;
+      v[u] = ok ? static_cast<V>(PartRow<HAS2>::val(x)) : 0;
+      valid |= static_cast<uint32_t>(ok) << u;
+    }
+    if (!combine) {
+      lost += __popc(smem_agg_rows<4, false>(st, k, v, valid, 0xffffffffu));
       continue;
     }
-    typename PartRow<HAS2>::T r[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int64_t i = base + u * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-      if (i < e) r[u] = rows[i];
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int64_t i = base + u * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-      const bool ok = i < e;
-      const int32_t k = ok ? PartRow<HAS2>::key(r[u]) : 0;
-      int64_t gs = ok ? PartRow<HAS2>::val(r[u]) : 0;
+    for (int u = 0; u < 4; ++u) {
+      int64_t gs = v[u];
       uint32_t gc = 1;
-      if (warp_combine(ok, k, gs, &gs, &gc))
-        if (!smem_agg_add(st, k, static_cast<uint64_t>(gs), gc)) ++lost;
+      if (warp_combine((valid >> u) & 1u, k[u], gs, &gs, &gc))
+        if (!smem_agg_add(st, k[u], static_cast<uint64_t>(gs), gc)) ++lost;
     }
   }
   if (lost) atomicAdd(overflow, static_cast<unsigned long long>(lost));
   __syncthreads();
   if (partial >= 0) {  // the whole table, as laid out in shared memory (16 bytes per slot)
     const int4* src = reinterpret_cast<const int4*>(agg_smem);
-    int4* dst = partials + static_cast<int64_t>(partial) * kAggSlots;
-    for (int i = threadIdx.x; i < kAggSlots; i += blockDim.x) dst[i] = src[i];
+    int4* dst = partials + static_cast<int64_t>(partial) * slots;
+    for (uint32_t i = threadIdx.x; i < slots; i += blockDim.x) dst[i] = src[i];
     return;
   }
   append_groups(st, capacity, out_keys, out_sums, out_counts, d_groups, overflow);
@@ -905,22 +1006,48 @@ __global__ void __launch_bounds__(kAggThreads) group_part_agg_kernel(
 // tables of its units (merge[b] = (first partial, count)) in a shared table
 // and appends the groups.
 __global__ void __launch_bounds__(kAggThreads) group_part_merge_kernel(
-    const int2* __restrict__ merge, const int4* __restrict__ partials, int64_t capacity,
+    const int2* __restrict__ merge, const int4* __restrict__ partials, uint32_t slots, int64_t capacity,
     int32_t* __restrict__ out_keys, int64_t* __restrict__ out_sums, int64_t* __restrict__ out_counts,
     unsigned long long* d_groups, unsigned long long* overflow) {
   extern __shared__ __align__(16) unsigned char agg_smem[];
-  const SmemAgg st = smem_agg(agg_smem, kAggSlots);
-  smem_agg_clear(st);
-  __syncthreads();
+  const SmemAgg st = smem_agg(agg_smem, slots);
   const int2 m = merge[blockIdx.x];
   unsigned int lost = 0;
-  for (int q = 0; q < m.y; ++q) {
+  // the first table as it is (same layout and hash), then the slots of the
+  // others, four per thread with their key lookups in flight together
+  int4* dst = reinterpret_cast<int4*>(agg_smem);
+  for (uint32_t i = threadIdx.x; i < slots; i += blockDim.x) dst[i] = partials[static_cast<int64_t>(m.x) * slots + i];
+  __syncthreads();
+  for (int q = 1; q < m.y; ++q) {
     const SmemAgg pt = smem_agg(reinterpret_cast<unsigned char*>(const_cast<int4*>(partials) +
-                                                                 static_cast<int64_t>(m.x + q) * kAggSlots),
-                                kAggSlots);
-    for (int i = threadIdx.x; i < kAggSlots; i += blockDim.x) {
-      const int32_t k = pt.key[i];
-      if (k != kEmptyKey && !smem_agg_add(st, k, pt.sum(i), pt.cnt[i])) ++lost;
+                                                                 static_cast<int64_t>(m.x + q) * slots),
+                                slots);
+    for (uint32_t i0 = 0; i0 < slots; i0 += 4 * kAggThreads) {
+      int32_t k[4];
+      uint32_t lo[4], hi[4], c[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t i = i0 + u * kAggThreads + threadIdx.x;
+        const bool in = i < slots;
+        k[u] = in ? pt.key[i] : kEmptyKey;
+        lo[u] = in ? pt.lo[i] : 0u;
+        hi[u] = in ? pt.lo[slots + i] : 0u;
+        c[u] = in ? pt.cnt[i] : 0u;
+      }
+      int at[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) at[u] = k[u] != kEmptyKey ? smem_find_insert(st, k[u], st.home(k[u])) : -2;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (at[u] < 0) {
+          lost += at[u] == -1;
+          continue;
+        }
+        const uint32_t old = atomicAdd(st.lo + at[u], lo[u]);
+        const uint32_t h = hi[u] + static_cast<uint32_t>(agg_high(old, static_cast<int32_t>(lo[u])));
+        if (h) atomicAdd(st.lo + slots + at[u], h);
+        atomicAdd(st.cnt + at[u], c[u]);
+      }
     }
   }
   if (lost) atomicAdd(overflow, static_cast<unsigned long long>(lost));
@@ -1197,12 +1324,46 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
     olap::PartPlan pp;
     pp.n = n;
     pp.key_offset = key_offset;
-    int64_t parts = std::max<int64_t>(512, capacity / olap::kAggSlots);
-    int lg = 0;
-    while ((int64_t(1) << lg) < parts) ++lg;
-    if (lg > 15) return olap::set_error(ctx, OLAP_ERR_UNSUPPORTED, "hash group-by capacity above 2^27 slots");
-    pp.n_parts = 1 << lg;
-    pp.part_shift = 32 - lg;
+    if (capacity > (int64_t(1) << 27))
+      return olap::set_error(ctx, OLAP_ERR_UNSUPPORTED, "hash group-by capacity above 2^27 slots");
+    // Partitions: whole waves of one block per SM (no half-empty last wave),
+    // as few as keep the buckets of a partition's table at about a key on
+    // average (a key outside its home bucket leaves the batched path: 0.1 % of
+    // them at 0.7 keys a bucket, 0.4 % at one), since the scatter's runs get
+    // shorter with every partition: three waves of 14,336-slot tables for 2^20
+    // groups, eight for 2^22.  Few groups take 8,192-slot tables, which are
+    // cleared and emptied faster.
+    const int64_t keys_max = capacity / 2, sms = ctx->sm_count;
+    auto need = [&](int64_t slots, int64_t per4) {  // waves at per4 / 4 keys per bucket
+      return (4 * keys_max + per4 * sms * (slots / 4) - 1) / (per4 * sms * (slots / 4));
+    };
+    pp.slots = olap::kAggSlots;
+    int64_t waves = need(olap::kAggSlots, 3);
+    if (waves > 2) {
+      pp.slots = olap::kAggMaxSlots;
+      waves = std::max<int64_t>(3, need(olap::kAggMaxSlots, 4));
+    }
+    // The tiled scatter keeps some words per partition in shared memory: with
+    // more partitions than fit, fewer, as long as `capacity` distinct keys
+    // still fit their tables (13,600 of 14,336 slots), then the shorter tile,
+    // then the scatter without tiles.
+    const size_t room = static_cast<size_t>(ctx->smem_optin) - 1024;
+    auto tile_smem = [&](int64_t w, int g) {
+      const int64_t p = w * sms;
+      return g == 4 ? (vals2 ? olap::scatter_smem<true, 4>(p) : olap::scatter_smem<false, 4>(p))
+                    : (vals2 ? olap::scatter_smem<true, 2>(p) : olap::scatter_smem<false, 2>(p));
+    };
+    int tile_g = 0;
+    for (int g : {4, 2}) {
+      int64_t w = waves;
+      while (w > 1 && tile_smem(w, g) > room) --w;
+      if (w == waves || w * sms * 13600 >= capacity) {
+        waves = w;
+        tile_g = g;
+        break;
+      }
+    }
+    pp.n_parts = static_cast<int32_t>(waves * sms);
     pp.n_blocks = ctx->sm_count * 2;
     pp.per = ((n + pp.n_blocks - 1) / pp.n_blocks + 3) & ~int64_t(3);
     if (pp.per < 4) pp.per = 4;
@@ -1217,7 +1378,7 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
     const size_t max_units = static_cast<size_t>(pp.n_parts) + olap::kMaxPartials;
     const size_t merge_off = (units_off + sizeof(olap::AggUnit) * max_units + 255) & ~size_t(255);
     const size_t part_off = (merge_off + sizeof(int2) * static_cast<size_t>(pp.n_parts) + 255) & ~size_t(255);
-    const size_t bytes = part_off + static_cast<size_t>(olap::kMaxPartials) * olap::kAggSlots * 16;
+    const size_t bytes = part_off + static_cast<size_t>(olap::kMaxPartials) * pp.slots * 16;
     mem = olap::big_scratch(ctx, bytes);
     if (!mem) return olap::set_error(ctx, OLAP_ERR_NOMEM, "device memory for the group partitions");
     long long* part_begin = reinterpret_cast<long long*>(mem);
@@ -1241,16 +1402,13 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
         e = cudaFuncSetAttribute(olap::group_part_scatter_kernel<false>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(psmem));
     }
-    const size_t asmem = static_cast<size_t>(olap::kAggSlots) * 16;
-    if (pp.n_parts <= olap::kTiledParts) {
-      const int tsm = static_cast<int>((vals2 ? 18 : 10) * olap::kScatterTile + 4 * psmem);
+    const size_t asmem = static_cast<size_t>(pp.slots) * 16;
+    const size_t tsmem = tile_g ? tile_smem(waves, tile_g) : 0;
+    auto scatter_tiled = [&](auto* rows, auto kern) {
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tsmem));
       if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(olap::group_part_scatter_tiled_kernel<true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, tsm);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(olap::group_part_scatter_tiled_kernel<false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, tsm);
-    }
+        kern<<<pp.n_blocks, olap::kScatterThreads, tsmem, ctx->stream>>>(pp, keys, vals, vals2, hist, cursor, rows);
+    };
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(olap::group_part_agg_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(asmem));
@@ -1309,37 +1467,33 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
       const olap::AggUnit* unit_arg = merges.empty() ? nullptr : d_units;
       const unsigned agg_grid = merges.empty() ? static_cast<unsigned>(pp.n_parts)
                                                : static_cast<unsigned>(units.size());
-      const bool tiled = pp.n_parts <= olap::kTiledParts;
-      const size_t tsmem = (vals2 ? 18 : 10) * static_cast<size_t>(olap::kScatterTile) + 4 * psmem;
       if (vals2) {
         auto* rows = reinterpret_cast<longlong2*>(rowbuf);
-        if (tiled)
-          olap::group_part_scatter_tiled_kernel<true><<<pp.n_blocks, 1024, tsmem, ctx->stream>>>(
-              pp, keys, vals, vals2, hist, cursor, rows);
-        else
+        if (e == cudaSuccess && tile_g == 4) scatter_tiled(rows, olap::group_part_scatter_tiled_kernel<true, 4>);
+        else if (e == cudaSuccess && tile_g == 2) scatter_tiled(rows, olap::group_part_scatter_tiled_kernel<true, 2>);
+        else if (e == cudaSuccess)
           olap::group_part_scatter_kernel<true><<<pp.n_blocks, 1024, psmem, ctx->stream>>>(pp, keys, vals, vals2,
                                                                                           hist, cursor, rows);
         if (e == cudaSuccess)
           olap::group_part_agg_kernel<true><<<agg_grid, olap::kAggThreads, asmem, ctx->stream>>>(
-              part_begin, unit_arg, rows, combine, capacity, out_keys, out_sums, out_counts, d_groups_u, overflow,
+              part_begin, unit_arg, rows, pp.slots, combine, capacity, out_keys, out_sums, out_counts, d_groups_u, overflow,
               d_partials);
       } else {
         auto* rows = reinterpret_cast<int2*>(rowbuf);
-        if (tiled)
-          olap::group_part_scatter_tiled_kernel<false><<<pp.n_blocks, 1024, tsmem, ctx->stream>>>(
-              pp, keys, vals, nullptr, hist, cursor, rows);
-        else
+        if (e == cudaSuccess && tile_g == 4) scatter_tiled(rows, olap::group_part_scatter_tiled_kernel<false, 4>);
+        else if (e == cudaSuccess && tile_g == 2) scatter_tiled(rows, olap::group_part_scatter_tiled_kernel<false, 2>);
+        else if (e == cudaSuccess)
           olap::group_part_scatter_kernel<false><<<pp.n_blocks, 1024, psmem, ctx->stream>>>(pp, keys, vals,
                                                                                            nullptr, hist, cursor,
                                                                                            rows);
         if (e == cudaSuccess)
           olap::group_part_agg_kernel<false><<<agg_grid, olap::kAggThreads, asmem, ctx->stream>>>(
-              part_begin, unit_arg, rows, combine, capacity, out_keys, out_sums, out_counts, d_groups_u, overflow,
+              part_begin, unit_arg, rows, pp.slots, combine, capacity, out_keys, out_sums, out_counts, d_groups_u, overflow,
               d_partials);
       }
       if (e == cudaSuccess && !merges.empty())
         olap::group_part_merge_kernel<<<static_cast<unsigned>(merges.size()), olap::kAggThreads, asmem,
-                                        ctx->stream>>>(d_merge, d_partials, capacity, out_keys, out_sums,
+                                        ctx->stream>>>(d_merge, d_partials, pp.slots, capacity, out_keys, out_sums,
                                                        out_counts, d_groups_u, overflow);
       if (e == cudaSuccess) e = cudaGetLastError();
     }
