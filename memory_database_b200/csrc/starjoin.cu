@@ -68,10 +68,33 @@ struct StarParams {
   int32_t cmp_off;             // CMP: per-warp survivor buffers (shared-memory offset)
   int32_t merge_global;        // probe consecutive global int8 dimensions together
   unsigned long long* wait_timeouts;
-  unsigned long long* oob_seen;  // vec kernel: set when a key is out of range (the range pass counts them)
 };
 
 enum { ACC_NONE = 0, ACC_SMEM = 1, ACC_GLOBAL = 2 };
+
+// 1 when row r is a range error: a key out of range, and no in-range key that
+// meets DIM_NULL (a row that a filter drops anyway is none).
+template <int ND>
+__device__ __forceinline__ unsigned int range_error_row(const StarParams& p, int64_t r) {
+  bool ok = true, filtered = false;
+#pragma unroll
+  for (int j = 0; j < ND; ++j) {
+    const uint32_t k = static_cast<uint32_t>(p.dim[j].fk[r]);
+    if (k >= p.dim[j].len) ok = false;
+    else if (p.dim[j].vec[k] == OLAP_DIM_NULL) filtered = true;
+  }
+  return !ok && !filtered;
+}
+
+// Zeroes what a launch accumulates into or sets (one launch for all of it).
+__global__ void zero_outputs_kernel(unsigned long long* a, int64_t na, unsigned long long* b, int nb, int32_t* flags,
+                                    int nf) {
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (int64_t i = t; i < na; i += stride) a[i] = 0;
+  if (t < nb) b[t] = 0;
+  if (t < nf) flags[t] = 0;
+}
 
 // Pass bitmap of one dimension vector: bit k of word k/32 is set when
 // vec[k] != DIM_NULL; *nonzero becomes 1 when a live code is not 0 (then the
@@ -223,6 +246,7 @@ __device__ __forceinline__ void finish_block(const StarParams& p, int64_t tot0, 
 // them, an mbarrier counts the bytes) while the warp probes the current
 // ones, so the DRAM latency overlaps the dependent dimension probes instead
 // of adding to them; registers hold only the current vectors.
+constexpr uint32_t kMetOob = 1u << 31;
 constexpr uint32_t kAsyncWaitLimit = 1u << 24;  // polls of a prefetch barrier before giving up
 
 // CMP: after the shared-memory dimensions, each warp packs its surviving
@@ -383,11 +407,11 @@ __global__ void __launch_bounds__(V == 8 ? 512 : 1024, 1) starjoin_vec_kernel(co
       const int c = r & 3;
       return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w;
     };
-    // Range check of every key (registers only).  A row with a key out of
-    // range is dropped here and only flagged: whether it is a range error
-    // (none of its in-range keys meets DIM_NULL) is decided by the range pass
-    // that runs after this kernel when the flag is set, so the rare case adds
-    // nothing to this loop's registers.
+    // Range check of every key (registers only).  A row with a key out of range
+    // is dropped here and its thread only marked (in the top bit of its count,
+    // no register of its own): whether it is a range error is decided after
+    // the loop.  Deciding it here, even in a call, cost the loop 12 % by the
+    // registers it held.
     uint32_t oob = 0;
 #pragma unroll
     for (int r = 0; r < V; ++r) {
@@ -398,7 +422,7 @@ __global__ void __launch_bounds__(V == 8 ? 512 : 1024, 1) starjoin_vec_kernel(co
     }
     oob &= alive;
     if (oob) {
-      *reinterpret_cast<volatile unsigned long long*>(p.oob_seen) = 1ull;
+      bad |= kMetOob;
       alive &= ~oob;
       // keys of dropped rows to 0: every key left in registers addresses
       // its vector, so no probe below can leave it, predicated or not
@@ -601,6 +625,11 @@ __global__ void __launch_bounds__(V == 8 ? 512 : 1024, 1) starjoin_vec_kernel(co
     for (int r = 0; r < V; ++r)
       if (alive & (1u << r)) add_row(static_cast<uint32_t>(g[r]), mx(ka, r), mx(kb, r));
   }
+  if (bad & kMetOob) {  // rare: this thread's rows once more, for the range errors among them
+    bad &= ~kMetOob;
+    for (uint64_t i = blockIdx.x * blockDim.x + tid; i < nvec; i += gstride)
+      for (int c = 0; c < 4; ++c) bad += range_error_row<ND>(p, p.vec_begin + 4 * static_cast<int64_t>(i) + c);
+  }
   // Head and tail rows outside the 16-byte aligned range (block 0).
   if (blockIdx.x == 0) {
     auto one = [&](int64_t r) {
@@ -611,8 +640,8 @@ __global__ void __launch_bounds__(V == 8 ? 512 : 1024, 1) starjoin_vec_kernel(co
         k[j] = static_cast<uint32_t>(p.dim[j].fk[r]);
         ok &= k[j] < p.dim[j].len;
       }
-      if (!ok) {  // dropped and flagged; the range pass decides whether it is a range error
-        *reinterpret_cast<volatile unsigned long long*>(p.oob_seen) = 1ull;
+      if (!ok) {
+        bad += range_error_row<ND>(p, r);
         return;
       }
       int64_t g = 0;
@@ -728,45 +757,6 @@ __global__ void __launch_bounds__(1024, 1) starjoin_scalar_kernel(const StarPara
 }
 
 using StarKernel = void (*)(const StarParams);
-
-// Range pass of the 128-bit kernel.  That kernel drops a row with a key out
-// of range and only sets p.oob_seen; when the flag is set, this pass counts
-// the rows of [row_begin, row_end) with a key out of range and no in-range
-// key meeting DIM_NULL (the rows the plain path counts as range errors).
-// With the flag clear (the normal case) every block returns at once.
-template <int ND>
-__global__ void __launch_bounds__(256) starjoin_range_pass_kernel(const StarParams p) {
-  if (*reinterpret_cast<const volatile unsigned long long*>(p.oob_seen) == 0ull) return;
-  unsigned int bad = 0;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t r = p.row_begin + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < p.row_end;
-       r += stride) {
-    uint32_t k[ND > 0 ? ND : 1];
-    bool ok = true;
-#pragma unroll
-    for (int j = 0; j < ND; ++j) {
-      k[j] = static_cast<uint32_t>(p.dim[j].fk[r]);
-      ok &= k[j] < p.dim[j].len;
-    }
-    if (ok) continue;
-    bool filtered = false;
-#pragma unroll
-    for (int j = 0; j < ND; ++j)
-      if (k[j] < p.dim[j].len && p.dim[j].vec[k[j]] == OLAP_DIM_NULL) filtered = true;
-    bad += filtered ? 0u : 1u;
-  }
-  const unsigned int wbad = __reduce_add_sync(0xffffffffu, bad);
-  if ((threadIdx.x & 31) == 0 && wbad) atomicAdd(p.range_err, static_cast<unsigned long long>(wbad));
-}
-
-static StarKernel pick_range_pass(int nd) {
-  switch (nd) {
-    case 1: return starjoin_range_pass_kernel<1>;
-    case 2: return starjoin_range_pass_kernel<2>;
-    case 3: return starjoin_range_pass_kernel<3>;
-    default: return starjoin_range_pass_kernel<4>;
-  }
-}
 
 template <int ND, int ACC, bool ASYNC>
 static StarKernel pick_vec_a(int aggk, int v) {
@@ -1042,7 +1032,6 @@ int plan_starjoin(olap_ctx* ctx, const olap_starjoin_query* q, int64_t* group_su
   // Bulk-copy prefetch: per warp, 32 vectors of each streamed column for each
   // group of 4 rows per thread, and one mbarrier; only when it fits.
   sp->wait_timeouts = &ctx->counters->wait_timeouts;
-  sp->oob_seen = &ctx->counters->oob_seen;
   sp->merge_global = tune_or(ctx, TUNE_MERGE_PROBES, 2) == 1 ? 1 : 0;
   pl->async = false;
   if (vec && tune_or(ctx, TUNE_ASYNC_LOADS, 1) == 2 && nd + (need_m1 ? 1 : 0) + (need_m2 ? 1 : 0) > 0) {
@@ -1073,8 +1062,7 @@ int plan_starjoin(olap_ctx* ctx, const olap_starjoin_query* q, int64_t* group_su
 }
 
 int launch_starjoin(olap_ctx* ctx, StarPlan& pl, cudaStream_t stream) {
-  // Pass bitmaps (and their code flags) first, on the same stream.
-  if (pl.nbits || pl.nnib) OLAP_CUDA_TRY(ctx, cudaMemsetAsync(pl.code_nz, 0, sizeof(int32_t) * 2 * OLAP_MAX_DIMS, stream));
+  // Pass bitmaps (their code flags are zero by now) first, on the same stream.
   for (int b = 0; b < pl.nnib; ++b) {
     const Probe& d = pl.sp.dim[pl.nib_dim[b]];
     const uint64_t nbytes = (static_cast<uint64_t>(d.len) + 1) / 2;
@@ -1108,14 +1096,8 @@ int launch_starjoin(olap_ctx* ctx, StarPlan& pl, cudaStream_t stream) {
   int64_t grid = static_cast<int64_t>(ctx->sm_count) * bps;
   grid = std::min<int64_t>(grid, (work_items + pl.block - 1) / pl.block);
   grid = std::max<int64_t>(grid, 1);
-  const bool range_pass = pl.vec && pl.nd >= 1;
-  if (range_pass) OLAP_CUDA_TRY(ctx, cudaMemsetAsync(sp.oob_seen, 0, sizeof(unsigned long long), stream));
   k<<<static_cast<unsigned>(grid), pl.block, pl.smem, stream>>>(sp);
   OLAP_CUDA_TRY(ctx, cudaGetLastError());
-  if (range_pass) {
-    pick_range_pass(pl.nd)<<<static_cast<unsigned>(ctx->sm_count) * 2, 256, 0, stream>>>(sp);
-    OLAP_CUDA_TRY(ctx, cudaGetLastError());
-  }
   return OLAP_OK;
 }
 
@@ -1124,11 +1106,15 @@ int starjoin_device(olap_ctx* ctx, const olap_starjoin_query* q, int64_t* group_
   StarPlan pl;
   int st = plan_starjoin(ctx, q, group_sums, totals, ar, &pl);
   if (st != OLAP_OK) return st;
-  if (!accumulate) {
-    if (group_sums)
-      OLAP_CUDA_TRY(ctx, cudaMemsetAsync(group_sums, 0,
-                                         sizeof(int64_t) * q->group_nums * q->n_aggs, stream));
-    if (totals) OLAP_CUDA_TRY(ctx, cudaMemsetAsync(totals, 0, sizeof(int64_t) * q->n_aggs, stream));
+  const int64_t n_out = group_sums && !accumulate ? q->group_nums * q->n_aggs : 0;
+  const int n_tot = totals && !accumulate ? q->n_aggs : 0;
+  const int n_flags = pl.nbits || pl.nnib ? 2 * OLAP_MAX_DIMS : 0;
+  if (n_out || n_tot || n_flags) {
+    const unsigned blocks = static_cast<unsigned>(std::min<int64_t>(ctx->sm_count * int64_t(2), (n_out + 511) / 512 + 1));
+    zero_outputs_kernel<<<blocks, 512, 0, stream>>>(reinterpret_cast<unsigned long long*>(group_sums), n_out,
+                                                    reinterpret_cast<unsigned long long*>(totals), n_tot, pl.code_nz,
+                                                    n_flags);
+    OLAP_CUDA_TRY(ctx, cudaGetLastError());
   }
   if (q->row_end == q->row_begin) return OLAP_OK;
   return launch_starjoin(ctx, pl, stream);
@@ -1381,8 +1367,8 @@ int olap_starjoin_launch_count(olap_ctx* ctx, const olap_starjoin_query* q, int 
   int64_t probe = 0;  // only its address: the plan records the output pointers
   const int st = olap::plan_starjoin(ctx, q, want_groups ? &probe : nullptr, &probe, ar, &pl);
   if (st != OLAP_OK) return st;
-  // the star-join, its prepasses, and the range pass after the 128-bit kernel
-  *kernels = q->row_end > q->row_begin ? 1 + pl.nbits + pl.nnib + (pl.vec && pl.nd >= 1 ? 1 : 0) : 0;
+  // the zeroing of the outputs, the star-join and its prepasses
+  *kernels = q->row_end > q->row_begin ? 2 + pl.nbits + pl.nnib : 0;
   return OLAP_OK;
 }
 
