@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kCompactThreads) compact_kernel(const Op op_in
 // marks stay in L2 between the two kernels; an input whose marks do not fit
 // the arena runs in chunks, the running total kept on the device.
 constexpr int kExpandThreads = 1024;
-constexpr int kExpandDirect = 256;  // selected items of a step up to which its lanes write their own
+constexpr int kExpandDirect = 8;  // selected items per word of a step up to which the lanes write their own
 constexpr int kMarkRounds = 4;  // tiles per warp of a mark kernel on a long input
 
 struct Marks {
@@ -272,22 +272,22 @@ struct Marks {
 
 // Emit: constexpr bool kVals; void emit(int64_t pos, int64_t item, int64_t v)
 // writes item `item` (of the whole input) at output position pos; v is the
-// index of its value in Marks::vals.  A warp takes a run of whole tiles, 1,024
-// items (a word per lane) at a step; only the first sum over the tiles before
-// a block's needs the whole block.  Bound by instructions: where few items of
-// a step are selected, each lane writes its own word's (neighbouring lanes
-// write neighbouring positions, so a store still covers few lines); where
-// many are, they are listed in shared memory first and written from there,
-// one line per store.
+// index of its value in Marks::vals.  A warp takes a run of whole tiles, up to
+// 1,024 items (a word per lane) at a step: several short tiles, or a part of
+// a long one.  Only the first sum over the tiles before a block's needs the
+// whole block.  Bound by instructions: where few items of a step are
+// selected, each lane writes its own word's (neighbouring lanes write
+// neighbouring positions, so a store still covers few lines); where many are,
+// the warp takes the words one after another, a lane per item.
 template <class Emit>
 __global__ void __launch_bounds__(kExpandThreads, 2) expand_kernel(const Emit em, const Marks mk, int64_t first_item,
                                                                    const unsigned long long* __restrict__ run_in,
                                                                    unsigned long long* __restrict__ run_out,
                                                                    unsigned long long* __restrict__ total) {
   constexpr int W = kExpandThreads / 32;
-  extern __shared__ uint16_t s_list[];  // [W][1024]
   __shared__ unsigned long long s_sum[W];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
   const int per = (mk.n_tiles + gridDim.x * W - 1) / (gridDim.x * W);  // tiles per warp
   const int b0 = min(static_cast<int>(blockIdx.x) * W * per, mk.n_tiles);
   unsigned long long s = 0;
@@ -304,11 +304,14 @@ __global__ void __launch_bounds__(kExpandThreads, 2) expand_kernel(const Emit em
   s = s_sum[lane] + (run_in && lane == 0 ? *run_in : 0ull);
   for (int t = b0 + lane; t < t0; t += 32) s += __ldg(mk.counts + t);
   int64_t base = warp_sum_i64(static_cast<int64_t>(s));
-  uint16_t* list = s_list + warp * 1024;
-  for (int t = t0; t < t1; ++t) {
+  const int wpt = mk.tile >> 5;                      // words per tile
+  const int tps = wpt <= 32 ? 32 / wpt : 1;          // tiles per step, one when a tile takes several steps
+  const int head = wpt <= 32 ? lane / wpt * wpt : 0; // lane of the first word of this lane's tile
+  for (int t = t0; t < t1; t += tps) {
     const int64_t tb = static_cast<int64_t>(t) * mk.tile;
-    const int len = static_cast<int>(tb + mk.tile < mk.n ? mk.tile : mk.n - tb);
-    int64_t v = tb;
+    const int64_t span = static_cast<int64_t>(min(tps, t1 - t)) * mk.tile;
+    const int len = static_cast<int>(tb + span < mk.n ? span : mk.n - tb);
+    int64_t v = tb + 32 * head;  // next value of this lane's tile
     for (int r = 0; r < len; r += 1024) {
       uint32_t word = r + 32 * lane < len ? __ldg(mk.bits + ((tb + r) >> 5) + lane) : 0u;
       const uint32_t c = __popc(word);
@@ -318,23 +321,26 @@ __global__ void __launch_bounds__(kExpandThreads, 2) expand_kernel(const Emit em
         const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= o) inc += y;
       }
-      uint32_t at = inc - c;
+      const uint32_t before = inc - c;
+      const uint32_t in_tile = Emit::kVals ? before - __shfl_sync(0xffffffffu, before, head) : 0u;
       const int all = static_cast<int>(__shfl_sync(0xffffffffu, inc, 31));
-      if (all <= kExpandDirect) {
-        const int64_t i0 = first_item + tb + r + 32 * lane - 1;
+      const int64_t item = first_item + tb + r;
+      const int words = (min(len - r, 1024) + 31) >> 5;
+      if (all <= kExpandDirect * words) {
+        int64_t pos = base + before, vi = v + in_tile;
         while (word) {
-          em.emit(base + at, i0 + __ffs(word), Emit::kVals ? v + at : 0);
-          ++at;
+          em.emit(pos++, item + 32 * lane + __ffs(word) - 1, Emit::kVals ? vi++ : 0);
           word &= word - 1;
         }
       } else {
-        while (word) {
-          list[at++] = static_cast<uint16_t>(32 * lane + __ffs(word) - 1);
-          word &= word - 1;
+#pragma unroll 4
+        for (int w = 0; w < words; ++w) {
+          const uint32_t x = __shfl_sync(0xffffffffu, word, w);
+          const uint32_t at = __popc(x & lt);
+          const int64_t pos = base + __shfl_sync(0xffffffffu, before, w) + at;
+          const int64_t vi = Emit::kVals ? __shfl_sync(0xffffffffu, v + in_tile, w) + at : 0;
+          if ((x >> lane) & 1u) em.emit(pos, item + 32 * w + lane, vi);
         }
-        __syncwarp();
-        for (int i = lane; i < all; i += 32) em.emit(base + i, first_item + tb + r + list[i], Emit::kVals ? v + i : 0);
-        __syncwarp();
       }
       base += all;
       v += all;
@@ -392,8 +398,6 @@ int mark_and_expand(olap_ctx* ctx, Arena& ar, int64_t n, size_t val_bytes, int64
   mk.counts = counts;
   if (!mk.bits || (val_bytes && !mk.vals)) return set_error(ctx, OLAP_ERR_CAPACITY, small);
   mk.tile = static_cast<int32_t>(mark_tile(chunk, warps));
-  constexpr int smem = kExpandThreads / 32 * 1024 * static_cast<int>(sizeof(uint16_t));
-  OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(expand_kernel<Emit>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   int which = 0;
   for (int64_t first = 0; first < n; first += chunk, which ^= 1) {
     mk.n = chunk < n - first ? chunk : n - first;
@@ -402,7 +406,7 @@ int mark_and_expand(olap_ctx* ctx, Arena& ar, int64_t n, size_t val_bytes, int64
     if (rc != OLAP_OK) return rc;
     const int64_t blocks = (mk.n_tiles + kExpandThreads / 32 - 1) / (kExpandThreads / 32);
     const int64_t cap = static_cast<int64_t>(ctx->sm_count) * 2;
-    expand_kernel<Emit><<<static_cast<unsigned>(blocks < cap ? blocks : cap), kExpandThreads, smem, ctx->stream>>>(
+    expand_kernel<Emit><<<static_cast<unsigned>(blocks < cap ? blocks : cap), kExpandThreads, 0, ctx->stream>>>(
         em, mk, first, first ? run + which : nullptr, run + (which ^ 1), first + mk.n == n ? total : nullptr);
     OLAP_CUDA_TRY(ctx, cudaGetLastError());
   }
