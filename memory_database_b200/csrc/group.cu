@@ -18,7 +18,6 @@
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
-#include <vector>
 
 #include "compact.cuh"
 
@@ -584,18 +583,23 @@ __global__ void __launch_bounds__(1024) group_part_hist_kernel(PartPlan pp, cons
   }
 }
 
-// Partition starts: part_begin[p] = rows of the partitions before p
-// (part_begin[P] = all rows); cursor[p] starts at part_begin[p].  One block.
-__global__ void __launch_bounds__(1024) group_part_scan_kernel(PartPlan pp, const unsigned long long* __restrict__ ptot,
-                                                               long long* __restrict__ part_begin,
-                                                               unsigned long long* __restrict__ cursor) {
-  __shared__ long long s_run[1024];
-  const int per = (pp.n_parts + blockDim.x - 1) / blockDim.x;
-  const int b = threadIdx.x * per;
-  const int e = b + per < pp.n_parts ? b + per : pp.n_parts;
-  long long s = 0;
-  for (int i = b; i < e; ++i) s += static_cast<long long>(ptot[i]);
-  s_run[threadIdx.x] = s;
+// A slice of a partition too large for one block: its table is written whole
+// to the partial table of the slice's number, and group_part_merge_kernel adds
+// the tables of a partition's slices up.
+constexpr int kMaxPartials = 256;  // slices, and partial tables
+struct AggSlice {
+  long long begin, end;
+};
+struct AggUnits {
+  int2 merge[kMaxPartials];       // per split partition: its first slice and their number
+  AggSlice slice[kMaxPartials];
+  long long limit;                // rows of a partition up to which one block takes it whole
+  int n_slices, n_merges;
+};
+
+// Exclusive scan over the block's 1,024 threads; *total gets the sum.
+__device__ __forceinline__ long long block_scan_1024(long long v, long long* s_run, long long* total) {
+  s_run[threadIdx.x] = v;
   __syncthreads();
   for (int o = 1; o < 1024; o <<= 1) {
     const long long y = threadIdx.x >= o ? s_run[threadIdx.x - o] : 0;
@@ -603,13 +607,73 @@ __global__ void __launch_bounds__(1024) group_part_scan_kernel(PartPlan pp, cons
     s_run[threadIdx.x] += y;
     __syncthreads();
   }
-  long long run = s_run[threadIdx.x] - s;
+  const long long x = s_run[threadIdx.x] - v;
+  *total = s_run[1023];
+  __syncthreads();
+  return x;
+}
+
+// Partition starts: part_begin[p] = rows of the partitions before p
+// (part_begin[P] = all rows); cursor[p] starts at part_begin[p].  One block.
+// The partition sizes also decide the work of the aggregation's blocks here,
+// on the device, so that the host need not wait for them: a partition far
+// above the average (skewed keys) is split into slices of at most `limit`
+// rows, so no single block gets it all.
+__global__ void __launch_bounds__(1024) group_part_scan_kernel(PartPlan pp, const unsigned long long* __restrict__ ptot,
+                                                               long long* __restrict__ part_begin,
+                                                               unsigned long long* __restrict__ cursor,
+                                                               AggUnits* __restrict__ units) {
+  __shared__ long long s_run[1024];
+  const int per = (pp.n_parts + blockDim.x - 1) / blockDim.x;
+  const int b = threadIdx.x * per;
+  const int e = b + per < pp.n_parts ? b + per : pp.n_parts;
+  long long s = 0;
+  for (int i = b; i < e; ++i) s += static_cast<long long>(ptot[i]);
+  long long all;
+  long long run = block_scan_1024(s, s_run, &all);
+  const long long first = run;
   for (int i = b; i < e; ++i) {
     part_begin[i] = run;
     cursor[i] = static_cast<unsigned long long>(run);
     run += static_cast<long long>(ptot[i]);
   }
-  if (threadIdx.x == blockDim.x - 1) part_begin[pp.n_parts] = s_run[threadIdx.x];
+  if (threadIdx.x == 0) part_begin[pp.n_parts] = all;
+  // slices of `limit` rows, twice as long until there are at most kMaxPartials
+  const long long avg = (pp.n + pp.n_parts - 1) / pp.n_parts;
+  long long limit = 2 * avg > 65536 ? 2 * avg : 65536;
+  long long n_slices, mine, slices;
+  for (;; limit *= 2) {
+    mine = 0;
+    for (int i = b; i < e; ++i) {
+      const long long sz = static_cast<long long>(ptot[i]);
+      if (sz > limit) mine += (sz + limit - 1) / limit;
+    }
+    slices = block_scan_1024(mine, s_run, &n_slices);
+    if (n_slices <= kMaxPartials) break;
+  }
+  if (threadIdx.x == 0) {
+    units->limit = limit;
+    units->n_slices = static_cast<int>(n_slices);
+    units->n_merges = 0;
+  }
+  if (n_slices == 0) return;
+  long long big = 0, n_merges;
+  for (int i = b; i < e; ++i) big += static_cast<long long>(ptot[i]) > limit;
+  big = block_scan_1024(big, s_run, &n_merges);
+  if (threadIdx.x == 0) units->n_merges = static_cast<int>(n_merges);
+  run = first;
+  for (int i = b; i < e; ++i) {
+    const long long sz = static_cast<long long>(ptot[i]);
+    if (sz > limit) {
+      const int k = static_cast<int>((sz + limit - 1) / limit);
+      units->merge[big++] = make_int2(static_cast<int>(slices), k);
+      for (int q = 0; q < k; ++q) {
+        const long long lo = run + q * limit;
+        units->slice[slices++] = AggSlice{lo, lo + limit < run + sz ? lo + limit : run + sz};
+      }
+    }
+    run += sz;
+  }
 }
 
 // A partitioned row: {key, value} (8 bytes) or, with a second value
@@ -700,7 +764,6 @@ __global__ void __launch_bounds__(1024) group_part_scatter_kernel(PartPlan pp, c
 // base, the tile index its write ends at, and the carried count.
 constexpr int kScatterThreads = 512;
 constexpr int kScatterBlocks = 2;
-constexpr int kMaxPartials = 256;  // partial tables of split partitions
 
 template <bool HAS2>
 constexpr int scatter_carry() {  // rows a sector holds, less one
@@ -906,41 +969,34 @@ __device__ __forceinline__ void append_groups(const SmemAgg& st, int64_t capacit
   }
 }
 
-// A block's share of the partitioned rows: a whole partition (partial < 0:
-// its groups go straight to the outputs), or a slice of a partition too
-// large for one block (its table is written whole to partial table
-// `partial`, and group_part_merge_kernel adds the slices' tables up).
-struct AggUnit {
-  long long begin, end;
-  int32_t partial;
-  int32_t pad;
-};
-
-// One block per unit (or, with units null, per partition): aggregate the
-// rows in a shared table, then append the groups or write the partial table.
+// Blocks [0, kMaxPartials): the slices of split partitions (none in the usual
+// case: they return at once), each to its partial table.  The others: one
+// partition each, aggregated in a shared table, its groups appended to the
+// outputs; a split one is left to its slices.
 template <bool HAS2>
 __global__ void __launch_bounds__(kAggThreads) group_part_agg_kernel(
-    const long long* __restrict__ part_begin, const AggUnit* __restrict__ units,
+    const long long* __restrict__ part_begin, const AggUnits* __restrict__ units,
     const typename PartRow<HAS2>::T* __restrict__ rows, uint32_t slots, int combine, int64_t capacity,
     int32_t* __restrict__ out_keys, int64_t* __restrict__ out_sums, int64_t* __restrict__ out_counts,
     unsigned long long* d_groups, unsigned long long* overflow, int4* __restrict__ partials) {
   extern __shared__ __align__(16) unsigned char agg_smem[];
   using V = std::conditional_t<HAS2, int64_t, int32_t>;
   using Row = typename PartRow<HAS2>::T;
+  int64_t b, e;
+  int partial = -1;
+  if (blockIdx.x < kMaxPartials) {
+    partial = blockIdx.x;
+    if (partial >= units->n_slices) return;
+    b = units->slice[partial].begin;
+    e = units->slice[partial].end;
+  } else {
+    b = part_begin[blockIdx.x - kMaxPartials];
+    e = part_begin[blockIdx.x - kMaxPartials + 1];
+    if (e - b > units->limit || b == e) return;
+  }
   const SmemAgg st = smem_agg(agg_smem, slots);
   smem_agg_clear(st);
   __syncthreads();
-  int64_t b, e;
-  int partial = -1;
-  if (units) {
-    const AggUnit u = units[blockIdx.x];
-    b = u.begin;
-    e = u.end;
-    partial = u.partial;
-  } else {
-    b = part_begin[blockIdx.x];
-    e = part_begin[blockIdx.x + 1];
-  }
   unsigned int lost = 0;
   const Row* p = rows + b + threadIdx.x;
   int64_t left = e - b;
@@ -1002,16 +1058,17 @@ __global__ void __launch_bounds__(kAggThreads) group_part_agg_kernel(
   append_groups(st, capacity, out_keys, out_sums, out_counts, d_groups, overflow);
 }
 
-// One block per partition split over several units: adds up the partial
-// tables of its units (merge[b] = (first partial, count)) in a shared table
+// One block per split partition: adds up its slices' tables in a shared table
 // and appends the groups.
 __global__ void __launch_bounds__(kAggThreads) group_part_merge_kernel(
-    const int2* __restrict__ merge, const int4* __restrict__ partials, uint32_t slots, int64_t capacity,
+    const AggUnits* __restrict__ units, const int4* __restrict__ partials, uint32_t slots, int64_t capacity,
     int32_t* __restrict__ out_keys, int64_t* __restrict__ out_sums, int64_t* __restrict__ out_counts,
-    unsigned long long* d_groups, unsigned long long* overflow) {
+    unsigned long long* d_groups, unsigned long long* overflow, const unsigned long long* timeouts) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) overflow[1] = *timeouts;  // beside the overflow count, for the caller's one copy
+  if (static_cast<int>(blockIdx.x) >= units->n_merges) return;
+  const int2 m = units->merge[blockIdx.x];
   extern __shared__ __align__(16) unsigned char agg_smem[];
   const SmemAgg st = smem_agg(agg_smem, slots);
-  const int2 m = merge[blockIdx.x];
   unsigned int lost = 0;
   // the first table as it is (same layout and hash), then the slots of the
   // others, four per thread with their key lookups in flight together
@@ -1055,39 +1112,43 @@ __global__ void __launch_bounds__(kAggThreads) group_part_merge_kernel(
   append_groups(st, capacity, out_keys, out_sums, out_counts, d_groups, overflow);
 }
 
-// Compaction of the occupied slots into (key, sum, count) arrays.
-struct SlotOp {
-  static constexpr int kGroups = kCompactGroups;
-  const int32_t* keys;
-  const unsigned long long* sums;
-  const unsigned long long* counts;
-  int32_t* out_keys;
-  int64_t* out_sums;
-  int64_t* out_counts;
-  int4 k4[kCompactGroups];
-
-  __device__ __forceinline__ bool vec_ok() const { return true; }
-  __device__ __forceinline__ void prefetch(int, int64_t) {}
-  template <bool kFull>
-  __device__ __forceinline__ uint32_t flags(int u, int64_t first, int nv) {
-    int32_t k[4] = {kEmptyKey, kEmptyKey, kEmptyKey, kEmptyKey};
-    for (int j = 0; j < nv; ++j) k[j] = keys[first + j];
-    k4[u] = make_int4(k[0], k[1], k[2], k[3]);
-    uint32_t m = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) m |= static_cast<uint32_t>(k[j] != kEmptyKey) << j;
-    return m;
-  }
-  __device__ __forceinline__ void emit(int u, int j, int64_t item, int64_t pos) {
-    out_keys[pos] = j == 0 ? k4[u].x : j == 1 ? k4[u].y : j == 2 ? k4[u].z : k4[u].w;
-    out_sums[pos] = static_cast<int64_t>(sums[item]);
-    if (out_counts) out_counts[pos] = static_cast<int64_t>(counts[item]);
-  }
-};
-
-__global__ void fill_i32_kernel(int32_t* p, int64_t n, int32_t v) {
+// The global table of plan 1 empty, and the counters zero (one launch).
+__global__ void group_table_init_kernel(HashAgg t, int64_t capacity, unsigned long long* d_groups) {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = v;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < capacity; i += stride) {
+    t.keys[i] = kEmptyKey;
+    t.sums[i] = 0;
+    t.counts[i] = 0;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *d_groups = 0;
+    *t.overflow = 0;
+  }
+}
+
+// Its occupied slots to the outputs, in no particular order (a block claims
+// its positions with one atomic).
+__global__ void __launch_bounds__(256) group_table_append_kernel(HashAgg t, int64_t capacity, int32_t* __restrict__ out_keys,
+                                                                 int64_t* __restrict__ out_sums,
+                                                                 int64_t* __restrict__ out_counts,
+                                                                 unsigned long long* d_groups,
+                                                                 const unsigned long long* timeouts) {
+  __shared__ unsigned int s_n;
+  __shared__ unsigned long long s_base;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (threadIdx.x == 0) s_n = 0;
+  if (i == 0) t.overflow[1] = *timeouts;  // beside the overflow count, for the caller's one copy
+  __syncthreads();
+  const int32_t k = i < capacity ? t.keys[i] : kEmptyKey;
+  const unsigned int at = k != kEmptyKey ? atomicAdd(&s_n, 1u) : 0u;
+  __syncthreads();
+  if (threadIdx.x == 0) s_base = s_n ? atomicAdd(d_groups, static_cast<unsigned long long>(s_n)) : 0ull;
+  __syncthreads();
+  if (k == kEmptyKey) return;
+  const unsigned long long o = s_base + at;  // at most `capacity` slots are occupied
+  out_keys[o] = k;
+  out_sums[o] = static_cast<int64_t>(t.sums[i]);
+  if (out_counts) out_counts[o] = static_cast<int64_t>(t.counts[i]);
 }
 
 // SUM(price * qty * (100 + tax)) in int64 (exact modulo 2^64).
@@ -1238,9 +1299,8 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
   OLAP_REQUIRE(ctx, out_keys && out_sums && d_groups, "null output");
   OLAP_REQUIRE(ctx, n == 0 || (keys && vals), "null column");
   olap::Arena ar(ctx);
-  unsigned long long* overflow = ar.take<unsigned long long>(1);
+  unsigned long long* overflow = ar.take<unsigned long long>(2);  // overflows, wait timeouts so far
   if (!overflow) return olap::set_error(ctx, OLAP_ERR_CAPACITY, "scratch arena exhausted");
-  OLAP_CUDA_TRY(ctx, cudaMemsetAsync(overflow, 0, sizeof(unsigned long long), ctx->stream));
   int st = OLAP_OK;
   char* mem = nullptr;
   cudaError_t e = cudaSuccess;
@@ -1265,9 +1325,9 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
     t.keys = reinterpret_cast<int32_t*>(t.counts + capacity);
     t.mask = static_cast<uint64_t>(capacity - 1);
     t.overflow = overflow;
-    e = cudaMemsetAsync(mem, 0, static_cast<size_t>(capacity) * 16, ctx->stream);
-    olap::fill_i32_kernel<<<olap::grid_of(ctx, capacity, 256, 8), 256, 0, ctx->stream>>>(t.keys, capacity,
-                                                                                       olap::kEmptyKey);
+    auto* d_groups_u = reinterpret_cast<unsigned long long*>(d_groups);
+    olap::group_table_init_kernel<<<olap::grid_of(ctx, capacity, 256, 8), 256, 0, ctx->stream>>>(t, capacity,
+                                                                                                d_groups_u);
     const uint32_t slots = static_cast<uint32_t>(capacity);  // per-block table
     if (n && e == cudaSuccess && batched) {
       // The block tables fill the shared memory once the keys are many: at
@@ -1308,21 +1368,9 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
                                                       slots, combine, t,
                                                       &ctx->counters->range_errors);
     }
-    olap::SlotOp op;
-    std::memset(&op, 0, sizeof(op));
-    op.keys = t.keys;
-    op.sums = t.sums;
-    op.counts = t.counts;
-    op.out_keys = out_keys;
-    op.out_sums = out_sums;
-    op.out_counts = out_counts;
-    olap::ScanTiles sc;
     if (e == cudaSuccess)
-      st = olap::make_scan_tiles(ctx, ar, capacity, reinterpret_cast<unsigned long long*>(d_groups), ctx->stream,
-                                 &sc, olap::compact_tile_items<olap::SlotOp>());
-    if (e == cudaSuccess && st == OLAP_OK)
-      olap::compact_kernel<olap::SlotOp><<<olap::compact_grid(ctx, sc.n_tiles), olap::kCompactThreads, 0,
-                                          ctx->stream>>>(op, capacity, sc);
+      olap::group_table_append_kernel<<<static_cast<unsigned>((capacity + 255) / 256), 256, 0, ctx->stream>>>(
+          t, capacity, out_keys, out_sums, out_counts, d_groups_u, &ctx->counters->wait_timeouts);
   } else {
     // Plan 2: partition, then one block per partition.
     olap::PartPlan pp;
@@ -1375,13 +1423,11 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
     // part_begin[P + 1], then ptot[P] and cursor[P] (zeroed together)
     const size_t begin_bytes = sizeof(long long) * (3 * static_cast<size_t>(pp.n_parts) + 1);
     const size_t row_bytes = vals2 ? 16 : 8;
-    // after the rows: the work units, the merge list and the partial tables
+    // after the rows: the slices, the merge list and the partial tables
     // of partitions too large for one block (at most kMaxPartials of them)
     const size_t rows_off = (begin_bytes + hist_bytes + 255) & ~size_t(255);
     const size_t units_off = (rows_off + static_cast<size_t>(n > 0 ? n : 1) * row_bytes + 255) & ~size_t(255);
-    const size_t max_units = static_cast<size_t>(pp.n_parts) + olap::kMaxPartials;
-    const size_t merge_off = (units_off + sizeof(olap::AggUnit) * max_units + 255) & ~size_t(255);
-    const size_t part_off = (merge_off + sizeof(int2) * static_cast<size_t>(pp.n_parts) + 255) & ~size_t(255);
+    const size_t part_off = (units_off + sizeof(olap::AggUnits) + 255) & ~size_t(255);
     const size_t bytes = part_off + static_cast<size_t>(olap::kMaxPartials) * pp.slots * 16;
     mem = olap::big_scratch(ctx, bytes);
     if (!mem) return olap::set_error(ctx, OLAP_ERR_NOMEM, "device memory for the group partitions");
@@ -1390,10 +1436,10 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
     auto* cursor = ptot + pp.n_parts;
     unsigned int* hist = reinterpret_cast<unsigned int*>(mem + begin_bytes);
     char* rowbuf = mem + rows_off;
-    auto* d_units = reinterpret_cast<olap::AggUnit*>(mem + units_off);
-    auto* d_merge = reinterpret_cast<int2*>(mem + merge_off);
+    auto* d_units = reinterpret_cast<olap::AggUnits*>(mem + units_off);
     auto* d_partials = reinterpret_cast<int4*>(mem + part_off);
     e = cudaMemsetAsync(d_groups, 0, sizeof(int64_t), ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(overflow, 0, sizeof(unsigned long long), ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(ptot, 0, sizeof(unsigned long long) * pp.n_parts, ctx->stream);
     const size_t psmem = sizeof(unsigned int) * pp.n_parts;
     if (e == cudaSuccess && psmem > 48 * 1024) {
@@ -1425,52 +1471,9 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
     if (e == cudaSuccess) {
       olap::group_part_hist_kernel<<<pp.n_blocks, 1024, psmem, ctx->stream>>>(pp, keys, hist, ptot,
                                                                               &ctx->counters->range_errors);
-      olap::group_part_scan_kernel<<<1, 1024, 0, ctx->stream>>>(pp, ptot, part_begin, cursor);
+      olap::group_part_scan_kernel<<<1, 1024, 0, ctx->stream>>>(pp, ptot, part_begin, cursor, d_units);
       auto* d_groups_u = reinterpret_cast<unsigned long long*>(d_groups);
-      // Partition sizes decide the blocks: a partition far above the average
-      // (skewed keys) is split into slices of at most `limit` rows whose
-      // partial tables are merged afterwards, so no single block gets it all.
-      std::vector<long long> pb(static_cast<size_t>(pp.n_parts) + 1);
-      e = cudaMemcpyAsync(pb.data(), part_begin, sizeof(long long) * pb.size(), cudaMemcpyDeviceToHost, ctx->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-      std::vector<olap::AggUnit> units;
-      std::vector<int2> merges;
-      if (e == cudaSuccess) {
-        const int64_t avg = (n + pp.n_parts - 1) / pp.n_parts;
-        int64_t limit = std::max<int64_t>(2 * avg, int64_t(1) << 16);
-        auto slices = [&](int64_t lim) {
-          int64_t t = 0;
-          for (int p = 0; p < pp.n_parts; ++p) {
-            const int64_t sz = pb[p + 1] - pb[p];
-            if (sz > lim) t += (sz + lim - 1) / lim;
-          }
-          return t;
-        };
-        while (slices(limit) > olap::kMaxPartials) limit *= 2;
-        int32_t np = 0;
-        for (int p = 0; p < pp.n_parts; ++p) {
-          const int64_t sz = pb[p + 1] - pb[p];
-          if (sz <= limit) continue;
-          const int64_t k = (sz + limit - 1) / limit;
-          merges.push_back(make_int2(np, static_cast<int>(k)));
-          for (int64_t q = 0; q < k; ++q) {
-            const long long lo = pb[p] + q * limit, hi = std::min<long long>(pb[p + 1], lo + limit);
-            units.push_back(olap::AggUnit{lo, hi, np++, 0});
-          }
-        }
-        if (!merges.empty()) {
-          for (int p = 0; p < pp.n_parts; ++p)
-            if (pb[p + 1] - pb[p] <= limit) units.push_back(olap::AggUnit{pb[p], pb[p + 1], -1, 0});
-          e = cudaMemcpyAsync(d_units, units.data(), sizeof(olap::AggUnit) * units.size(), cudaMemcpyHostToDevice,
-                              ctx->stream);
-          if (e == cudaSuccess)
-            e = cudaMemcpyAsync(d_merge, merges.data(), sizeof(int2) * merges.size(), cudaMemcpyHostToDevice,
-                                ctx->stream);
-        }
-      }
-      const olap::AggUnit* unit_arg = merges.empty() ? nullptr : d_units;
-      const unsigned agg_grid = merges.empty() ? static_cast<unsigned>(pp.n_parts)
-                                               : static_cast<unsigned>(units.size());
+      const unsigned agg_grid = static_cast<unsigned>(pp.n_parts + olap::kMaxPartials);
       if (vals2) {
         auto* rows = reinterpret_cast<longlong2*>(rowbuf);
         if (e == cudaSuccess && tile_g == 4) scatter_tiled(rows, olap::group_part_scatter_tiled_kernel<true, 4>);
@@ -1480,7 +1483,7 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
                                                                                           hist, cursor, rows);
         if (e == cudaSuccess)
           olap::group_part_agg_kernel<true><<<agg_grid, olap::kAggThreads, asmem, ctx->stream>>>(
-              part_begin, unit_arg, rows, pp.slots, combine, capacity, out_keys, out_sums, out_counts, d_groups_u, overflow,
+              part_begin, d_units, rows, pp.slots, combine, capacity, out_keys, out_sums, out_counts, d_groups_u, overflow,
               d_partials);
       } else {
         auto* rows = reinterpret_cast<int2*>(rowbuf);
@@ -1492,23 +1495,24 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
                                                                                            rows);
         if (e == cudaSuccess)
           olap::group_part_agg_kernel<false><<<agg_grid, olap::kAggThreads, asmem, ctx->stream>>>(
-              part_begin, unit_arg, rows, pp.slots, combine, capacity, out_keys, out_sums, out_counts, d_groups_u, overflow,
+              part_begin, d_units, rows, pp.slots, combine, capacity, out_keys, out_sums, out_counts, d_groups_u, overflow,
               d_partials);
       }
-      if (e == cudaSuccess && !merges.empty())
-        olap::group_part_merge_kernel<<<static_cast<unsigned>(merges.size()), olap::kAggThreads, asmem,
-                                        ctx->stream>>>(d_merge, d_partials, pp.slots, capacity, out_keys, out_sums,
-                                                       out_counts, d_groups_u, overflow);
+      // a split partition has at least two slices
+      if (e == cudaSuccess)
+        olap::group_part_merge_kernel<<<olap::kMaxPartials / 2, olap::kAggThreads, asmem, ctx->stream>>>(
+            d_units, d_partials, pp.slots, capacity, out_keys, out_sums, out_counts, d_groups_u, overflow,
+            &ctx->counters->wait_timeouts);
       if (e == cudaSuccess) e = cudaGetLastError();
     }
   }
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess && st == OLAP_OK) st = olap::check_cuda(ctx, e, "group_hash");
-  unsigned long long ov = 0;
-  if (st == OLAP_OK) cudaMemcpyAsync(&ov, overflow, sizeof(ov), cudaMemcpyDeviceToHost, ctx->stream);
+  unsigned long long ov[2] = {0, 0};
+  if (st == OLAP_OK) cudaMemcpyAsync(ov, overflow, sizeof(ov), cudaMemcpyDeviceToHost, ctx->stream);
   OLAP_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  if (st == OLAP_OK && ov) return olap::set_error(ctx, OLAP_ERR_CAPACITY, "group hash table full");
-  if (st == OLAP_OK) st = olap::check_timeouts(ctx, ctx->stream);
+  if (st == OLAP_OK && ov[0]) return olap::set_error(ctx, OLAP_ERR_CAPACITY, "group hash table full");
+  if (st == OLAP_OK && ov[1]) st = olap::check_timeouts(ctx, ctx->stream);
   return st;
 }
 
