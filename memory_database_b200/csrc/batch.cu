@@ -12,15 +12,17 @@
 // attributes (the input of the plain star-join).
 //
 // The batched path runs up to 64 such queries in one persistent pass over
-// the shared fact table, in two kernels:
-//  * per dimension row, a 64-bit mask of the queries whose predicate the row
-//    passes (a query that does not use the table passes every row), next to
-//    the row's group attribute: a 16-byte record, 74 MB for the four
-//    headline tables, kept hot in L2;
+// the shared fact table:
+//  * a table's filter attribute falls into one of at most 129 intervals between
+//    the queries' range ends, and all rows of an interval pass the same
+//    queries; so a batch gives each dimension row a 16-bit record, its interval
+//    and its group attribute (9.2 MB for the four headline tables), and keeps
+//    the query mask of each interval in shared memory;
 //  * over the fact rows: each row's record is probed once per table (only
-//    while some live query still uses the table), the masks are ANDed with
-//    the mask of the queries whose fact range covers the row, and only the
-//    queries left in the mask do per-query work (group id, one int64 atomic).
+//    while some live query still uses the table), the intervals' masks are
+//    ANDed with the mask of the queries whose fact range covers the row, and
+//    only the queries left in the mask do per-query work (group id, one int64
+//    atomic).
 // Per query the result is bit-identical to the plain star-join over the
 // dimension vectors that olap_build_dimvec builds for it.
 #include <algorithm>
@@ -90,15 +92,30 @@ struct BatchDesc {
   int32_t n_seg;
 };
 
-struct DimRecord {
-  unsigned long long mask;  // bit q: the row passes query q's predicate on this table
-  int32_t grp;              // group attribute
-  int32_t pad;
+// Intervals of a table's filter attribute: interval 0 lies below every query's
+// range end, interval i from cut[i - 1] on.  mask[i]: the queries whose range
+// on the table holds interval i (a query that does not use the table passes
+// every row); mask[kIntervals + i]: the same without the queries that group by
+// the table, for rows whose group attribute is no int8 code (DIM_NULL in the
+// dimension vector the plain path builds).
+constexpr int kMaxCuts = 2 * kMaxBatchQueries;
+constexpr int kIntervals = kMaxCuts + 1;
+struct BatchCuts {
+  int32_t cut[OLAP_MAX_DIMS][kMaxCuts];  // ascending, INT32_MAX after the last
+  int32_t n[OLAP_MAX_DIMS];
+  int32_t pad[OLAP_MAX_DIMS];
+  unsigned long long mask[OLAP_MAX_DIMS][2 * kIntervals];
 };
+
+// A dimension row: its interval (plus kIntervals without a group code) in the
+// low 9 bits, its group code above.
+constexpr int kRecordGroupShift = 9;
+constexpr int kBatchStagedRows = 4096;  // records of the smallest table kept in shared memory up to this many
 
 struct BatchParams {
   const int2* attrs[OLAP_MAX_DIMS];   // packed attribute records per table
-  DimRecord* rec[OLAP_MAX_DIMS];      // per-batch query masks per table
+  uint16_t* rec[OLAP_MAX_DIMS];       // per-batch records per table
+  BatchCuts* cuts;
   uint32_t dim_len[OLAP_MAX_DIMS];
   const int32_t* fk[OLAP_MAX_DIMS];
   const int32_t* m1;
@@ -127,75 +144,41 @@ __device__ __forceinline__ int64_t batch_value(int agg, int32_t x, int32_t y) {
   }
 }
 
-// Query masks of the rows of table t.
-__global__ void __launch_bounds__(256) batch_records_kernel(const BatchParams p, int t) {
-  __shared__ int32_t slo[kMaxBatchQueries], shi[kMaxBatchQueries];
-  __shared__ unsigned long long s_uses, s_grouped;
-  const BatchDesc& D = *p.desc;
-  const int nq = D.n_queries;
-  if (threadIdx.x == 0) {
-    unsigned long long u = 0, g = 0;
-    for (int q = 0; q < nq; ++q) {
-      if ((D.q[q].uses >> t) & 1) u |= 1ull << q;
-      if ((D.q[q].grouped >> t) & 1) g |= 1ull << q;
-    }
-    s_uses = u;
-    s_grouped = g;
-  }
-  for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-    slo[q] = D.q[q].lo[t];
-    shi[q] = D.q[q].hi[t];
-  }
-  __syncthreads();
-  const unsigned long long uses = s_uses, grouped = s_grouped;
-  const unsigned long long all = nq == 64 ? ~0ull : ((1ull << nq) - 1);
+// The rows' records, table blockIdx.y: the interval by binary search among the
+// cuts (64 range tests per row took 291 us for the four headline tables).
+__global__ void __launch_bounds__(256) batch_records_kernel(const BatchParams p) {
+  __shared__ int32_t s_cut[kMaxCuts];
+  const int t = blockIdx.y;
+  if (!((p.tables_used >> t) & 1)) return;
   const int64_t n = p.dim_len[t];
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += stride) {
+  int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (static_cast<int64_t>(blockIdx.x) * blockDim.x >= n) return;
+  for (int i = threadIdx.x; i < kMaxCuts; i += blockDim.x) s_cut[i] = p.cuts->cut[t][i];
+  const int nc = p.cuts->n[t];
+  __syncthreads();
+  for (; k < n; k += stride) {
     const int2 a = p.attrs[t][k];
-    // a group value that is not an int8 code is DIM_NULL in the dimension
-    // vector the plain path builds
+    int at = 0;  // cuts <= the attribute
+#pragma unroll
+    for (int w = kMaxCuts / 2; w > 0; w >>= 1)
+      if (s_cut[at + w - 1] <= a.x) at += w;
+    at += s_cut[at] <= a.x;
+    at = min(at, nc);
     const bool code_ok = static_cast<uint32_t>(a.y) < static_cast<uint32_t>(OLAP_DIM_NULL);
-    unsigned long long m = all & ~uses;
-    for (int q = 0; q < nq; ++q) {
-      const bool pass = a.x >= slo[q] && a.x < shi[q] && (code_ok || !((grouped >> q) & 1));
-      m |= static_cast<unsigned long long>(pass && ((uses >> q) & 1)) << q;
-    }
-    DimRecord r;
-    r.mask = m;
-    r.grp = a.y;
-    r.pad = 0;
-    reinterpret_cast<ulonglong2*>(p.rec[t])[k] = make_ulonglong2(r.mask, static_cast<uint32_t>(r.grp));
+    p.rec[t][k] = static_cast<uint16_t>(code_ok ? at | a.y << kRecordGroupShift : at + kIntervals);
   }
-}
-
-// Record loads.  They are asm without `volatile`, which the compiler may
-// execute where their guard does not hold, so the callers pass the record of
-// key 0 (every table has at least one) in place of a key out of range.
-__device__ __forceinline__ ulonglong2 ld_record(const DimRecord* r, uint64_t pol) {
-  ulonglong2 v;
-  asm("ld.global.nc.L2::cache_hint.v2.u64 {%0,%1}, [%2], %3;" : "=l"(v.x), "=l"(v.y) : "l"(r), "l"(pol));
-  return v;
-}
-__device__ __forceinline__ unsigned long long ld_record_mask(const DimRecord* r, uint64_t pol) {
-  unsigned long long v;
-  asm("ld.global.nc.L2::cache_hint.u64 %0, [%1], %2;" : "=l"(v) : "l"(r), "l"(pol));
-  return v;
-}
-__device__ __forceinline__ int32_t ld_record_grp(const DimRecord* r, uint64_t pol) {
-  int32_t v;
-  asm("ld.global.nc.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(v) : "l"(&r->grp), "l"(pol));
-  return v;
 }
 
 // The fact pass: persistent, 4 rows per thread per step (128-bit loads).
-// PAR = false: the tables are probed one after another, smallest first, each
-// only for the rows that still have a live query using it (up to four
-// dependent L2 round trips per step, 16-byte records).  PAR = true: every
-// used table's query mask is read in one round trip (the union of a batch's
-// predicates passes nearly every row, so the skipped probes save little),
-// then the group attributes only of the tables that a surviving query groups
-// by; more registers, so at most 512 threads per block.
+// A random read costs L1 a cycle per lane whatever its size, so the smallest
+// table's records are kept in shared memory when they are few; the others'
+// share L2 with little else.  PAR = false: the tables are probed one after
+// another, smallest first, each only for the rows that still have a live query
+// using it (up to four dependent round trips per step).  PAR = true: every used
+// table's record is read in one round trip (the union of a batch's predicates
+// passes nearly every row, so the skipped probes save little); more registers,
+// so at most 512 threads per block.
 template <bool PAR>
 __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_kernel(const BatchParams p) {
   __shared__ BatchQuery sq[kMaxBatchQueries];
@@ -205,6 +188,8 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
   __shared__ int4 s_qf[kMaxBatchQueries];  // per query: group factor at each probe position (0: not grouped)
   __shared__ int4 s_qi[kMaxBatchQueries];  // per query: {group_nums, smem_off, out_offset lo, hi}
   __shared__ unsigned int s_bad;
+  __shared__ unsigned long long s_int[OLAP_MAX_DIMS][2 * kIntervals];  // by probe position: interval -> query mask
+  __shared__ uint16_t s_rec[kBatchStagedRows];                        // the first table's records
   const BatchDesc& D = *p.desc;
   unsigned long long* const out = D.out;
   const int tid = threadIdx.x;
@@ -245,18 +230,12 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
     smask[i] = D.seg_mask[i];
   }
   if (tid == 0) s_bad = 0;
+#pragma unroll
+  for (int o = 0; o < OLAP_MAX_DIMS; ++o)
+    for (int i = tid; o < ntab && i < 2 * kIntervals; i += blockDim.x) s_int[o][i] = p.cuts->mask[tab[o]][i];
+  const bool staged = ntab > 0 && tlen[0] <= kBatchStagedRows;
+  for (uint32_t i = tid; staged && i < tlen[0]; i += blockDim.x) s_rec[i] = p.rec[tab[0]][i];
   __syncthreads();
-  // queries grouping by the table at each probe position (their factor there is not 0)
-  unsigned long long tgrp[OLAP_MAX_DIMS] = {0ull, 0ull, 0ull, 0ull};
-  if (PAR) {
-    for (int q = 0; q < nq; ++q) {
-      const int4 f = s_qf[q];
-      tgrp[0] |= static_cast<unsigned long long>(f.x != 0) << q;
-      tgrp[1] |= static_cast<unsigned long long>(f.y != 0) << q;
-      tgrp[2] |= static_cast<unsigned long long>(f.z != 0) << q;
-      tgrp[3] |= static_cast<unsigned long long>(f.w != 0) << q;
-    }
-  }
   const uint64_t pol_stream = policy_evict_first();
   const uint64_t pol_keep = policy_evict_last();
   const int agg = p.agg;
@@ -336,59 +315,44 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
       return q;
     };
     int32_t gr[OLAP_MAX_DIMS][4] = {};
+    // the record of row k in table o, read while `want` (and its key is in range)
+    auto record = [&](int o, int k, bool want) -> uint32_t {
+      const bool in = want && ((inr >> (4 * o + k)) & 1u);
+      if (o == 0 && staged) return s_rec[in ? key[0][k] : 0];
+      return in ? __ldg(p.rec[tab[o]] + key[o][k]) : 0u;
+    };
+    // its interval's queries stay (all of them where the record was not wanted)
+    auto apply = [&](int o, int k, uint32_t r, bool want) {
+      const bool in = want && ((inr >> (4 * o + k)) & 1u);
+      m[k] &= in ? s_int[o][r & ((1u << kRecordGroupShift) - 1u)] : ~0ull;
+      gr[o][k] = static_cast<int32_t>(r >> kRecordGroupShift);
+    };
     if (PAR) {
-      // every used table's query mask of the 4 rows in one round trip
-      unsigned long long tm[OLAP_MAX_DIMS][4];
+      uint32_t rec[OLAP_MAX_DIMS][4];
 #pragma unroll
       for (int o = 0; o < OLAP_MAX_DIMS; ++o) {
         if (o >= ntab) continue;
-        const unsigned long long ut = tuses[o];
-        const DimRecord* rt = p.rec[tab[o]];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const bool in = (inr >> (4 * o + k)) & 1u;
-          tm[o][k] = ((m[k] & ut) && in) ? ld_record_mask(rt + (in ? key[o][k] : 0), pol_keep) : ~0ull;
-        }
+        for (int k = 0; k < 4; ++k) rec[o][k] = record(o, k, m[k] != 0ull);
       }
 #pragma unroll
       for (int o = 0; o < OLAP_MAX_DIMS; ++o) {
         if (o >= ntab) continue;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) m[k] &= tm[o][k];
-      }
-      // group attributes where a surviving query groups by the table (and
-      // its key is in range)
-#pragma unroll
-      for (int o = 0; o < OLAP_MAX_DIMS; ++o) {
-        if (o >= ntab) continue;
-        const unsigned long long ug = tgrp[o];
-        const DimRecord* rt = p.rec[tab[o]];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const bool in = (inr >> (4 * o + k)) & 1u;
-          gr[o][k] = ((m[k] & ug) != 0ull && in) ? ld_record_grp(rt + (in ? key[o][k] : 0), pol_keep) : 0;
-        }
+        for (int k = 0; k < 4; ++k) apply(o, k, rec[o][k], m[k] != 0ull);
       }
     } else {
-      // Probe the tables, smallest first, breadth-first across the 4 rows; a
-      // table is probed for a row only while a live query of the row uses it.
+      // breadth-first across the 4 rows; a table is probed for a row only
+      // while a live query of the row uses it
 #pragma unroll
       for (int o = 0; o < OLAP_MAX_DIMS; ++o) {
         if (o >= ntab) continue;
         const unsigned long long ut = tuses[o];
-        const DimRecord* rt = p.rec[tab[o]];
-        ulonglong2 rec[4];
+        uint32_t rec[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const bool in = (inr >> (4 * o + k)) & 1u;
-          rec[k] = ((m[k] & ut) && in) ? ld_record(rt + (in ? key[o][k] : 0), pol_keep)
-                                       : make_ulonglong2(~0ull, 0ull);
-        }
+        for (int k = 0; k < 4; ++k) rec[k] = record(o, k, (m[k] & ut) != 0ull);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          m[k] &= rec[k].x;
-          gr[o][k] = static_cast<int32_t>(static_cast<uint32_t>(rec[k].y));
-        }
+        for (int k = 0; k < 4; ++k) apply(o, k, rec[k], (m[k] & ut) != 0ull);
       }
     }
     if (inr != (1u << (4 * ntab)) - 1u) {  // rare: some key out of range
@@ -441,9 +405,53 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
   if (tid == 0 && s_bad) atomicAdd(p.range_err, static_cast<unsigned long long>(s_bad));
 }
 
-// Zero the batch's outputs (their location and size come with the descriptor,
-// so a recorded graph serves any output buffer and query count).
+// Intervals of table t (one block): the queries' range ends sorted by counting
+// the smaller ones, then each interval's queries.
+__device__ __forceinline__ void batch_cuts(const BatchParams& p, int t) {
+  __shared__ int32_t s_lo[kMaxBatchQueries], s_hi[kMaxBatchQueries], s_cut[kMaxCuts];
+  __shared__ unsigned long long s_uses, s_grouped;
+  const BatchDesc& D = *p.desc;
+  const int nq = D.n_queries;
+  if (threadIdx.x == 0) s_uses = s_grouped = 0;
+  for (int i = threadIdx.x; i < kMaxCuts; i += blockDim.x) s_cut[i] = INT32_MAX;
+  __syncthreads();
+  for (int q = threadIdx.x; q < nq; q += blockDim.x) {
+    s_lo[q] = D.q[q].lo[t];
+    s_hi[q] = D.q[q].hi[t];
+    if ((D.q[q].uses >> t) & 1) atomicOr(&s_uses, 1ull << q);
+    if ((D.q[q].grouped >> t) & 1) atomicOr(&s_grouped, 1ull << q);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * nq; i += blockDim.x) {
+    const int32_t v = i < nq ? s_lo[i] : s_hi[i - nq];
+    int at = 0;
+    for (int c = 0; c < 2 * nq; ++c) {
+      const int32_t w = c < nq ? s_lo[c] : s_hi[c - nq];
+      at += w < v || (w == v && c < i);
+    }
+    s_cut[at] = v;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kMaxCuts; i += blockDim.x) p.cuts->cut[t][i] = s_cut[i];
+  if (threadIdx.x == 0) p.cuts->n[t] = 2 * nq;
+  const unsigned long long all = nq == 64 ? ~0ull : ((1ull << nq) - 1);
+  for (int i = threadIdx.x; i <= 2 * nq; i += blockDim.x) {
+    unsigned long long m = 0;
+    if (i > 0) {
+      const int32_t v = s_cut[i - 1];  // the interval's first value, when it holds any
+      for (int q = 0; q < nq; ++q) m |= static_cast<unsigned long long>(s_lo[q] <= v && v < s_hi[q]) << q;
+    }
+    m = (m & s_uses) | (all & ~s_uses);
+    p.cuts->mask[t][i] = m;
+    p.cuts->mask[t][kIntervals + i] = m & ~(s_grouped & s_uses);
+  }
+}
+
+// The tables' intervals (one block each), and zeroes in the batch's outputs
+// (their location and size come with the descriptor, so a recorded graph
+// serves any output buffer and query count).
 __global__ void batch_zero_kernel(const BatchParams p) {
+  if (blockIdx.x < OLAP_MAX_DIMS && ((p.tables_used >> blockIdx.x) & 1)) batch_cuts(p, blockIdx.x);
   const BatchDesc& D = *p.desc;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -481,7 +489,7 @@ static unsigned grid_n(const olap_ctx* ctx, int64_t n, int threads) {
 
 // Batch handle: two staging slots (pinned host and device descriptors, one
 // recorded graph each) so that one batch can be prepared while the previous
-// one runs; packed attribute records and query-mask records per table.
+// one runs; packed attributes and 16-bit records per table.
 struct olap_batch {
   olap_ctx* ctx = nullptr;
   int max_queries = 0;
@@ -496,7 +504,8 @@ struct olap_batch {
   int64_t runs = 0;
   int64_t captures = 0;                 // graphs recorded so far
   int2* attrs[OLAP_MAX_DIMS] = {};
-  olap::DimRecord* rec[OLAP_MAX_DIMS] = {};
+  uint16_t* rec[OLAP_MAX_DIMS] = {};
+  olap::BatchCuts* d_cuts[2] = {};      // device, per staging slot
   int64_t attr_len[OLAP_MAX_DIMS] = {};
   int block = olap::kBatchThreads;        // scan kernel block size (olap_batch_tune / _autotune)
   int smem_slots = olap::kBatchSmemSlots; // per-block shared accumulators
@@ -531,12 +540,14 @@ int olap_batch_create(olap_ctx* ctx, int max_queries, olap_batch** out) {
   for (int s = 0; s < 2 && ok; ++s) {
     ok &= cudaMalloc(&b->d_desc[s], sizeof(olap::BatchDesc)) == cudaSuccess;
     ok &= cudaMallocHost(&b->h_desc[s], sizeof(olap::BatchDesc)) == cudaSuccess;
+    ok &= cudaMalloc(&b->d_cuts[s], sizeof(olap::BatchCuts)) == cudaSuccess;
     ok &= cudaEventCreateWithFlags(&b->done[s], cudaEventDisableTiming) == cudaSuccess;
   }
   if (!ok) {
     cudaGetLastError();
     for (int s = 0; s < 2; ++s) {
       if (b->d_desc[s]) cudaFree(b->d_desc[s]);
+      if (b->d_cuts[s]) cudaFree(b->d_cuts[s]);
       if (b->h_desc[s]) cudaFreeHost(b->h_desc[s]);
       if (b->done[s]) cudaEventDestroy(b->done[s]);
     }
@@ -555,6 +566,7 @@ int olap_batch_destroy(olap_batch* b) {
     if (b->exec[s]) cudaGraphExecDestroy(b->exec[s]);
     if (b->graph[s]) cudaGraphDestroy(b->graph[s]);
     cudaFree(b->d_desc[s]);
+    cudaFree(b->d_cuts[s]);
     cudaFreeHost(b->h_desc[s]);
     cudaEventDestroy(b->done[s]);
   }
@@ -583,7 +595,7 @@ int olap_batch_set_dimension(olap_batch* b, int table, const int32_t* filter_att
     b->rec[table] = nullptr;
     b->attr_len[table] = 0;
     OLAP_CUDA_TRY(ctx, cudaMalloc(&b->attrs[table], sizeof(int2) * n));
-    OLAP_CUDA_TRY(ctx, cudaMalloc(&b->rec[table], sizeof(olap::DimRecord) * n));
+    OLAP_CUDA_TRY(ctx, cudaMalloc(&b->rec[table], sizeof(uint16_t) * n));
     b->attr_len[table] = n;
   }
   olap::pack_dim_attrs_kernel<<<olap::grid_n(ctx, n, 256), 256, 0, ctx->stream>>>(filter_attr, group_attr, n,
@@ -707,6 +719,7 @@ int olap_batch_run(olap_batch* b, const olap_batch_query* queries, int n_queries
   p.m2 = m2;
   p.n_rows = n_rows;
   p.desc = b->d_desc[slot];
+  p.cuts = b->d_cuts[slot];
   p.tables_used = tables;
   p.agg = agg;
   p.smem_slots = b->smem_slots;
@@ -718,9 +731,8 @@ int olap_batch_run(olap_batch* b, const olap_batch_query* queries, int n_queries
   const size_t scan_smem = sizeof(unsigned long long) * static_cast<size_t>(b->smem_slots);
   const bool par = b->parallel_probe != 0 && b->block <= 512;
   void (*scan)(const olap::BatchParams) = par ? olap::batch_scan_kernel<true> : olap::batch_scan_kernel<false>;
-  if (scan_smem > 48 * 1024)
-    OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            static_cast<int>(scan_smem)));
+  OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(scan_smem)));
   int bps = 1;
   OLAP_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, scan, b->block, scan_smem));
   const unsigned grid = static_cast<unsigned>(ctx->sm_count) * static_cast<unsigned>(bps < 1 ? 1 : bps);
@@ -733,9 +745,11 @@ int olap_batch_run(olap_batch* b, const olap_batch_query* queries, int n_queries
       olap::batch_zero_kernel<<<static_cast<unsigned>(ctx->sm_count) * 2, 512, 0, st>>>(p);
       e = cudaGetLastError();
     }
-    for (int t = 0; t < OLAP_MAX_DIMS && e == cudaSuccess; ++t) {
-      if (!((tables >> t) & 1)) continue;
-      olap::batch_records_kernel<<<olap::grid_n(ctx, b->attr_len[t], 256), 256, 0, st>>>(p, t);
+    int64_t longest = 0;
+    for (int t = 0; t < OLAP_MAX_DIMS; ++t)
+      if ((tables >> t) & 1) longest = std::max(longest, b->attr_len[t]);
+    if (e == cudaSuccess && longest) {
+      olap::batch_records_kernel<<<dim3(olap::grid_n(ctx, longest, 256), OLAP_MAX_DIMS), 256, 0, st>>>(p);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess && n_rows > 0) {
