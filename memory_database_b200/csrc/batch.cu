@@ -126,6 +126,7 @@ struct BatchParams {
   int32_t probe_order;                // 4 x 2-bit table ids, smallest table first
   int32_t agg;                        // OLAP_AGG_* of every query (one aggregate)
   int32_t smem_slots;                 // per-block shared accumulators (dynamic shared memory)
+  int32_t packed;                     // every factor and output offset fits QueryPlace
   int32_t block;                      // threads per block of the scan (part of a recorded graph)
   unsigned long long* range_err;
 };
@@ -179,14 +180,24 @@ __global__ void __launch_bounds__(256) batch_records_kernel(const BatchParams p)
 // table's record is read in one round trip (the union of a batch's predicates
 // passes nearly every row, so the skipped probes save little); more registers,
 // so at most 512 threads per block.
-template <bool PAR>
+//
+// Per surviving (row, query) one emission.  The row's group codes are the bytes
+// of one word in probe order, so with factors of 16 bits (PACK) the group id
+// is two dot products, and everything an emission needs of its query is one
+// 16-byte shared read.  A lane's rows are ascending, so its fact-range segment
+// only ever moves forward and its mask stays in registers.
+template <bool PAR, bool PACK>
 __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_kernel(const BatchParams p) {
-  __shared__ BatchQuery sq[kMaxBatchQueries];
   __shared__ int64_t sseg[kMaxSegments];
   __shared__ unsigned long long smask[kMaxSegments];
   extern __shared__ unsigned long long sacc[];  // p.smem_slots per-block accumulators
-  __shared__ int4 s_qf[kMaxBatchQueries];  // per query: group factor at each probe position (0: not grouped)
-  __shared__ int4 s_qi[kMaxBatchQueries];  // per query: {group_nums, smem_off, out_offset lo, hi}
+  // Per query: its group factor at each probe position (0: not grouped; PACK:
+  // four 16-bit ones in two words), its groups, and where they are: a shared
+  // slot, or -1 - the offset in `out` (PACK), or {smem_off, offset} (!PACK).
+  __shared__ int4 s_qf[kMaxBatchQueries];
+  __shared__ int4 s_qi[PACK ? 1 : kMaxBatchQueries];
+  constexpr int kQueue = 224;  // per warp; with the largest accumulators the block still fits an SM
+  __shared__ uint16_t s_queue[PAR ? 16 : kBatchMaxThreads / 32][kQueue];
   __shared__ unsigned int s_bad;
   __shared__ unsigned long long s_int[OLAP_MAX_DIMS][2 * kIntervals];  // by probe position: interval -> query mask
   __shared__ uint16_t s_rec[kBatchStagedRows];                        // the first table's records
@@ -215,14 +226,18 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
   }
   for (int i = tid; i < nq; i += blockDim.x) {
     const BatchQuery& Q = D.q[i];
-    sq[i] = Q;
     int32_t f[OLAP_MAX_DIMS] = {0, 0, 0, 0};
 #pragma unroll
     for (int o = 0; o < OLAP_MAX_DIMS; ++o)
       if (o < ntab && ((Q.grouped >> tab[o]) & 1)) f[o] = Q.factor[tab[o]];
-    s_qf[i] = make_int4(f[0], f[1], f[2], f[3]);
-    s_qi[i] = make_int4(static_cast<int32_t>(Q.group_nums), Q.smem_off, static_cast<int32_t>(Q.out_offset),
-                        static_cast<int32_t>(Q.out_offset >> 32));
+    if (PACK) {
+      s_qf[i] = make_int4(f[0] | f[1] << 16, f[2] | f[3] << 16, static_cast<int32_t>(Q.group_nums),
+                          Q.smem_off >= 0 ? Q.smem_off : -1 - static_cast<int32_t>(Q.out_offset));
+    } else {
+      s_qf[i] = make_int4(f[0], f[1], f[2], f[3]);
+      s_qi[i] = make_int4(static_cast<int32_t>(Q.group_nums), Q.smem_off, static_cast<int32_t>(Q.out_offset),
+                          static_cast<int32_t>(Q.out_offset >> 32));
+    }
   }
   for (int i = tid; i < p.smem_slots; i += blockDim.x) sacc[i] = 0ull;
   for (int i = tid; i < nseg; i += blockDim.x) {
@@ -242,11 +257,76 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
   const bool need_m1 = agg == OLAP_AGG_M1_PLUS_M2 || agg == OLAP_AGG_M1 || agg == OLAP_AGG_M1_TIMES_M2;
   const bool need_m2 = agg == OLAP_AGG_M1_PLUS_M2 || agg == OLAP_AGG_M2 || agg == OLAP_AGG_M1_TIMES_M2;
   unsigned int bad = 0;
+  // one (row, query) pair: the row's packed codes c4 and value v
+  auto emit = [&](int q, uint32_t c4, int64_t v) {
+    const int4 f = s_qf[q];
+    if (PACK) {
+      const uint32_t g = __dp2a_hi(static_cast<uint32_t>(f.y), c4, __dp2a_lo(static_cast<uint32_t>(f.x), c4, 0u));
+      if (g >= static_cast<uint32_t>(f.z)) {
+        ++bad;
+      } else if (f.w >= 0) {
+        smem_add_split(reinterpret_cast<uint32_t*>(sacc), p.smem_slots, f.w + g, static_cast<uint64_t>(v));
+      } else {
+        atomicAdd(&out[static_cast<int64_t>(-1 - f.w) + g], static_cast<unsigned long long>(v));
+      }
+    } else {
+      const int4 qi = s_qi[q];
+      const int32_t g = static_cast<int32_t>(c4 & 255u) * f.x + static_cast<int32_t>((c4 >> 8) & 255u) * f.y +
+                        static_cast<int32_t>((c4 >> 16) & 255u) * f.z + static_cast<int32_t>(c4 >> 24) * f.w;
+      if (static_cast<uint32_t>(g) >= static_cast<uint32_t>(qi.x)) {
+        ++bad;
+      } else if (qi.y >= 0) {
+        smem_add_split(reinterpret_cast<uint32_t*>(sacc), p.smem_slots, qi.y + g, static_cast<uint64_t>(v));
+      } else {
+        const int64_t base = (static_cast<int64_t>(qi.w) << 32) | static_cast<uint32_t>(qi.z);
+        atomicAdd(&out[base + g], static_cast<unsigned long long>(v));
+      }
+    }
+  };
+  // The warp's 32 rows of one register slot: (row, query) pairs listed in
+  // shared memory, then emitted 32 at a time with every lane busy.  (Each lane
+  // emitting its own row's queries left 3 lanes busy on average: a row has
+  // about one query, but some row of the 32 has four.)
+  const int lane = tid & 31;
+  uint16_t* queue = s_queue[tid >> 5];
+  auto emit_rows = [&](unsigned long long mk, uint32_t c4, int32_t x, int32_t y) {
+    uint32_t lo = static_cast<uint32_t>(mk), hi = static_cast<uint32_t>(mk >> 32);
+    const int cnt = __popc(lo) + __popc(hi);
+    int inc = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int z = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += z;
+    }
+    const int all = __shfl_sync(0xffffffffu, inc, 31);
+    if (all > kQueue) {  // more than the list holds
+      const int64_t v = batch_value(agg, x, y);
+      for (; lo; lo &= lo - 1) emit(__ffs(lo) - 1, c4, v);
+      for (; hi; hi &= hi - 1) emit(__ffs(hi) + 31, c4, v);
+      __syncwarp();
+      return;
+    }
+    uint16_t* at = queue + (inc - cnt);
+    for (; lo; lo &= lo - 1) *at++ = static_cast<uint16_t>(lane << 6 | (__ffs(lo) - 1));
+    for (; hi; hi &= hi - 1) *at++ = static_cast<uint16_t>(lane << 6 | (__ffs(hi) + 31));
+    __syncwarp();
+    for (int b = 0; b < all; b += 32) {
+      const uint32_t e = b + lane < all ? queue[b + lane] : 0u;
+      const uint32_t c = __shfl_sync(0xffffffffu, c4, e >> 6);
+      const int32_t xs = __shfl_sync(0xffffffffu, x, e >> 6), ys = __shfl_sync(0xffffffffu, y, e >> 6);
+      if (b + lane < all) emit(static_cast<int>(e & 63u), c, batch_value(agg, xs, ys));
+    }
+    __syncwarp();
+  };
   const int64_t n4 = (p.n_rows + 3) >> 2;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + tid; i < n4; i += stride) {
+  int seg = 0;                                           // segment of the step's first row
+  int64_t seg_end = nseg > 1 ? sseg[1] : INT64_MAX;      // where it ends
+  unsigned long long seg_mask = smask[0];
+  // every lane of a warp runs the same steps (one past the end has no rows)
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + tid; i - lane < n4; i += stride) {
     const int64_t r0 = 4 * i;
-    const int nv = r0 + 4 <= p.n_rows ? 4 : static_cast<int>(p.n_rows - r0);
+    const int nv = r0 + 4 <= p.n_rows ? 4 : r0 < p.n_rows ? static_cast<int>(p.n_rows - r0) : 0;
     const bool full = nv == 4;
     // Arrays are indexed by probe position o (table t = tab[o]), so that
     // every index is a compile-time constant.
@@ -268,7 +348,8 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
         const int4 v = ld_stream_v4(p.m1 + r0, pol_stream);
         x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
       } else {
-        for (int k = 0; k < nv; ++k) x[k] = p.m1[r0 + k];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = k < nv ? p.m1[r0 + k] : 0;
       }
     }
     if (need_m2) {
@@ -276,22 +357,24 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
         const int4 v = ld_stream_v4(p.m2 + r0, pol_stream);
         y[0] = v.x; y[1] = v.y; y[2] = v.z; y[3] = v.w;
       } else {
-        for (int k = 0; k < nv; ++k) y[k] = p.m2[r0 + k];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y[k] = k < nv ? p.m2[r0 + k] : 0;
       }
     }
-    // Queries whose fact range covers each row: segment of r0 by binary
-    // search, later rows step forward.
-    int lo = 0, hi = nseg - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (sseg[mid] <= r0) lo = mid; else hi = mid - 1;
+    // Queries whose fact range covers each row.
+    while (seg_end <= r0) {
+      ++seg;
+      seg_end = seg + 1 < nseg ? sseg[seg + 1] : INT64_MAX;
+      seg_mask = smask[seg];
     }
-    unsigned long long m[4];
-    int s = lo;
+    unsigned long long m[4] = {seg_mask, seg_mask, seg_mask, seg_mask};
+    if (!full || seg_end < r0 + 4) {
+      int s = seg;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      while (s + 1 < nseg && sseg[s + 1] <= r0 + k) ++s;
-      m[k] = k < nv ? smask[s] : 0ull;
+      for (int k = 0; k < 4; ++k) {
+        while (s + 1 < nseg && sseg[s + 1] <= r0 + k) ++s;
+        m[k] = k < nv ? smask[s] : 0ull;
+      }
     }
     // A key out of range drops the row for the queries that use the table;
     // the table is not probed for it, and the row counts once per such query
@@ -314,7 +397,7 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
         if (o < ntab && !((inr >> (4 * o + k)) & 1u)) q |= tuses[o];
       return q;
     };
-    int32_t gr[OLAP_MAX_DIMS][4] = {};
+    uint32_t codes[4] = {0u, 0u, 0u, 0u};  // the row's group codes, a byte per probe position
     // the record of row k in table o, read while `want` (and its key is in range)
     auto record = [&](int o, int k, bool want) -> uint32_t {
       const bool in = want && ((inr >> (4 * o + k)) & 1u);
@@ -325,7 +408,7 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
     auto apply = [&](int o, int k, uint32_t r, bool want) {
       const bool in = want && ((inr >> (4 * o + k)) & 1u);
       m[k] &= in ? s_int[o][r & ((1u << kRecordGroupShift) - 1u)] : ~0ull;
-      gr[o][k] = static_cast<int32_t>(r >> kRecordGroupShift);
+      codes[k] |= (r >> kRecordGroupShift) << (8 * o);
     };
     if (PAR) {
       uint32_t rec[OLAP_MAX_DIMS][4];
@@ -364,37 +447,17 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
       }
     }
     // Per-query work only for the queries left in each row's mask.
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      unsigned long long mk = m[k];
-      if (!mk) continue;
-      const int64_t v = batch_value(agg, x[k], y[k]);
-      while (mk) {
-        const int q = __ffsll(static_cast<long long>(mk)) - 1;
-        mk &= mk - 1;
-        // two 16-byte shared reads per emission: the query's factors by probe
-        // position (0 for tables it does not group by) and its placement
-        const int4 f = s_qf[q];
-        const int4 qi = s_qi[q];
-        const int32_t g = gr[0][k] * f.x + gr[1][k] * f.y + gr[2][k] * f.z + gr[3][k] * f.w;
-        if (static_cast<uint32_t>(g) >= static_cast<uint32_t>(qi.x)) {
-          ++bad;
-          continue;
-        }
-        if (qi.y >= 0) {
-          smem_add_split(reinterpret_cast<uint32_t*>(sacc), p.smem_slots, qi.y + g, static_cast<uint64_t>(v));
-        } else {
-          const int64_t base = (static_cast<int64_t>(qi.w) << 32) | static_cast<uint32_t>(qi.z);
-          atomicAdd(&out[base + g], static_cast<unsigned long long>(v));
-        }
-      }
-    }
+    __syncwarp();
+    emit_rows(m[0], codes[0], x[0], y[0]);
+    emit_rows(m[1], codes[1], x[1], y[1]);
+    emit_rows(m[2], codes[2], x[2], y[2]);
+    emit_rows(m[3], codes[3], x[3], y[3]);
   }
   const unsigned int wbad = __reduce_add_sync(0xffffffffu, bad);
   if ((tid & 31) == 0 && wbad) atomicAdd(&s_bad, wbad);
   __syncthreads();
   for (int q = 0; q < nq; ++q) {
-    const BatchQuery& Q = sq[q];
+    const BatchQuery& Q = D.q[q];
     if (Q.smem_off < 0) continue;
     for (int64_t g = tid; g < Q.group_nums; g += blockDim.x) {
       const unsigned long long v = smem_split_get(reinterpret_cast<const uint32_t*>(sacc), p.smem_slots,
@@ -730,7 +793,15 @@ int olap_batch_run(olap_batch* b, const olap_batch_query* queries, int n_queries
   OLAP_REQUIRE(ctx, n_rows == 0 || ((!need_m1 || m1) && (!need_m2 || m2)), "measure columns required");
   const size_t scan_smem = sizeof(unsigned long long) * static_cast<size_t>(b->smem_slots);
   const bool par = b->parallel_probe != 0 && b->block <= 512;
-  void (*scan)(const olap::BatchParams) = par ? olap::batch_scan_kernel<true> : olap::batch_scan_kernel<false>;
+  // 16-bit factors and 31-bit output offsets (every batch but extreme ones)
+  bool packed = off <= INT32_MAX;
+  for (int q = 0; q < n_queries; ++q)
+    for (int t = 0; t < OLAP_MAX_DIMS; ++t)
+      if ((D.q[q].grouped >> t) & 1) packed &= D.q[q].factor[t] >= 0 && D.q[q].factor[t] <= UINT16_MAX;
+  p.packed = packed;  // a recorded graph launches one kind of scan
+  void (*scan)(const olap::BatchParams) =
+      packed ? (par ? olap::batch_scan_kernel<true, true> : olap::batch_scan_kernel<false, true>)
+             : (par ? olap::batch_scan_kernel<true, false> : olap::batch_scan_kernel<false, false>);
   OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           static_cast<int>(scan_smem)));
   int bps = 1;
