@@ -673,6 +673,261 @@ __global__ void __launch_bounds__(V == 8 ? 512 : 1024, 1) starjoin_vec_kernel(co
   finish_block<ACC>(p, tot0, tot1, bad, sacc, nacc, red, &red_bad);
 }
 
+// The plain scan (4 rows per thread and step, loads straight to registers).
+// Bound by instructions first and by DRAM second, so
+//  * a row is dropped without a branch: its largest code (`top`) stays DIM_NULL,
+//    and from then on it reads entry 0 of the vectors in L2, one line for all
+//    such rows;
+//  * the measures of a step are read only for the lanes that have a surviving
+//    row, when few lanes of the warp had one in the step before (kLateLanes):
+//    at 1 % survivors that leaves 17 of the 24 bytes per row.  They arrive
+//    while the next step's rows are probed and are added up there, so no step
+//    waits for them; with more survivors they are read with the keys.
+constexpr int kLateLanes = 10;
+
+template <int ND, int ACC, int AGGK>
+__global__ void __launch_bounds__(1024, 1) starjoin_scan_kernel(const StarParams p) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ long long red[32][2];
+  __shared__ unsigned int red_bad;
+  __shared__ int32_t s_code_nz[OLAP_MAX_DIMS];
+  __shared__ int32_t s_nib_ok[OLAP_MAX_DIMS];
+  unsigned char* sdim = smem;
+  unsigned long long* sacc = reinterpret_cast<unsigned long long*>(smem + p.smem_dim_bytes);
+  uint32_t* sw = reinterpret_cast<uint32_t*>(sacc);  // accumulator words: low words, then high words
+  const int tid = threadIdx.x;
+  const int64_t nacc = p.n_groups * p.n_aggs;
+  if (tid == 0) red_bad = 0;
+  if (tid < OLAP_MAX_DIMS)
+    s_code_nz[tid] = (tid < ND && p.dim[tid].code_flag >= 0) ? p.code_nonzero[p.dim[tid].code_flag] : 0;
+  if (tid < OLAP_MAX_DIMS)
+    s_nib_ok[tid] = (tid < ND && p.dim[tid].noff >= 0)
+                        ? (p.code_nonzero[OLAP_MAX_DIMS + p.dim[tid].nib_flag] == 0 ? 1 : 0)
+                        : 0;
+  stage_block<ND, ACC>(p, sdim, sacc, nacc);
+  __syncthreads();
+  uint32_t need_code = 0, nib_ok = 0;  // bit j: dimension j
+#pragma unroll
+  for (int j = 0; j < ND; ++j) {
+    need_code |= static_cast<uint32_t>(s_code_nz[j] != 0) << j;
+    nib_ok |= static_cast<uint32_t>(s_nib_ok[j] != 0) << j;
+  }
+  const uint64_t pol = policy_evict_first();
+  const uint32_t n_groups = static_cast<uint32_t>(p.n_groups);
+  int64_t tot0 = 0, tot1 = 0;
+  unsigned int bad = 0;
+  const bool need_m1 = AGGK == AGGK_GENERIC ? p.need_m1 != 0 : true;
+  const bool need_m2 = AGGK == AGGK_GENERIC ? p.need_m2 != 0 : true;
+  // One surviving row: group id check, aggregates, accumulate.
+  auto add_row = [&](uint32_t gg, int32_t x, int32_t y) {
+    if (gg >= n_groups) {
+      ++bad;
+      return;
+    }
+    int64_t v0, v1 = 0;
+    if (AGGK == AGGK_M1PM2) {
+      v0 = static_cast<int64_t>(x) + y;
+    } else if (AGGK == AGGK_M1_M1M2) {
+      v0 = x;
+      v1 = static_cast<int64_t>(x) * y;
+    } else {
+      v0 = agg_value(p.agg0, x, y);
+      v1 = p.n_aggs > 1 ? agg_value(p.agg1, x, y) : 0;
+    }
+    tot0 += v0;
+    if (ACC == ACC_SMEM) smem_add_split(sw, nacc, gg, static_cast<uint64_t>(v0));
+    if (ACC == ACC_GLOBAL) atomicAdd(&p.out[gg], static_cast<unsigned long long>(v0));
+    if (AGGK == AGGK_M1_M1M2 || (AGGK == AGGK_GENERIC && p.n_aggs > 1)) {
+      tot1 += v1;
+      if (ACC == ACC_SMEM) smem_add_split(sw, nacc, n_groups + gg, static_cast<uint64_t>(v1));
+      if (ACC == ACC_GLOBAL) atomicAdd(&p.out[n_groups + gg], static_cast<unsigned long long>(v1));
+    }
+  };
+  const uint32_t nvec = static_cast<uint32_t>((p.vec_end - p.vec_begin) >> 2);
+  const uint32_t gstride = gridDim.x * blockDim.x;
+  int4 ma = make_int4(0, 0, 0, 0), mb = ma;  // measures of the rows in hand
+  uint32_t pend = 0;                         // rows whose late measures are on their way
+  int32_t pg[4] = {0, 0, 0, 0};              // and their group ids
+  bool late = false;
+  auto add_pending = [&] {
+    if (pend & 1u) add_row(static_cast<uint32_t>(pg[0]), ma.x, mb.x);
+    if (pend & 2u) add_row(static_cast<uint32_t>(pg[1]), ma.y, mb.y);
+    if (pend & 4u) add_row(static_cast<uint32_t>(pg[2]), ma.z, mb.z);
+    if (pend & 8u) add_row(static_cast<uint32_t>(pg[3]), ma.w, mb.w);
+    pend = 0;
+  };
+  // every lane of a warp runs the same steps
+  for (uint32_t w0 = blockIdx.x * blockDim.x + (tid & ~31u); w0 < nvec; w0 += gstride) {
+    const uint32_t i = w0 + (tid & 31u);
+    const bool in = i < nvec;
+    const int64_t row = p.vec_begin + 4ll * (in ? i : w0);  // a valid vector on every lane
+    int4 kf[ND > 0 ? ND : 1];
+#pragma unroll
+    for (int j = 0; j < ND; ++j) kf[j] = ld_stream_v4_ordered(p.dim[j].fk + row, pol);
+    if (pend) add_pending();
+    if (!late) {
+      ma = ld_stream_v4_if(need_m1, p.m1 + row, pol);
+      mb = ld_stream_v4_if(need_m2, p.m2 + row, pol);
+    }
+    auto key = [&](int r, int j) -> uint32_t {
+      const int4& v = kf[j];
+      return static_cast<uint32_t>(r == 0 ? v.x : r == 1 ? v.y : r == 2 ? v.z : v.w);
+    };
+    int32_t top[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) top[r] = in ? INT8_MIN : OLAP_DIM_NULL;
+    // Range check of every key.  A row with a key out of range is dropped here
+    // and its thread only marked (in the top bit of its count): whether it is a
+    // range error is decided after the loop.
+    uint32_t oob = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      bool ok = true;
+#pragma unroll
+      for (int j = 0; j < ND; ++j) ok &= key(r, j) < p.dim[j].len;
+      if (!ok) oob |= 1u << r;
+    }
+    if (oob) {
+      if (in) bad |= kMetOob;
+      // keys of dropped rows to 0, so that no probe leaves its vector
+#pragma unroll
+      for (int j = 0; j < ND; ++j) {
+        if (oob & 1u) kf[j].x = 0;
+        if (oob & 2u) kf[j].y = 0;
+        if (oob & 4u) kf[j].z = 0;
+        if (oob & 8u) kf[j].w = 0;
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if ((oob >> r) & 1u) top[r] = OLAP_DIM_NULL;
+    }
+    int32_t g[4] = {0, 0, 0, 0};
+    auto dead0 = [&](int r, int j) -> uint32_t { return top[r] == OLAP_DIM_NULL ? 0u : key(r, j); };
+    bool skip = false;  // this dimension was probed with the previous one
+#pragma unroll
+    for (int j = 0; j < ND; ++j) {
+      if (skip) {
+        skip = false;
+        continue;
+      }
+      const Probe& d = p.dim[j];
+      int32_t c[4];
+      if (d.noff >= 0 && ((nib_ok >> j) & 1u)) {
+        // 4-bit codes in shared memory (15 = DIM_NULL)
+        const uint32_t* sn = reinterpret_cast<const uint32_t*>(sdim + d.noff);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const uint32_t k = key(r, j);
+          c[r] = static_cast<int32_t>(sn[k >> 3] >> ((k << 2) & 31u)) & 15;
+          top[r] = max(top[r], c[r] + (OLAP_DIM_NULL - 15));
+          g[r] += c[r] * d.factor;
+        }
+      } else if (d.soff >= 0) {
+        const int8_t* sv = reinterpret_cast<const int8_t*>(sdim + d.soff);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) c[r] = sv[key(r, j)];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          top[r] = max(top[r], c[r]);
+          g[r] += c[r] * d.factor;
+        }
+      } else if (d.boff >= 0 || d.bits) {
+        // pass bitmap; the codes of the survivors are fetched after the filters
+        const uint32_t* sb = reinterpret_cast<const uint32_t*>(sdim + d.boff);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const uint32_t k = d.boff >= 0 ? key(r, j) : dead0(r, j);
+          const uint32_t w = d.boff >= 0 ? sb[k >> 5] : __ldg(d.bits + (k >> 5));
+          if (!((w >> (k & 31)) & 1u)) top[r] = OLAP_DIM_NULL;
+        }
+      } else {
+        // int8 probe through L2; with merge_global, the next dimension's too
+        // when it is also one (both in flight: one round trip instead of two)
+        const int j1 = j + 1 < ND ? j + 1 : j;
+        const Probe& d1 = p.dim[j1];
+        const bool two = p.merge_global && j + 1 < ND && d1.soff < 0 && d1.boff < 0 && !d1.bits &&
+                         !(d1.noff >= 0 && ((nib_ok >> j1) & 1u));
+        int32_t c1[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) c[r] = __ldg(d.vec + dead0(r, j));
+        if (two) {
+#pragma unroll
+          for (int r = 0; r < 4; ++r) c1[r] = __ldg(d1.vec + dead0(r, j1));
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          top[r] = max(top[r], c[r]);
+          g[r] += c[r] * d.factor;
+        }
+        if (two) {
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            top[r] = max(top[r], c1[r]);
+            g[r] += c1[r] * d1.factor;
+          }
+          skip = true;
+        }
+      }
+    }
+    uint32_t alive = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) alive |= static_cast<uint32_t>(top[r] != OLAP_DIM_NULL) << r;
+    const int lanes = __popc(__ballot_sync(0xffffffffu, alive != 0));
+    if (lanes) {
+#pragma unroll
+      for (int j = 0; j < ND; ++j) {
+        if (p.dim[j].soff < 0 && p.dim[j].bits && ((need_code >> j) & 1u)) {
+#pragma unroll
+          for (int r = 0; r < 4; ++r) g[r] += __ldg(p.dim[j].vec + dead0(r, j)) * p.dim[j].factor;
+        }
+      }
+      pend = alive;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) pg[r] = g[r];
+      if (late) {
+        ma = ld_stream_v4_if(need_m1 && alive, p.m1 + row, pol);
+        mb = ld_stream_v4_if(need_m2 && alive, p.m2 + row, pol);
+      } else {
+        add_pending();
+      }
+    }
+    late = lanes <= kLateLanes;
+  }
+  if (pend) add_pending();
+  if (bad & kMetOob) {  // rare: this thread's rows once more, for the range errors among them
+    bad &= ~kMetOob;
+    for (uint64_t i = blockIdx.x * blockDim.x + tid; i < nvec; i += gstride)
+      for (int c = 0; c < 4; ++c) bad += range_error_row<ND>(p, p.vec_begin + 4 * static_cast<int64_t>(i) + c);
+  }
+  // Head and tail rows outside the 16-byte aligned range (block 0).
+  if (blockIdx.x == 0) {
+    auto one = [&](int64_t r) {
+      uint32_t k[ND > 0 ? ND : 1];
+      bool ok = true;
+#pragma unroll
+      for (int j = 0; j < ND; ++j) {
+        k[j] = static_cast<uint32_t>(p.dim[j].fk[r]);
+        ok &= k[j] < p.dim[j].len;
+      }
+      if (!ok) {
+        bad += range_error_row<ND>(p, r);
+        return;
+      }
+      int32_t g = 0;  // the host checked that it fits
+#pragma unroll
+      for (int j = 0; j < ND; ++j) {
+        const int32_t c = p.dim[j].soff >= 0 ? static_cast<int8_t>(sdim[p.dim[j].soff + k[j]]) : p.dim[j].vec[k[j]];
+        if (c == OLAP_DIM_NULL) return;
+        g += c * p.dim[j].factor;
+      }
+      add_row(static_cast<uint32_t>(g), p.need_m1 ? p.m1[r] : 0, p.need_m2 ? p.m2[r] : 0);
+    };
+    for (int64_t r = p.row_begin + tid; r < p.vec_begin; r += blockDim.x) one(r);
+    for (int64_t r = p.vec_end + tid; r < p.row_end; r += blockDim.x) one(r);
+  }
+  finish_block<ACC>(p, tot0, tot1, bad, sacc, nacc, red, &red_bad);
+}
+
 // Generic path: one row per thread step, 32-bit loads, int64 group ids.  Used
 // for columns that are not 16-byte aligned and for plans whose group-id
 // arithmetic could leave int32.
@@ -758,8 +1013,19 @@ __global__ void __launch_bounds__(1024, 1) starjoin_scalar_kernel(const StarPara
 
 using StarKernel = void (*)(const StarParams);
 
+// 4 rows per thread without prefetch: the plain scan.
+template <int ND, int ACC>
+static StarKernel pick_scan(int aggk) {
+  switch (aggk) {
+    case AGGK_M1PM2: return starjoin_scan_kernel<ND, ACC, AGGK_M1PM2>;
+    case AGGK_M1_M1M2: return starjoin_scan_kernel<ND, ACC, AGGK_M1_M1M2>;
+    default: return starjoin_scan_kernel<ND, ACC, AGGK_GENERIC>;
+  }
+}
+
 template <int ND, int ACC, bool ASYNC>
 static StarKernel pick_vec_a(int aggk, int v) {
+  if (v < 8 && !ASYNC) return pick_scan<ND, ACC>(aggk);
   if (v >= 8) {
     switch (aggk) {
       case AGGK_M1PM2: return starjoin_vec_kernel<ND, ACC, AGGK_M1PM2, 8, ASYNC, false>;
@@ -768,9 +1034,9 @@ static StarKernel pick_vec_a(int aggk, int v) {
     }
   }
   switch (aggk) {
-    case AGGK_M1PM2: return starjoin_vec_kernel<ND, ACC, AGGK_M1PM2, 4, ASYNC, false>;
-    case AGGK_M1_M1M2: return starjoin_vec_kernel<ND, ACC, AGGK_M1_M1M2, 4, ASYNC, false>;
-    default: return starjoin_vec_kernel<ND, ACC, AGGK_GENERIC, 4, ASYNC, false>;
+    case AGGK_M1PM2: return starjoin_vec_kernel<ND, ACC, AGGK_M1PM2, 4, true, false>;
+    case AGGK_M1_M1M2: return starjoin_vec_kernel<ND, ACC, AGGK_M1_M1M2, 4, true, false>;
+    default: return starjoin_vec_kernel<ND, ACC, AGGK_GENERIC, 4, true, false>;
   }
 }
 
