@@ -10,9 +10,9 @@
 // Here the sum is int64 fixed point: SUM price_cents * (100 - discount_pct),
 // exactly 100 x 100 x the decimal revenue.
 //
-// Three passes: suppliers -> int8 nation vector and its 4-bit codes (staged
-// in shared memory by the line pass), orders -> int8 nation vector (one byte per order,
-// L2-resident for the line pass), lines -> per-nation int64 sums in shared
+// Three passes: suppliers -> int8 code vector and its 4-bit form (staged in
+// shared memory by the line pass), orders -> int8 code vector (one byte per
+// order, L2-resident for the line pass), lines -> per-nation int64 sums in shared
 // memory, flushed once per block.  Customer and supplier keys are 1-based as
 // in the reference; orders are addressed by row (l_orderkey_new).
 #include <algorithm>
@@ -29,47 +29,49 @@ __device__ __forceinline__ bool nation_ok(uint64_t mask, int32_t n) {
   return static_cast<uint32_t>(n) < kQ5MaxNations && ((mask >> n) & 1ull);
 }
 
-// set_bitmap + nation -> region: bit n set when nation n's region has key `region`.
-__global__ void q5_nation_mask_kernel(const int32_t* __restrict__ r_regionkey, int64_t n_region,
-                                      const int32_t* __restrict__ n_regionkey, int64_t n_nation, int32_t region,
-                                      unsigned long long* __restrict__ mask) {
+// What the supplier and order vectors hold for nation n: -1 when its region does
+// not pass, else its rank among the region's nations (equal ranks are equal
+// nations, and up to 15 of them fit 4 bits), or the nation itself in a region
+// of more than 15.
+constexpr int kQ5MaxCodes = 15;
+__device__ __forceinline__ int32_t q5_code(uint64_t mask, bool ranks, int32_t n) {
+  if (!nation_ok(mask, n)) return -1;
+  return ranks ? __popcll(mask & ((1ull << n) - 1ull)) : n;
+}
+
+// Before the passes, in one launch: the region's nations as a bit mask
+// (set_bitmap, every block for itself, block 0 for the later kernels), the
+// supplier vector and its 4-bit codes (two suppliers per thread, 15 = none; of
+// use while the region has at most 15 nations), and zeroes in the sums.
+__global__ void __launch_bounds__(256) q5_prepare_kernel(const int32_t* __restrict__ r_regionkey, int64_t n_region,
+                                                         const int32_t* __restrict__ n_regionkey, int64_t n_nation,
+                                                         int32_t region, const int32_t* __restrict__ s_nationkey,
+                                                         int64_t n_supp, unsigned long long* __restrict__ d_mask,
+                                                         int8_t* __restrict__ dim_s, uint8_t* __restrict__ nib,
+                                                         unsigned long long* __restrict__ sums) {
+  __shared__ unsigned int s_half[2];
   const int n = threadIdx.x;
-  const bool ok = n < n_nation && n_regionkey[n] >= 0 && n_regionkey[n] < n_region &&
-                  r_regionkey[n_regionkey[n]] == region;
-  __shared__ unsigned long long s[2];
-  const unsigned int b = __ballot_sync(0xffffffffu, ok);
-  if ((n & 31) == 0) s[n >> 5] = b;
-  __syncthreads();
-  if (n == 0) *mask = s[0] | (s[1] << 32);
-}
-
-__global__ void q5_supplier_kernel(const int32_t* __restrict__ s_nationkey, int64_t n_supp,
-                                   const unsigned long long* __restrict__ d_mask, int8_t* __restrict__ dim_s) {
-  const uint64_t nmask = *d_mask;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_supp; i += stride) {
-    const int32_t n = s_nationkey[i];
-    dim_s[i] = nation_ok(nmask, n) ? static_cast<int8_t>(n) : static_cast<int8_t>(-1);
+  if (n < kQ5MaxNations) {
+    const bool ok = n < n_nation && n_regionkey[n] >= 0 && n_regionkey[n] < n_region &&
+                    r_regionkey[n_regionkey[n]] == region;
+    const unsigned int b = __ballot_sync(0xffffffffu, ok);
+    if ((n & 31) == 0) s_half[n >> 5] = b;
   }
-}
-
-// 4-bit codes of the supplier nations for the line pass: code c < 15 is the
-// c-th nation of the region's mask, 15 none.  Exact when the region has at
-// most 15 nations; the line pass checks that before it uses them.
-__global__ void q5_supplier_nib_kernel(const int8_t* __restrict__ dim_s, int64_t n_supp,
-                                       const unsigned long long* __restrict__ d_mask, uint8_t* __restrict__ nib) {
-  const uint64_t nmask = *d_mask;
-  auto code = [&](int32_t n) -> uint32_t {
-    if (n < 0) return 15u;
-    const uint32_t c = static_cast<uint32_t>(__popcll(nmask & ((1ull << n) - 1ull)));
-    return c < 15u ? c : 15u;
-  };
+  __syncthreads();
+  const uint64_t nmask = s_half[0] | (static_cast<uint64_t>(s_half[1]) << 32);
+  const bool ranks = __popcll(nmask) <= kQ5MaxCodes;
+  if (blockIdx.x == 0) {
+    if (n == 0) *d_mask = nmask;
+    if (n < n_nation) sums[n] = 0;
+  }
   const int64_t nbytes = (n_supp + 1) >> 1;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < nbytes; i += stride) {
-    const uint32_t lo = code(dim_s[2 * i]);
-    const uint32_t hi = 2 * i + 1 < n_supp ? code(dim_s[2 * i + 1]) : 15u;
-    nib[i] = static_cast<uint8_t>(lo | (hi << 4));
+    const int32_t lo = q5_code(nmask, ranks, s_nationkey[2 * i]);
+    const int32_t hi = 2 * i + 1 < n_supp ? q5_code(nmask, ranks, s_nationkey[2 * i + 1]) : -1;
+    dim_s[2 * i] = static_cast<int8_t>(lo);
+    if (2 * i + 1 < n_supp) dim_s[2 * i + 1] = static_cast<int8_t>(hi);
+    nib[i] = static_cast<uint8_t>((lo & 15) | (hi & 15) << 4);
   }
 }
 
@@ -77,7 +79,14 @@ __global__ void q5_orders_kernel(const int32_t* __restrict__ o_custkey, const in
                                  int64_t n_orders, const int32_t* __restrict__ c_nationkey, int64_t n_cust,
                                  const unsigned long long* __restrict__ d_mask, int32_t date1, int32_t date2,
                                  int8_t* __restrict__ dim_o, unsigned long long* range_err) {
-  const uint64_t nmask = *d_mask;
+  __shared__ int8_t s_code[kQ5MaxNations];  // by nation: 25 us per 15M orders; 34 us with the rank counted per order
+  if (threadIdx.x < kQ5MaxNations) {
+    const uint64_t nmask = *d_mask;
+    s_code[threadIdx.x] =
+        static_cast<int8_t>(q5_code(nmask, __popcll(nmask) <= kQ5MaxCodes, static_cast<int32_t>(threadIdx.x)));
+  }
+  __syncthreads();
+  auto code = [&](int32_t n) -> int32_t { return static_cast<uint32_t>(n) < kQ5MaxNations ? s_code[n] : -1; };
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const uint64_t pol = policy_evict_first();
@@ -89,7 +98,7 @@ __global__ void q5_orders_kernel(const int32_t* __restrict__ o_custkey, const in
         ++bad;
       } else {
         const int32_t n = __ldg(c_nationkey + (c - 1));
-        if (nation_ok(nmask, n)) v = static_cast<int8_t>(n);
+        v = static_cast<int8_t>(code(n));
       }
     }
     dim_o[i] = v;
@@ -112,7 +121,7 @@ __global__ void q5_orders_kernel(const int32_t* __restrict__ o_custkey, const in
     uint32_t packed = 0;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const int8_t v = (n[e] >= 0 && nation_ok(nmask, n[e])) ? static_cast<int8_t>(n[e]) : static_cast<int8_t>(-1);
+      const int8_t v = static_cast<int8_t>(code(n[e]));
       packed |= static_cast<uint32_t>(static_cast<uint8_t>(v)) << (8 * e);
     }
     reinterpret_cast<uint32_t*>(dim_o)[i] = packed;
@@ -121,91 +130,98 @@ __global__ void q5_orders_kernel(const int32_t* __restrict__ o_custkey, const in
   if (bad) atomicAdd(range_err, static_cast<unsigned long long>(bad));
 }
 
-// stage_s: 0 probes the int8 supplier vector through L1/L2; 2 stages the
-// 4-bit codes in shared memory (half the bytes of the int8 vector, so more
-// blocks fit an SM), and falls back to 0 when the region has more than 15
-// nations.
-__global__ void __launch_bounds__(512, 3) q5_lines_kernel(const int32_t* __restrict__ l_suppkey,
-                                                       const int32_t* __restrict__ l_order,
-                                                       const int32_t* __restrict__ price,
-                                                       const int32_t* __restrict__ disc, int64_t n_lines,
-                                                       const int8_t* __restrict__ dim_s, int64_t n_supp,
-                                                       const uint8_t* __restrict__ nib_s,
-                                                       const unsigned long long* __restrict__ d_mask,
-                                                       const int8_t* __restrict__ dim_o, int64_t n_orders,
-                                                       unsigned long long* __restrict__ sums,
-                                                       unsigned long long* range_err, int stage_s) {
-  extern __shared__ int8_t s_dim[];  // staged supplier nations or their 4-bit codes (stage_s)
-  __shared__ unsigned long long s_sum[kQ5MaxNations];
-  __shared__ int8_t s_nat[16];       // 4-bit code -> nation
+// Price and discount are read only for the lines that match (a fifth of the
+// suppliers, a seventh of the orders and equal nations leave about one in
+// 175): two thirds of their sectors are never read.
+// kStaged: the 4-bit supplier codes in shared memory (half the bytes of the
+// int8 vector, so four blocks fit an SM), unless the region has more than 15
+// nations; else the int8 vector through L1/L2.  Lines that drop out
+// are carried along without a branch, and codes are compared, not nations.
+// Bound by the order gathers' sectors and by instructions: 60M lines, 100,000
+// suppliers, 173 us (all four columns read, branches, nations) -> 151 us (late
+// reads) -> 115 us.
+template <bool kStaged>
+__global__ void __launch_bounds__(512, 4) q5_lines_kernel(
+    const int32_t* __restrict__ l_suppkey, const int32_t* __restrict__ l_order, const int32_t* __restrict__ price,
+    const int32_t* __restrict__ disc, int64_t n_lines, const int8_t* __restrict__ dim_s, int64_t n_supp,
+    const uint8_t* __restrict__ nib_s, const unsigned long long* __restrict__ d_mask,
+    const int8_t* __restrict__ dim_o, int64_t n_orders, unsigned long long* __restrict__ sums,
+    unsigned long long* range_err) {
+  extern __shared__ __align__(16) uint32_t s_nib[];  // kStaged: eight codes per word
+  __shared__ unsigned long long s_sum[kQ5MaxNations];  // by code
+  __shared__ int8_t s_nat[kQ5MaxNations];              // code -> nation
   const int tid = threadIdx.x;
-  const uint64_t nmask = stage_s == 2 ? *d_mask : 0ull;
-  const int mode = stage_s == 2 && __popcll(nmask) > 15 ? 0 : stage_s;
-  for (int i = tid; i < kQ5MaxNations; i += blockDim.x) s_sum[i] = 0;
-  if (mode == 2 && tid < 16) {
-    // the tid-th set bit of the mask
-    uint64_t m = nmask;
-    for (int k = 0; k < tid && m; ++k) m &= m - 1;
-    s_nat[tid] = m ? static_cast<int8_t>(__ffsll(static_cast<long long>(m)) - 1) : static_cast<int8_t>(-1);
+  const uint64_t nmask = *d_mask;
+  const bool ranks = __popcll(nmask) <= kQ5MaxCodes;
+  const bool staged = kStaged && ranks;
+  for (int i = tid; i < kQ5MaxNations; i += blockDim.x) {
+    s_sum[i] = 0;
+    if (!ranks) s_nat[i] = static_cast<int8_t>(i);
+    else if (nation_ok(nmask, i)) s_nat[q5_code(nmask, true, i)] = static_cast<int8_t>(i);
   }
-  if (mode == 2)
-    for (int64_t i = tid; i < ((n_supp + 1) >> 1); i += blockDim.x) s_dim[i] = static_cast<int8_t>(nib_s[i]);
+  if (staged) {
+    const int64_t nbytes = (n_supp + 1) >> 1;
+    for (int64_t i = tid; i < (nbytes >> 2); i += blockDim.x) s_nib[i] = __ldg(reinterpret_cast<const uint32_t*>(nib_s) + i);
+    for (int64_t i = (nbytes & ~int64_t(3)) + tid; i < nbytes; i += blockDim.x) reinterpret_cast<uint8_t*>(s_nib)[i] = nib_s[i];
+  }
   __syncthreads();
-  // nation of supplier row s (0-based), -1 when it is not in the region
-  auto snation = [&](int32_t s) -> int32_t {
-    if (mode == 2) {
-      const uint32_t c = (static_cast<uint8_t>(s_dim[s >> 1]) >> ((s & 1) << 2)) & 15u;
-      return c == 15u ? -1 : s_nat[c];
-    }
-    return dim_s[s];
+  // code of supplier row s (0-based): 15 or -1 when it is not in the region
+  auto scode = [&](uint32_t s) -> int32_t {
+    return staged ? static_cast<int32_t>(s_nib[s >> 3] >> ((s << 2) & 31u)) & 15 : __ldg(dim_s + s);
   };
+  const int32_t none = staged ? 15 : -1;
+  const uint32_t n_s = static_cast<uint32_t>(n_supp < INT32_MAX ? n_supp : INT32_MAX);
+  const uint32_t n_o = static_cast<uint32_t>(n_orders < INT32_MAX ? n_orders : int64_t(INT32_MAX) + 1);
   const uint64_t pol = policy_evict_first();
   const uint64_t keep = policy_evict_last();
   unsigned int bad = 0;
-  auto one = [&](int32_t sk, int32_t ok, int32_t p, int32_t dc) {
-    const bool in = sk >= 1 && sk <= n_supp && ok >= 0 && ok < n_orders;
-    if (!in) {
-      ++bad;
-      return;
-    }
-    const int32_t ns = snation(sk - 1);
-    if (ns < 0) return;
-    const int32_t no = static_cast<int8_t>(ld_probe_s8_if(in, dim_o + ok, keep, -2));
-    if (no != ns) return;
-    smem_add_u64(&s_sum[ns], static_cast<uint64_t>(static_cast<int64_t>(p) * (100 - dc)));
+  auto add = [&](int32_t code, int64_t r) {
+    smem_add_u64(&s_sum[code], static_cast<uint64_t>(static_cast<int64_t>(__ldg(price + r)) * (100 - __ldg(disc + r))));
   };
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + tid;
-  const bool vec = ((reinterpret_cast<uintptr_t>(l_suppkey) | reinterpret_cast<uintptr_t>(l_order) |
-                     reinterpret_cast<uintptr_t>(price) | reinterpret_cast<uintptr_t>(disc)) & 15) == 0;
-  const int64_t n4 = vec ? n_lines >> 2 : 0;
+  const bool vec = ((reinterpret_cast<uintptr_t>(l_suppkey) | reinterpret_cast<uintptr_t>(l_order)) & 15) == 0;
+  const int64_t n4 = vec && n_s && n_o ? n_lines >> 2 : 0;
   for (int64_t i = t0; i < n4; i += stride) {
-    const int4 a = ld_stream_v4(l_suppkey + 4 * i, pol), b = ld_stream_v4(l_order + 4 * i, pol);
-    const int4 c = ld_stream_v4(price + 4 * i, pol), d = ld_stream_v4(disc + 4 * i, pol);
-    // The four lines in stages, so that their order-vector gathers are in
-    // flight together: supplier nation, then order nation, then the sums.
-    const int32_t sk[4] = {a.x, a.y, a.z, a.w}, ok[4] = {b.x, b.y, b.z, b.w};
-    const int32_t pr[4] = {c.x, c.y, c.z, c.w}, dc[4] = {d.x, d.y, d.z, d.w};
-    int32_t ns[4], no[4];
+    const int4 a = ld_stream_v4_ordered(l_suppkey + 4 * i, pol), b = ld_stream_v4_ordered(l_order + 4 * i, pol);
+    // 0-based supplier, order; the four lines in stages, so that their
+    // order-vector gathers are in flight together
+    uint32_t sk[4] = {static_cast<uint32_t>(a.x) - 1u, static_cast<uint32_t>(a.y) - 1u, static_cast<uint32_t>(a.z) - 1u,
+                      static_cast<uint32_t>(a.w) - 1u};
+    uint32_t ok[4] = {static_cast<uint32_t>(b.x), static_cast<uint32_t>(b.y), static_cast<uint32_t>(b.z),
+                      static_cast<uint32_t>(b.w)};
+    uint32_t out = 0;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      ns[e] = -1;
-      if (sk[e] < 1 || sk[e] > n_supp || ok[e] < 0 || ok[e] >= n_orders) ++bad;
-      else ns[e] = snation(sk[e] - 1);
+    for (int e = 0; e < 4; ++e) out |= static_cast<uint32_t>(sk[e] >= n_s || ok[e] >= n_o) << e;
+    if (out) {  // rare: keys to 0, so that no read leaves its vector
+      bad += __popc(out);
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if ((out >> e) & 1u) sk[e] = ok[e] = 0u;
     }
+    int32_t cs[4], co[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) no[e] = static_cast<int8_t>(ld_probe_s8_if(ns[e] >= 0, dim_o + ok[e], keep, -2));
+    for (int e = 0; e < 4; ++e) cs[e] = scode(sk[e]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) co[e] = static_cast<int8_t>(ld_probe_s8_if(cs[e] != none, dim_o + ok[e], keep, -2));
 #pragma unroll
     for (int e = 0; e < 4; ++e)
-      if (ns[e] >= 0 && no[e] == ns[e])
-        smem_add_u64(&s_sum[ns[e]], static_cast<uint64_t>(static_cast<int64_t>(pr[e]) * (100 - dc[e])));
+      if (cs[e] == co[e] && cs[e] != none && !((out >> e) & 1u)) add(cs[e], 4 * i + e);
   }
-  for (int64_t r = 4 * n4 + t0; r < n_lines; r += stride) one(l_suppkey[r], l_order[r], price[r], disc[r]);
+  for (int64_t r = 4 * n4 + t0; r < n_lines; r += stride) {
+    const uint32_t sk = static_cast<uint32_t>(l_suppkey[r]) - 1u, ok = static_cast<uint32_t>(l_order[r]);
+    if (sk >= n_s || ok >= n_o) {
+      ++bad;
+      continue;
+    }
+    const int32_t c = scode(sk);
+    if (c != none && dim_o[ok] == c) add(c, r);
+  }
   const unsigned int wbad = __reduce_add_sync(0xffffffffu, bad);
   if ((tid & 31) == 0 && wbad) atomicAdd(range_err, static_cast<unsigned long long>(wbad));
   __syncthreads();
   for (int i = tid; i < kQ5MaxNations; i += blockDim.x)
-    if (s_sum[i]) atomicAdd(&sums[i], s_sum[i]);
+    if (s_sum[i]) atomicAdd(&sums[s_nat[i]], s_sum[i]);
 }
 
 // ---- batched: one pass over orders and lineitem for up to 64 queries ------
@@ -286,11 +302,36 @@ __global__ void q5b_orders_kernel(const int32_t* __restrict__ o_custkey, const i
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const uint64_t pol = policy_evict_first();
   unsigned int bad = 0;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_orders; i += stride) {
-    const int32_t d = ld_stream_s32(o_orderdate + i, pol);
-    const int32_t c = ld_stream_s32(o_custkey + i, pol);
+  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  // 4 orders per thread, as in the single query's pass (15M orders, 64 queries:
+  // 81 -> 73 us); a date no query wants leaves the customer unread and unchecked
+  const bool vec = ((reinterpret_cast<uintptr_t>(o_custkey) | reinterpret_cast<uintptr_t>(o_orderdate) |
+                     reinterpret_cast<uintptr_t>(dim_o)) & 15) == 0;
+  const int64_t n4 = vec ? n_orders >> 2 : 0;
+  for (int64_t i = t0; i < n4; i += stride) {
+    const int4 dv = ld_stream_v4(o_orderdate + 4 * i, pol), cv = ld_stream_v4(o_custkey + 4 * i, pol);
+    const int32_t d[4] = {dv.x, dv.y, dv.z, dv.w}, c[4] = {cv.x, cv.y, cv.z, cv.w};
+    uint64_t dm[4];
+    int32_t n[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      dm[e] = q5_date_mask(D, s_date, d[e]);
+      const bool okc = c[e] >= 1 && c[e] <= n_cust;
+      bad += dm[e] && !okc;
+      n[e] = (dm[e] && okc) ? __ldg(c_nationkey + (c[e] - 1)) : -1;
+    }
+    uint32_t packed = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const bool ok = static_cast<uint32_t>(n[e]) < kQ5MaxNations && (s_nat[n[e]] & dm[e]);
+      packed |= (ok ? static_cast<uint32_t>(n[e]) : 0xffu) << (8 * e);
+    }
+    reinterpret_cast<uint32_t*>(dim_o)[i] = packed;
+  }
+  for (int64_t i = 4 * n4 + t0; i < n_orders; i += stride) {
     int8_t v = -1;
-    const uint64_t dm = q5_date_mask(D, s_date, d);
+    const uint64_t dm = q5_date_mask(D, s_date, o_orderdate[i]);
+    const int32_t c = o_custkey[i];
     if (dm) {
       if (c < 1 || c > n_cust) {
         ++bad;
@@ -304,6 +345,9 @@ __global__ void q5b_orders_kernel(const int32_t* __restrict__ o_custkey, const i
   if (bad) atomicAdd(range_err, static_cast<unsigned long long>(bad));
 }
 
+// Price and discount are read with the keys here: with 64 queries one line in
+// 25 matches, and reading them late cost more in divergence than the bytes it
+// saved (60M lines: 339 us as it is, 422 us with late reads).
 // Shared memory: [date table: span x 8][sums: n_q x n_nation x 8][supplier nations].
 __global__ void __launch_bounds__(1024, 1) q5b_lines_kernel(
     const int32_t* __restrict__ l_suppkey, const int32_t* __restrict__ l_order, const int32_t* __restrict__ price,
@@ -420,33 +464,28 @@ int olap_q5_chain(olap_ctx* ctx, const olap_q5_tables* t, int32_t region, int32_
   unsigned long long* nmask = ar.take<unsigned long long>(1);
   if (!dim_s || !nib_s || !dim_o || !nmask)
     return olap::set_error(ctx, OLAP_ERR_CAPACITY, "scratch arena too small for Q5 vectors");
-  olap::q5_nation_mask_kernel<<<1, 64, 0, ctx->stream>>>(t->r_regionkey, t->n_region, t->n_regionkey, t->n_nation,
-                                                        region, nmask);
-  OLAP_CUDA_TRY(ctx, cudaMemsetAsync(nation_sums, 0, sizeof(int64_t) * t->n_nation, ctx->stream));
-  if (t->n_supp)
-    olap::q5_supplier_kernel<<<olap::grid_q5(ctx, t->n_supp, 256), 256, 0, ctx->stream>>>(t->s_nationkey, t->n_supp,
-                                                                                         nmask, dim_s);
+  olap::q5_prepare_kernel<<<olap::grid_q5(ctx, (t->n_supp + 1) / 2, 256), 256, 0, ctx->stream>>>(
+      t->r_regionkey, t->n_region, t->n_regionkey, t->n_nation, region, t->s_nationkey, t->n_supp, nmask, dim_s, nib_s,
+      reinterpret_cast<unsigned long long*>(nation_sums));
   if (t->n_orders)
     olap::q5_orders_kernel<<<olap::grid_q5(ctx, t->n_orders, 256), 256, 0, ctx->stream>>>(
         t->o_custkey, t->o_orderdate, t->n_orders, t->c_nationkey, t->n_cust, nmask, date1, date2, dim_o,
         &ctx->counters->range_errors);
-  // Supplier nations in shared memory as 4-bit codes when they fit (160 KB).
-  const int stage = t->n_lines && t->n_supp > 0 && (t->n_supp + 1) / 2 <= 160 * 1024 ? 2 : 0;
-  if (stage == 2)
-    olap::q5_supplier_nib_kernel<<<olap::grid_q5(ctx, (t->n_supp + 1) / 2, 256), 256, 0, ctx->stream>>>(
-        dim_s, t->n_supp, nmask, nib_s);
   if (t->n_lines) {
-    const size_t smem = stage == 2 ? static_cast<size_t>(((t->n_supp + 1) / 2 + 15) & ~int64_t(15)) : 0;
-    if (smem > 48 * 1024)
-      OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(olap::q5_lines_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    // Supplier codes in shared memory when they fit (160 KB).
+    const bool stage = t->n_supp > 0 && (t->n_supp + 1) / 2 <= 160 * 1024;
+    const size_t smem = stage ? static_cast<size_t>(((t->n_supp + 1) / 2 + 15) & ~int64_t(15)) : 0;
+    auto lines = stage ? olap::q5_lines_kernel<true> : olap::q5_lines_kernel<false>;
+    if (smem)  // always: static and dynamic together may pass 48 KB
+      OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(lines, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               static_cast<int>(smem)));
     int bps = 1;
-    OLAP_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, olap::q5_lines_kernel, 512, smem));
+    OLAP_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, lines, 512, smem));
     int64_t grid = static_cast<int64_t>(ctx->sm_count) * (bps < 1 ? 1 : bps);
     grid = std::min<int64_t>(grid, (t->n_lines / 4 + 511) / 512 + 1);
-    olap::q5_lines_kernel<<<static_cast<unsigned>(grid), 512, smem, ctx->stream>>>(
+    lines<<<static_cast<unsigned>(grid), 512, smem, ctx->stream>>>(
         t->l_suppkey, t->l_orderkey, t->l_price, t->l_discount, t->n_lines, dim_s, t->n_supp, nib_s, nmask, dim_o,
-        t->n_orders, reinterpret_cast<unsigned long long*>(nation_sums), &ctx->counters->range_errors, stage);
+        t->n_orders, reinterpret_cast<unsigned long long*>(nation_sums), &ctx->counters->range_errors);
   }
   OLAP_CUDA_TRY(ctx, cudaGetLastError());
   return OLAP_OK;
@@ -501,7 +540,7 @@ int olap_q5_batch(olap_ctx* ctx, const olap_q5_tables* t, const olap_q5_query* q
                                                                                           t->n_supp, nat_q, dim_s);
   const size_t date_bytes = sizeof(unsigned long long) * static_cast<size_t>(D.span);
   if (t->n_orders) {
-    if (date_bytes > 48 * 1024)
+    if (date_bytes)  // always: static and dynamic together may pass 48 KB
       OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(olap::q5b_orders_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               static_cast<int>(date_bytes)));
     olap::q5b_orders_kernel<<<olap::grid_q5(ctx, t->n_orders, 256), 256, date_bytes, ctx->stream>>>(
@@ -514,7 +553,7 @@ int olap_q5_batch(olap_ctx* ctx, const olap_q5_tables* t, const olap_q5_query* q
     const size_t budget = static_cast<size_t>(ctx->smem_optin) - 2048;  // static shared + headroom
     const bool stage = fixed + stage_bytes <= budget;
     const size_t smem = fixed + (stage ? stage_bytes : 0);
-    if (smem > 48 * 1024)
+    if (smem)
       OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(olap::q5b_lines_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               static_cast<int>(smem)));
     int bps = 1;
