@@ -40,7 +40,8 @@ def _ctx(ctx: Context | None) -> Context:
 
 
 def _i64(dev):
-    return _torch().zeros(1, dtype=_torch().int64, device=dev)
+    """A count or sum; every call writes it, of no rows too, so it is not cleared here."""
+    return _torch().empty(1, dtype=_torch().int64, device=dev)
 
 
 # ---- select ------------------------------------------------------------------
@@ -259,7 +260,7 @@ def aggalgo_f64(size_R: int, l_tax, l_quantity, l_extendedprice, ctx: Context | 
     """aggalgo_rowwise (aggregation:28-37) in double, reduced in a fixed order."""
     torch = _torch()
     c = _ctx(ctx)
-    s = torch.zeros(1, dtype=torch.float64, device=l_tax.device)
+    s = torch.empty(1, dtype=torch.float64, device=l_tax.device)
     check(lib.olap_agg_f64(c.handle, int(size_R), _ptr(l_tax), _ptr(l_quantity), _ptr(l_extendedprice), _ptr(s)),
           c.handle)
     return float(s.item())
