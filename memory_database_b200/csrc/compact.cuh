@@ -267,7 +267,10 @@ __global__ void __launch_bounds__(kCompactThreads) compact_kernel(const Op op_in
 // the arena runs in chunks, the running total kept on the device.
 constexpr int kExpandThreads = 1024;
 constexpr int kExpandDirect = 8;  // selected items per word of a step up to which the lanes write their own
+constexpr int kExpandStaged = 24;  // ... up to which they go through shared memory
 constexpr int kMarkRounds = 4;  // tiles per warp of a mark kernel on a long input
+
+constexpr size_t kExpandSmem = kExpandThreads * kExpandStaged * sizeof(uint16_t);  // a step's items, per warp
 
 struct Marks {
   uint32_t* bits;    // bit i % 32 of word i / 32: item i of the chunk is selected
@@ -296,9 +299,10 @@ __global__ void __launch_bounds__(kExpandThreads, 2) expand_kernel(const Emit em
                                                                    unsigned long long* __restrict__ total) {
   constexpr int W = kExpandThreads / 32;
   __shared__ unsigned long long s_sum[W];
-  __shared__ uint16_t s_at[Emit::kVals ? 1 : W][32 * kExpandDirect];  // items of a step, in order
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lt = (1u << lane) - 1u;
+  extern __shared__ uint16_t s_items[];
+  uint16_t* const s_at = s_items + warp * 32 * kExpandStaged;  // items of a step, in order
   const int per = (mk.n_tiles + gridDim.x * W - 1) / (gridDim.x * W);  // tiles per warp
   const int b0 = min(static_cast<int>(blockIdx.x) * W * per, mk.n_tiles);
   unsigned long long s = 0;
@@ -337,27 +341,26 @@ __global__ void __launch_bounds__(kExpandThreads, 2) expand_kernel(const Emit em
       const int all = static_cast<int>(__shfl_sync(0xffffffffu, inc, 31));
       const int64_t item = first_item + tb + r;
       const int words = (min(len - r, 1024) + 31) >> 5;
-      if (all <= kExpandDirect * words) {
-        if constexpr (Emit::kVals) {
-          int64_t pos = base + before, vi = v + in_tile;
-          while (word) {
-            em.emit(pos++, item + 32 * lane + __ffs(word) - 1, vi++);
-            word &= word - 1;
-          }
-        } else {
-          uint16_t* at = s_at[warp] + before;
-          while (word) {
-            *at++ = static_cast<uint16_t>(32 * lane + __ffs(word) - 1);
-            word &= word - 1;
-          }
-          __syncwarp();
-          for (int k0 = 0; k0 < all; k0 += 32) {  // same trips in every lane: 69 us; a loop per lane 80
-            const int k = k0 + lane;
-            const int off = k < all ? s_at[warp][k] : 0;
-            if (k < all) em.emit(base + k, item + off, 0);
-          }
-          __syncwarp();
+      if (Emit::kVals && all <= kExpandDirect * words) {
+        int64_t pos = base + before, vi = v + in_tile;
+        while (word) {
+          em.emit(pos++, item + 32 * lane + __ffs(word) - 1, vi++);
+          word &= word - 1;
         }
+      } else if (all <= kExpandStaged * words) {
+        for (int k = before; word; ++k) {
+          s_at[k] = static_cast<uint16_t>(32 * lane + __ffs(word) - 1);
+          word &= word - 1;
+        }
+        __syncwarp();
+        const int64_t ahead = Emit::kVals ? v + in_tile - before : 0;  // value index less position, by lane
+        for (int k0 = 0; k0 < all; k0 += 32) {  // same trips in every lane: 69 us; a loop per lane 80
+          const int k = k0 + lane;
+          const int off = k < all ? s_at[k] : 0;
+          const int64_t vi = Emit::kVals ? __shfl_sync(0xffffffffu, ahead, off >> 5) + k : 0;
+          if (k < all) em.emit(base + k, item + off, vi);
+        }
+        __syncwarp();
       } else {
 #pragma unroll 4
         for (int w = 0; w < words; ++w) {
@@ -424,6 +427,8 @@ int mark_and_expand(olap_ctx* ctx, Arena& ar, int64_t n, size_t val_bytes, int64
   mk.counts = counts;
   if (!mk.bits || (val_bytes && !mk.vals)) return set_error(ctx, OLAP_ERR_CAPACITY, small);
   mk.tile = static_cast<int32_t>(mark_tile(chunk, warps));
+  OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(expand_kernel<Emit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(kExpandSmem)));
   int which = 0;
   for (int64_t first = 0; first < n; first += chunk, which ^= 1) {
     mk.n = chunk < n - first ? chunk : n - first;
@@ -432,7 +437,7 @@ int mark_and_expand(olap_ctx* ctx, Arena& ar, int64_t n, size_t val_bytes, int64
     if (rc != OLAP_OK) return rc;
     const int64_t blocks = (mk.n_tiles + kExpandThreads / 32 - 1) / (kExpandThreads / 32);
     const int64_t cap = static_cast<int64_t>(ctx->sm_count) * 2;
-    expand_kernel<Emit><<<static_cast<unsigned>(blocks < cap ? blocks : cap), kExpandThreads, 0, ctx->stream>>>(
+    expand_kernel<Emit><<<static_cast<unsigned>(blocks < cap ? blocks : cap), kExpandThreads, kExpandSmem, ctx->stream>>>(
         em, mk, first, first ? run + which : nullptr, run + (which ^ 1), first + mk.n == n ? total : nullptr);
     OLAP_CUDA_TRY(ctx, cudaGetLastError());
   }
