@@ -310,7 +310,8 @@ OLAP_API int olap_plan_olapcore(const double sele[4], const int bitmap[4], const
  * (select/test_select_option.cpp:172-205, 391-423; if_sv is in_rowids).
  * out_rowids holds up to (in_rowids ? n_in : col_len) entries; *d_count
  * receives the count.  in_rowids entries outside [0, col_len) are dropped and
- * counted as range errors. */
+ * counted as range errors.  out_rowids may be in_rowids itself (refinement in
+ * place). */
 OLAP_API int olap_select_rowids(olap_ctx* ctx, const int32_t* col, int64_t col_len, int32_t val,
                                 int cmp, const int32_t* in_rowids, int64_t n_in,
                                 int32_t* out_rowids, int64_t* d_count);

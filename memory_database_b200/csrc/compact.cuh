@@ -281,6 +281,30 @@ struct Marks {
   int32_t n_tiles;
 };
 
+// First position of each warp's run of `per` whole tiles (warp w of block b takes
+// them from tile (b W + w) per on): *run_in and every tile before its own.  All
+// threads of a block of kThreads call it.
+template <int kThreads>
+__device__ __forceinline__ int64_t expand_base(const Marks& mk, int per, const unsigned long long* __restrict__ run_in) {
+  constexpr int W = kThreads / 32;
+  __shared__ unsigned long long s_sum[W];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int b0 = min(static_cast<int>(blockIdx.x) * W * per, mk.n_tiles);
+  unsigned long long s = 0;
+  for (int i = tid; i < (b0 >> 2); i += kThreads) {
+    const uint4 c = __ldg(reinterpret_cast<const uint4*>(mk.counts) + i);
+    s += static_cast<unsigned long long>(c.x) + c.y + c.z + c.w;
+  }
+  if (tid < (b0 & 3)) s += __ldg(mk.counts + (b0 & ~3) + tid);
+  const int t0 = min(b0 + warp * per, mk.n_tiles);
+  s = static_cast<unsigned long long>(warp_sum_i64(static_cast<int64_t>(s)));
+  if (lane == 0) s_sum[warp] = s;
+  __syncthreads();
+  s = (lane < W ? s_sum[lane] : 0ull) + (run_in && lane == 0 ? *run_in : 0ull);
+  for (int t = b0 + lane; t < t0; t += 32) s += __ldg(mk.counts + t);
+  return warp_sum_i64(static_cast<int64_t>(s));
+}
+
 // Emit: constexpr bool kVals; void emit(int64_t pos, int64_t item, int64_t v)
 // writes item `item` (of the whole input) at output position pos; v is the
 // index of its value in Marks::vals.  A warp takes a run of whole tiles, up to
@@ -298,27 +322,13 @@ __global__ void __launch_bounds__(kExpandThreads, 2) expand_kernel(const Emit em
                                                                    unsigned long long* __restrict__ run_out,
                                                                    unsigned long long* __restrict__ total) {
   constexpr int W = kExpandThreads / 32;
-  __shared__ unsigned long long s_sum[W];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lt = (1u << lane) - 1u;
   extern __shared__ uint16_t s_items[];
   uint16_t* const s_at = s_items + warp * 32 * kExpandStaged;  // items of a step, in order
   const int per = (mk.n_tiles + gridDim.x * W - 1) / (gridDim.x * W);  // tiles per warp
-  const int b0 = min(static_cast<int>(blockIdx.x) * W * per, mk.n_tiles);
-  unsigned long long s = 0;
-  for (int i = tid; i < (b0 >> 2); i += kExpandThreads) {
-    const uint4 c = __ldg(reinterpret_cast<const uint4*>(mk.counts) + i);
-    s += static_cast<unsigned long long>(c.x) + c.y + c.z + c.w;
-  }
-  if (tid < (b0 & 3)) s += __ldg(mk.counts + (b0 & ~3) + tid);
-  const int t0 = min(b0 + warp * per, mk.n_tiles), t1 = min(t0 + per, mk.n_tiles);
-  s = static_cast<unsigned long long>(warp_sum_i64(static_cast<int64_t>(s)));
-  if (lane == 0) s_sum[warp] = s;
-  __syncthreads();
-  // this warp's first position: every tile before its own
-  s = s_sum[lane] + (run_in && lane == 0 ? *run_in : 0ull);
-  for (int t = b0 + lane; t < t0; t += 32) s += __ldg(mk.counts + t);
-  int64_t base = warp_sum_i64(static_cast<int64_t>(s));
+  int64_t base = expand_base<kExpandThreads>(mk, per, run_in);
+  const int t0 = min((static_cast<int>(blockIdx.x) * W + warp) * per, mk.n_tiles), t1 = min(t0 + per, mk.n_tiles);
   const int wpt = mk.tile >> 5;                      // words per tile
   const int tps = wpt <= 32 ? 32 / wpt : 1;          // tiles per step, one when a tile takes several steps
   const int head = wpt <= 32 ? lane / wpt * wpt : 0; // lane of the first word of this lane's tile
@@ -381,6 +391,44 @@ __global__ void __launch_bounds__(kExpandThreads, 2) expand_kernel(const Emit em
   }
 }
 
+// Where the values are all that is wanted (no items, so no marks): each tile's
+// run of values to its place in `out`.  Bound by the latency of the runs, which
+// are short: four loads per lane in flight.
+constexpr int kRunThreads = 512;
+constexpr int kRunBlocks = 3;  // per SM
+struct RunCopy {
+  int32_t* out;
+};
+template <class Copy>
+__global__ void __launch_bounds__(kRunThreads, kRunBlocks) run_copy_kernel(
+    const Copy rc, const Marks mk, int64_t, const unsigned long long* __restrict__ run_in,
+    unsigned long long* __restrict__ run_out, unsigned long long* __restrict__ total) {
+  constexpr int W = kRunThreads / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = (mk.n_tiles + gridDim.x * W - 1) / (gridDim.x * W);
+  int64_t base = expand_base<kRunThreads>(mk, per, run_in);
+  const int t0 = min((static_cast<int>(blockIdx.x) * W + warp) * per, mk.n_tiles), t1 = min(t0 + per, mk.n_tiles);
+  const uint64_t pol = policy_evict_first();
+  for (int t = t0; t < t1; ++t) {
+    const int32_t* src = static_cast<const int32_t*>(mk.vals) + static_cast<int64_t>(t) * mk.tile + lane;
+    const int c = static_cast<int>(__ldg(mk.counts + t));
+    int32_t* dst = rc.out + base + lane;
+    for (int k = 0; k < c; k += 128) {
+      int32_t v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = ld_stream_s32_if(k + 32 * u + lane < c, src + k + 32 * u, pol, 0);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (k + 32 * u + lane < c) dst[k + 32 * u] = v[u];
+    }
+    base += c;
+  }
+  if (t1 == mk.n_tiles && t0 < t1 && lane == 0) {
+    if (run_out) *run_out = static_cast<unsigned long long>(base);
+    if (total) *total = static_cast<unsigned long long>(base);
+  }
+}
+
 // Items per warp tile for n items on `warps` resident warps: kMarkRounds
 // tiles per warp, the same number for each, down to one step of 128 items.
 inline int64_t mark_tile(int64_t n, int64_t warps) {
@@ -427,17 +475,24 @@ int mark_and_expand(olap_ctx* ctx, Arena& ar, int64_t n, size_t val_bytes, int64
   mk.counts = counts;
   if (!mk.bits || (val_bytes && !mk.vals)) return set_error(ctx, OLAP_ERR_CAPACITY, small);
   mk.tile = static_cast<int32_t>(mark_tile(chunk, warps));
-  OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(expand_kernel<Emit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(kExpandSmem)));
+  constexpr bool kRuns = std::is_same_v<Emit, RunCopy>;
+  void (*out_kernel)(const Emit, const Marks, int64_t, const unsigned long long*, unsigned long long*, unsigned long long*);
+  if constexpr (kRuns) out_kernel = run_copy_kernel<Emit>;
+  else out_kernel = expand_kernel<Emit>;
+  constexpr size_t out_smem = kRuns ? 0 : kExpandSmem;
+  constexpr int out_threads = kRuns ? kRunThreads : kExpandThreads;
+  if (!kRuns)
+    OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            static_cast<int>(kExpandSmem)));
   int which = 0;
   for (int64_t first = 0; first < n; first += chunk, which ^= 1) {
     mk.n = chunk < n - first ? chunk : n - first;
     mk.n_tiles = static_cast<int32_t>((mk.n + mk.tile - 1) / mk.tile);
     const int rc = mark(mk, first, em);
     if (rc != OLAP_OK) return rc;
-    const int64_t blocks = (mk.n_tiles + kExpandThreads / 32 - 1) / (kExpandThreads / 32);
-    const int64_t cap = static_cast<int64_t>(ctx->sm_count) * 2;
-    expand_kernel<Emit><<<static_cast<unsigned>(blocks < cap ? blocks : cap), kExpandThreads, kExpandSmem, ctx->stream>>>(
+    const int64_t blocks = (mk.n_tiles + out_threads / 32 - 1) / (out_threads / 32);
+    const int64_t cap = static_cast<int64_t>(ctx->sm_count) * (kRuns ? kRunBlocks : 2);
+    out_kernel<<<static_cast<unsigned>(blocks < cap ? blocks : cap), out_threads, out_smem, ctx->stream>>>(
         em, mk, first, first ? run + which : nullptr, run + (which ^ 1), first + mk.n == n ? total : nullptr);
     OLAP_CUDA_TRY(ctx, cudaGetLastError());
   }

@@ -26,29 +26,26 @@ __device__ __forceinline__ int32_t lane4(const int4& v, int k) {
   return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w;
 }
 
-// Marks of cmp(col[r], val) over the column (kRid false) or over the rows of an
-// input selection vector; a warp takes whole tiles.  Bound by the column read:
-// full tiles of an aligned column take four 16-byte loads per lane at a time,
-// and two lanes' 4-bit results make one byte of the bitmap (row order, no
-// ballots).  With a selection vector or unaligned, 32 rows at a time, lane =
-// row, one ballot per word.  The predicate is col <= val (the caller turns <
-// into it), none when `none`.  counts may be null (the bitmap alone).
-template <bool kRid>
-__global__ void __launch_bounds__(512) select_mark_kernel(const int32_t* __restrict__ col, int64_t col_len,
-                                                          const int32_t* __restrict__ in_rowids, int64_t n,
-                                                          int32_t val, int none, int vec, uint32_t* __restrict__ bits,
+// Marks of cmp(col[r], val) over the column; a warp takes whole tiles.  Bound by
+// the column read: full tiles of an aligned column (kVec) take four 16-byte
+// loads per lane at a time, and two lanes' 4-bit results make one byte of the
+// bitmap (row order, no ballots).  An unaligned column takes 32 rows at a time,
+// lane = row, one ballot per word.  The predicate is col <= val (the caller
+// turns < into it), none when `none`.  counts may be null (the bitmap alone).
+template <bool kVec>
+__global__ void __launch_bounds__(512) select_mark_kernel(const int32_t* __restrict__ col, int64_t n, int32_t val,
+                                                          int none, uint32_t* __restrict__ bits,
                                                           uint32_t* __restrict__ counts, int32_t tile,
-                                                          int64_t n_tiles, unsigned long long* range_err) {
+                                                          int64_t n_tiles) {
   const int lane = threadIdx.x & 31;
   const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   const uint64_t pol = policy_evict_first();
   const uint32_t keep = none ? 0u : 15u;
-  unsigned int bad = 0;
   for (int64_t t = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; t < n_tiles; t += n_warps) {
     const int64_t first = t * tile;
     const int64_t end = first + tile < n ? first + tile : n;
     uint32_t c = 0;
-    if (!kRid && vec && first + tile <= n) {
+    if (kVec && first + tile <= n) {
       const int32_t* src = col + first + 4 * lane;
       unsigned char* dst = reinterpret_cast<unsigned char*>(bits) + (first >> 3) + (lane >> 1);
       auto put = [&](const int4 v, int at) {
@@ -69,22 +66,19 @@ __global__ void __launch_bounds__(512) select_mark_kernel(const int32_t* __restr
       }
       for (; at < tile; at += 128) put(ld_stream_v4_ordered(src + at, pol), at);
     } else {
-      for (int64_t r0 = first; r0 < end; r0 += 32) {
-        const int64_t r = r0 + lane;
-        bool pass = false;
-        if (r < end) {
-          if (kRid) {
-            const int32_t row = __ldg(in_rowids + r);
-            if (row < 0 || row >= col_len) ++bad;  // not a row of col: dropped and counted
-            else pass = __ldg(col + row) <= val && !none;
-          } else {
-            pass = __ldg(col + r) <= val && !none;
+      constexpr int G = 1;  // words at a time
+      for (int64_t r0 = first; r0 < end; r0 += 32 * G) {
+        int32_t v[G];
+#pragma unroll
+        for (int u = 0; u < G; ++u)
+          v[u] = ld_stream_s32_if(r0 + 32 * u + lane < end, col + r0 + 32 * u + lane, pol, 0);
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+          const uint32_t word = __ballot_sync(0xffffffffu, v[u] <= val && !none && r0 + 32 * u + lane < end);
+          if (lane == 0 && r0 + 32 * u < end) {
+            bits[(r0 >> 5) + u] = word;
+            c += __popc(word);
           }
-        }
-        const uint32_t word = __ballot_sync(0xffffffffu, pass);
-        if (lane == 0) {
-          bits[r0 >> 5] = word;
-          c += __popc(word);
         }
       }
     }
@@ -93,18 +87,86 @@ __global__ void __launch_bounds__(512) select_mark_kernel(const int32_t* __restr
       if (lane == 0) counts[t] = c;
     }
   }
-  if (kRid && bad) atomicAdd(range_err, static_cast<unsigned long long>(bad));
 }
 
-// Selected rows: their ids, or the entries of the input selection vector.
-struct SelectEmit {
+// Selected rows: their ids.
+struct RowEmit {
   static constexpr bool kVals = false;
-  const int32_t* in_rowids;
   int32_t* out;
-  __device__ __forceinline__ void emit(int64_t pos, int64_t item, int64_t) const {
-    out[pos] = in_rowids ? __ldg(in_rowids + item) : static_cast<int32_t>(item);
-  }
+  __device__ __forceinline__ void emit(int64_t pos, int64_t item, int64_t) const { out[pos] = static_cast<int32_t>(item); }
 };
+
+// Refinement of a selection vector: the passing entries of each tile go to
+// `vals` (those of tile t from element t * tile on), from where they are
+// copied to the output once their positions are known (run_copy_kernel).  By
+// then no block reads the vector any more, so the output may be the vector
+// itself.  Lane l takes the entries 32 u + l of a step, whose rows are close
+// when the vector is dense.  Bound by the latency of the two dependent reads:
+// the next step's entries load while this one's rows are looked up (2^27
+// entries, all rows in order, 30 % pass, with the copy: 500 us in one pass with
+// look-back, 644 us with one entry per lane and step, 356 us so; every tenth
+// row: 174, 174 and 150 us a call).
+__global__ void __launch_bounds__(512, 3) select_refine_kernel(const int32_t* __restrict__ col, uint32_t col_len,
+                                                               const int32_t* __restrict__ in_rowids, int32_t val,
+                                                               int none, const Marks mk,
+                                                               unsigned long long* range_err) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t lt = (1u << lane) - 1u;
+  const int n_warps = static_cast<int>((gridDim.x * blockDim.x) >> 5);
+  const uint64_t pol = policy_evict_first();
+  const uint32_t keep = none ? 0u : 15u;
+  const int32_t* const at = col_len ? col : in_rowids;  // an entry outside the column looks up its first word
+  unsigned int bad = 0;
+  for (int t = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5); t < mk.n_tiles; t += n_warps) {
+    const int64_t first = static_cast<int64_t>(t) * mk.tile;
+    const int len = static_cast<int>(first + mk.tile < mk.n ? mk.tile : mk.n - first);
+    const int whole = len & ~127;  // entries in full steps: all but the chunk's last
+    const int32_t* src = in_rowids + first + lane;
+    int32_t* vals = static_cast<int32_t*>(mk.vals) + first;
+    uint32_t c = 0;
+    int32_t next[4];
+    auto load_next = [&](int r) {
+      if (r < whole) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) next[u] = ld_stream_s32(src + r + 32 * u, pol);
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) next[u] = ld_stream_s32_if(r + 32 * u + lane < len, src + r + 32 * u, pol, 0);
+      }
+    };
+    load_next(0);
+    for (int r = 0; r < len; r += 128) {
+      uint32_t has = 15u;
+      if (r >= whole) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (r + 32 * u + lane >= len) has &= ~(1u << u);
+      }
+      int32_t row[4], v[4];
+      uint32_t in = 0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        row[u] = next[u];
+        in |= static_cast<uint32_t>(static_cast<uint32_t>(row[u]) < col_len) << u;
+      }
+      in &= has;
+      bad += __popc(has ^ in);  // not rows of col: dropped and counted
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = __ldg(at + ((in >> u) & 1u ? row[u] : 0));
+      if (r + 128 < len) load_next(r + 128);
+      in &= keep;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool pass = ((in >> u) & 1u) && v[u] <= val;
+        const uint32_t w = __ballot_sync(0xffffffffu, pass);
+        if (pass) vals[c + __popc(w & lt)] = row[u];
+        c += __popc(w);
+      }
+    }
+    if (lane == 0) mk.counts[t] = c;
+  }
+  if (bad) atomicAdd(range_err, static_cast<unsigned long long>(bad));
+}
 
 // Rows where Ra <= c and Rc <= c; writes the pair (Ra, Rc).
 struct ProjectOp {
@@ -371,21 +433,26 @@ int olap_select_rowids(olap_ctx* ctx, const int32_t* col, int64_t col_len, int32
   unsigned long long* total = d_count ? reinterpret_cast<unsigned long long*>(d_count)
                                       : ar.take<unsigned long long>(1);
   if (!total) return olap::set_error(ctx, OLAP_ERR_CAPACITY, "scratch arena exhausted");
-  const olap::SelectEmit em{in_rowids, out_rowids};
   const olap::LePred le(val, cmp);
+  if (in_rowids)
+    return olap::mark_and_expand(
+        ctx, ar, n, sizeof(int32_t), ctx->sm_count * int64_t(48), olap::RunCopy{out_rowids}, total,
+        [&](const olap::Marks& mk, int64_t first, const olap::RunCopy&) {
+          unsigned grid, block;
+          olap::mark_grid(ctx, mk.n_tiles, 512, 3, &grid, &block);
+          olap::select_refine_kernel<<<grid, block, 0, ctx->stream>>>(col, static_cast<uint32_t>(col_len), in_rowids + first, le.val, le.none,
+                                                                      mk, &ctx->counters->range_errors);
+          OLAP_CUDA_TRY(ctx, cudaGetLastError());
+          return OLAP_OK;
+        });
+  auto* const kernel = olap::al16(col) ? olap::select_mark_kernel<true> : olap::select_mark_kernel<false>;
   return olap::mark_and_expand(
-      ctx, ar, n, 0, ctx->sm_count * int64_t(64), em, total,
-      [&](const olap::Marks& mk, int64_t first, const olap::SelectEmit&) {
+      ctx, ar, n, 0, ctx->sm_count * int64_t(64), olap::RowEmit{out_rowids}, total,
+      [&](const olap::Marks& mk, int64_t first, const olap::RowEmit&) {
         unsigned grid, block;
         olap::mark_grid(ctx, mk.n_tiles, 512, 4, &grid, &block);
-        if (in_rowids)
-          olap::select_mark_kernel<true><<<grid, block, 0, ctx->stream>>>(
-              col, col_len, in_rowids + first, mk.n, le.val, le.none, 0, mk.bits, mk.counts, mk.tile, mk.n_tiles,
-              &ctx->counters->range_errors);
-        else
-          olap::select_mark_kernel<false><<<grid, block, 0, ctx->stream>>>(
-              col + first, col_len, nullptr, mk.n, le.val, le.none, olap::al16(col), mk.bits, mk.counts, mk.tile,
-              mk.n_tiles, nullptr);
+        kernel<<<grid, block, 0, ctx->stream>>>(col + first, mk.n, le.val, le.none, mk.bits, mk.counts, mk.tile,
+                                                mk.n_tiles);
         OLAP_CUDA_TRY(ctx, cudaGetLastError());
         return OLAP_OK;
       });
@@ -422,9 +489,9 @@ int olap_select_bitmap(olap_ctx* ctx, const int32_t* col, int64_t n, int32_t val
   const int64_t n_tiles = (n + tile - 1) / tile;
   unsigned grid, block;
   olap::mark_grid(ctx, n_tiles, 512, 4, &grid, &block);
-  olap::select_mark_kernel<false><<<grid, block, 0, ctx->stream>>>(col, n, nullptr, n, le.val, le.none, olap::al16(col),
-                                                                  bitmap, nullptr, static_cast<int32_t>(tile), n_tiles,
-                                                                  nullptr);
+  auto* const kernel = olap::al16(col) ? olap::select_mark_kernel<true> : olap::select_mark_kernel<false>;
+  kernel<<<grid, block, 0, ctx->stream>>>(col, n, le.val, le.none, bitmap, nullptr, static_cast<int32_t>(tile),
+                                          n_tiles);
   OLAP_CUDA_TRY(ctx, cudaGetLastError());
   return OLAP_OK;
 }
