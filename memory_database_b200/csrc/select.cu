@@ -29,9 +29,11 @@ __device__ __forceinline__ int32_t lane4(const int4& v, int k) {
 // Marks of cmp(col[r], val) over the column; a warp takes whole tiles.  Bound by
 // the column read: full tiles of an aligned column (kVec) take four 16-byte
 // loads per lane at a time, and two lanes' 4-bit results make one byte of the
-// bitmap (row order, no ballots).  An unaligned column takes 32 rows at a time,
-// lane = row, one ballot per word.  The predicate is col <= val (the caller
-// turns < into it), none when `none`.  counts may be null (the bitmap alone).
+// bitmap (row order, no ballots).  An unaligned column takes 128 rows at a
+// time, lane l the rows 32 u + l, so that a ballot is a word and four loads are
+// in flight (2^27 rows to a bitmap: 460 us with one row per lane and step,
+// 154 us so).  The predicate is col <= val (the caller turns < into it), none
+// when `none`.  counts may be null (the bitmap alone).
 template <bool kVec>
 __global__ void __launch_bounds__(512) select_mark_kernel(const int32_t* __restrict__ col, int64_t n, int32_t val,
                                                           int none, uint32_t* __restrict__ bits,
@@ -66,7 +68,7 @@ __global__ void __launch_bounds__(512) select_mark_kernel(const int32_t* __restr
       }
       for (; at < tile; at += 128) put(ld_stream_v4_ordered(src + at, pol), at);
     } else {
-      constexpr int G = 1;  // words at a time
+      constexpr int G = kVec ? 1 : 4;  // words at a time (kVec: only the last tile comes here)
       for (int64_t r0 = first; r0 < end; r0 += 32 * G) {
         int32_t v[G];
 #pragma unroll
