@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(512, 4) q5_lines_kernel(
   };
   const int32_t none = staged ? 15 : -1;
   const uint32_t n_s = static_cast<uint32_t>(n_supp < INT32_MAX ? n_supp : INT32_MAX);
-  const uint32_t n_o = static_cast<uint32_t>(n_orders < INT32_MAX ? n_orders : int64_t(INT32_MAX) + 1);
+  const uint32_t n_o = static_cast<uint32_t>(n_orders <= INT32_MAX ? n_orders : int64_t(INT32_MAX) + 1);
   const uint64_t pol = policy_evict_first();
   const uint64_t keep = policy_evict_last();
   unsigned int bad = 0;
