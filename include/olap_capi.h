@@ -99,7 +99,11 @@ typedef struct olap_ctx olap_ctx;
 OLAP_API int olap_ctx_create(int device, size_t scratch_bytes, olap_ctx** out);
 OLAP_API int olap_ctx_destroy(olap_ctx* ctx);
 /* Run later calls on cuda_stream (a cudaStream_t); NULL is CUDA's legacy
- * default stream.  The context's own stream is released on the first call. */
+ * default stream.  The context's own stream is released on the first call.
+ * Calls share the context's scratch, so work on the new stream waits (on the
+ * device) for the work of earlier calls on the stream it replaces, which must
+ * not have been destroyed yet.  A stream being captured is not ordered: when a
+ * graph runs, its user orders it with the context's other work. */
 OLAP_API int olap_ctx_set_stream(olap_ctx* ctx, void* cuda_stream);
 OLAP_API void* olap_ctx_get_stream(olap_ctx* ctx);
 /* Waits for the context stream; OLAP_ERR_TIMEOUT when a bounded device wait

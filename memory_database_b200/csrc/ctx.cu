@@ -30,6 +30,31 @@ __global__ void max_i32_kernel(const int32_t* __restrict__ col, int64_t n, int* 
   if ((threadIdx.x & 31) == 0 && m != INT32_MIN) atomicMax(out, m);
 }
 
+// True while work on s goes into a graph instead of running (and where that
+// cannot be told because a capture is under way).
+static bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
+// Orders `next` behind the work in flight on the context's stream: the calls
+// of both use the same scratch.  Without an effect on a stream being captured,
+// whose work does not run yet; the next stream then waits for what came before.
+static int order_streams(olap_ctx* ctx, cudaStream_t next) {
+  if (!capturing(ctx->stream)) {
+    if (ctx->earlier_owed) OLAP_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, ctx->earlier, 0));
+    if (cudaEventRecord(ctx->earlier, ctx->stream) == cudaSuccess) ctx->earlier_set = true;
+    else cudaGetLastError();  // no work can be in flight on a stream that takes none
+  }
+  ctx->earlier_owed = ctx->earlier_set && capturing(next);
+  if (ctx->earlier_set && !ctx->earlier_owed) OLAP_CUDA_TRY(ctx, cudaStreamWaitEvent(next, ctx->earlier, 0));
+  return OLAP_OK;
+}
+
 }  // namespace olap
 
 extern "C" {
@@ -76,6 +101,7 @@ int olap_ctx_create(int device, size_t scratch_bytes, olap_ctx** out) {
   auto fail = [&](int st) {
     if (c->arena) cudaFree(c->arena);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
+    if (c->earlier) cudaEventDestroy(c->earlier);
     delete c;
     return st;
   };
@@ -88,6 +114,7 @@ int olap_ctx_create(int device, size_t scratch_bytes, olap_ctx** out) {
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
     return fail(OLAP_ERR_CUDA);
   c->own_stream = true;
+  if (cudaEventCreateWithFlags(&c->earlier, cudaEventDisableTiming) != cudaSuccess) return fail(OLAP_ERR_CUDA);
   c->arena_bytes = scratch_bytes ? scratch_bytes : (size_t(64) << 20);
   if (c->arena_bytes < (size_t(1) << 20)) c->arena_bytes = size_t(1) << 20;
   if (cudaMalloc(&c->arena, c->arena_bytes) != cudaSuccess) {
@@ -106,10 +133,12 @@ int olap_ctx_destroy(olap_ctx* ctx) {
   if (!ctx) return OLAP_ERR_INVALID;
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+  if (ctx->earlier_owed) cudaEventSynchronize(ctx->earlier);
   if (ctx->arena) cudaFree(ctx->arena);
   if (ctx->big) cudaFree(ctx->big);
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
+  cudaEventDestroy(ctx->earlier);
   delete ctx;
   return OLAP_OK;
 }
@@ -123,6 +152,9 @@ int olap_ctx_set_stream(olap_ctx* ctx, void* cuda_stream) {
   if (ctx->own_stream && ctx->stream) {
     cudaStreamSynchronize(ctx->stream);
     cudaStreamDestroy(ctx->stream);
+  } else {
+    const int st = olap::order_streams(ctx, s);
+    if (st != OLAP_OK) return st;
   }
   ctx->stream = s;
   ctx->own_stream = false;

@@ -37,6 +37,10 @@ struct olap_ctx {
   int64_t l2_bytes = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  // The work of the caller streams used before `stream` (olap_ctx_set_stream).
+  cudaEvent_t earlier = nullptr;
+  bool earlier_set = false;     // recorded at least once
+  bool earlier_owed = false;    // `stream` does not wait for it (it was being captured)
 
   // Scratch arena: one cudaMalloc at creation, bump-allocated per call and
   // reset at the start of each call (calls on one context are stream-ordered).
