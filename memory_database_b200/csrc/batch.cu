@@ -126,7 +126,8 @@ struct BatchParams {
   int32_t probe_order;                // 4 x 2-bit table ids, smallest table first
   int32_t agg;                        // OLAP_AGG_* of every query (one aggregate)
   int32_t smem_slots;                 // per-block shared accumulators (dynamic shared memory)
-  int32_t packed;                     // every factor and output offset fits QueryPlace
+  int32_t packed;                     // every factor fits 16 bits, every output offset 31
+  int32_t vec;                        // the fact columns read start on 16-byte boundaries
   int32_t block;                      // threads per block of the scan (part of a recorded graph)
   unsigned long long* range_err;
 };
@@ -327,7 +328,7 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + tid; i - lane < n4; i += stride) {
     const int64_t r0 = 4 * i;
     const int nv = r0 + 4 <= p.n_rows ? 4 : r0 < p.n_rows ? static_cast<int>(p.n_rows - r0) : 0;
-    const bool full = nv == 4;
+    const bool full = nv == 4, vec = full && p.vec;  // vec: 16-byte loads, which must stay inside that guard
     // Arrays are indexed by probe position o (table t = tab[o]), so that
     // every index is a compile-time constant.
     int32_t key[OLAP_MAX_DIMS][4];
@@ -336,16 +337,16 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
     for (int o = 0; o < OLAP_MAX_DIMS; ++o) {
       if (o >= ntab) continue;
       const int32_t* f = p.fk[tab[o]];
-      if (full) {
-        const int4 v = ld_stream_v4(f + r0, pol_stream);
+      if (vec) {
+        const int4 v = ld_stream_v4_ordered(f + r0, pol_stream);
         key[o][0] = v.x; key[o][1] = v.y; key[o][2] = v.z; key[o][3] = v.w;
       } else {
         for (int k = 0; k < 4; ++k) key[o][k] = k < nv ? f[r0 + k] : 0;
       }
     }
     if (need_m1) {
-      if (full) {
-        const int4 v = ld_stream_v4(p.m1 + r0, pol_stream);
+      if (vec) {
+        const int4 v = ld_stream_v4_ordered(p.m1 + r0, pol_stream);
         x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
       } else {
 #pragma unroll
@@ -353,8 +354,8 @@ __global__ void __launch_bounds__(PAR ? 512 : kBatchMaxThreads, 1) batch_scan_ke
       }
     }
     if (need_m2) {
-      if (full) {
-        const int4 v = ld_stream_v4(p.m2 + r0, pol_stream);
+      if (vec) {
+        const int4 v = ld_stream_v4_ordered(p.m2 + r0, pol_stream);
         y[0] = v.x; y[1] = v.y; y[2] = v.z; y[3] = v.w;
       } else {
 #pragma unroll
@@ -791,6 +792,10 @@ int olap_batch_run(olap_batch* b, const olap_batch_query* queries, int n_queries
   const bool need_m1 = agg == OLAP_AGG_M1_PLUS_M2 || agg == OLAP_AGG_M1 || agg == OLAP_AGG_M1_TIMES_M2;
   const bool need_m2 = agg == OLAP_AGG_M1_PLUS_M2 || agg == OLAP_AGG_M2 || agg == OLAP_AGG_M1_TIMES_M2;
   OLAP_REQUIRE(ctx, n_rows == 0 || ((!need_m1 || m1) && (!need_m2 || m2)), "measure columns required");
+  uintptr_t starts = (need_m1 ? reinterpret_cast<uintptr_t>(m1) : 0) | (need_m2 ? reinterpret_cast<uintptr_t>(m2) : 0);
+  for (int t = 0; t < OLAP_MAX_DIMS; ++t)
+    if ((tables >> t) & 1) starts |= reinterpret_cast<uintptr_t>(fk[t]);
+  p.vec = (starts & 15) == 0;
   const size_t scan_smem = sizeof(unsigned long long) * static_cast<size_t>(b->smem_slots);
   const bool par = b->parallel_probe != 0 && b->block <= 512;
   // 16-bit factors and 31-bit output offsets (every batch but extreme ones)
