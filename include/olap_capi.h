@@ -166,9 +166,9 @@ typedef struct olap_starjoin_query {
 OLAP_API int olap_starjoin_groupsum(olap_ctx* ctx, const olap_starjoin_query* q,
                            int64_t* group_sums, int64_t* totals);
 /* Kernels one olap_starjoin_groupsum call of this query launches with the
- * context's current knobs (the zeroing of the outputs, one prepass per
- * dimension staged as a pass bitmap or as 4-bit codes, and the star-join);
- * nothing is launched. */
+ * context's current knobs (the zeroing of the outputs, and unless the row range
+ * is empty one prepass per dimension staged as a pass bitmap or as 4-bit codes
+ * and the star-join); nothing is launched. */
 OLAP_API int olap_starjoin_launch_count(olap_ctx* ctx, const olap_starjoin_query* q, int want_groups,
                                         int* kernels);
 

@@ -1633,8 +1633,8 @@ int olap_starjoin_launch_count(olap_ctx* ctx, const olap_starjoin_query* q, int 
   int64_t probe = 0;  // only its address: the plan records the output pointers
   const int st = olap::plan_starjoin(ctx, q, want_groups ? &probe : nullptr, &probe, ar, &pl);
   if (st != OLAP_OK) return st;
-  // the zeroing of the outputs, the star-join and its prepasses
-  *kernels = q->row_end > q->row_begin ? 2 + pl.nbits + pl.nnib : 0;
+  // the zeroing of the outputs, and over any rows the star-join and its prepasses
+  *kernels = q->row_end > q->row_begin ? 2 + pl.nbits + pl.nnib : 1;
   return OLAP_OK;
 }
 
