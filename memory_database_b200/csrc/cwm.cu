@@ -102,19 +102,23 @@ __device__ __forceinline__ uint32_t stage_dims(const DimSet& d, unsigned char* s
 }
 
 // All dimensions of the rows in one pass, a warp on a tile of rows at a time,
-// 128 rows at a step, lane l the rows 4 l .. 4 l + 3 (16-byte key loads when
-// the columns are aligned).  Every key is range-checked first (a row with one
-// out of range is dropped and counted), then the dimensions are probed: those
+// 128 rows at a step: lane l the rows 4 l .. 4 l + 3 by 16-byte key loads (VEC),
+// or where a column is not aligned the rows 32 u + l, so that the loads of a
+// warp are still runs (60M rows to the vector: 788 us with four neighbours per
+// lane there, 252 us so).  Every key is range-checked first (a row with one out
+// of range is dropped and counted), then the dimensions are probed: those
 // staged in shared memory, smallest first, then the rest through L2; with LATE
 // the first of them last (a dimension that keeps nearly everything filters
 // nothing before the L2 probes).  Bound by instructions, so a row is dropped
 // without a branch or a predicate: its largest code stays DIM_NULL, and from
 // then on it reads entry 0 of the vectors in L2, one line for all such rows.
-template <int MODE, bool LATE>
+template <int MODE, bool LATE, bool VEC>
 __device__ __forceinline__ void cwm_probe_rows(const DimSet& d, const unsigned char* sdim, uint32_t staged, int64_t n,
-                                               int vec, int32_t tile, int64_t n_tiles, void* __restrict__ out,
-                                               const Marks& mk, int64_t* tot, unsigned int* bad) {
+                                               int32_t tile, int64_t n_tiles, void* __restrict__ out, const Marks& mk,
+                                               int64_t* tot, unsigned int* bad) {
   const int lane = threadIdx.x & 31;
+  const uint32_t lt = (1u << lane) - 1u;
+  auto off = [lane](int u) { return VEC ? 4 * lane + u : 32 * u + lane; };  // a step's row of register slot u
   const uint64_t pol = policy_evict_first();
   const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   for (int64_t t = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; t < n_tiles; t += n_warps) {
@@ -122,27 +126,32 @@ __device__ __forceinline__ void cwm_probe_rows(const DimSet& d, const unsigned c
     const int len = static_cast<int>(first + tile < n ? tile : n - first);
     uint32_t c = 0;
     for (int r0 = 0; r0 < len; r0 += 128) {
-      const int64_t r = first + r0 + 4 * lane;
+      const int64_t r = first + r0;
       uint32_t k[OLAP_MAX_DIMS][4];
       int32_t top[4];  // largest code of the row so far: DIM_NULL once a dimension misses
-      const bool full = vec && r0 + 128 <= len;
+      const bool full = r0 + 128 <= len;
       if (full) {
 #pragma unroll
         for (int j = 0; j < OLAP_MAX_DIMS; ++j) {
           if (j >= d.nd) continue;
-          const int4 v = ld_stream_v4(d.fk[j] + r, pol);
-          k[j][0] = v.x; k[j][1] = v.y; k[j][2] = v.z; k[j][3] = v.w;
+          if (VEC) {
+            const int4 v = ld_stream_v4(d.fk[j] + r + 4 * lane, pol);
+            k[j][0] = v.x; k[j][1] = v.y; k[j][2] = v.z; k[j][3] = v.w;
+          } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) k[j][u] = static_cast<uint32_t>(ld_stream_s32(d.fk[j] + r + off(u), pol));
+          }
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) top[u] = INT8_MIN;
       } else {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const bool in = r0 + 4 * lane + u < len;
+          const bool in = r0 + off(u) < len;
           top[u] = in ? INT8_MIN : OLAP_DIM_NULL;
 #pragma unroll
           for (int j = 0; j < OLAP_MAX_DIMS; ++j)
-            if (j < d.nd) k[j][u] = static_cast<uint32_t>(ld_stream_s32_if(in, d.fk[j] + r + u, pol, 0));
+            if (j < d.nd) k[j][u] = static_cast<uint32_t>(ld_stream_s32_if(in, d.fk[j] + r + off(u), pol, 0));
         }
       }
       uint32_t out_of_range = 0;
@@ -198,21 +207,33 @@ __device__ __forceinline__ void cwm_probe_rows(const DimSet& d, const unsigned c
         int32_t v[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) v[u] = live[u] ? g[u] : OLAP_GROUP_NULL;
-        if (full) {
+        if (VEC && full) {
           if (MODE == CWM_SV16)
-            *reinterpret_cast<short4*>(static_cast<int16_t*>(out) + r) =
+            *reinterpret_cast<short4*>(static_cast<int16_t*>(out) + r + 4 * lane) =
                 make_short4(static_cast<int16_t>(v[0]), static_cast<int16_t>(v[1]), static_cast<int16_t>(v[2]),
                             static_cast<int16_t>(v[3]));
           else
-            *reinterpret_cast<int4*>(static_cast<int32_t*>(out) + r) = make_int4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<int4*>(static_cast<int32_t*>(out) + r + 4 * lane) = make_int4(v[0], v[1], v[2], v[3]);
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           if (MODE == CWM_SV32) *tot += v[u] != OLAP_GROUP_NULL;
-          if (full || r0 + 4 * lane + u >= len) continue;
-          if (MODE == CWM_SV16) static_cast<int16_t*>(out)[r + u] = static_cast<int16_t>(v[u]);
-          else static_cast<int32_t*>(out)[r + u] = v[u];
+          if ((VEC && full) || r0 + off(u) >= len) continue;
+          if (MODE == CWM_SV16) static_cast<int16_t*>(out)[r + off(u)] = static_cast<int16_t>(v[u]);
+          else static_cast<int32_t*>(out)[r + off(u)] = v[u];
         }
+      } else if (!VEC) {
+        // a ballot is a word of the bitmap; the ids of a step go out as one run
+        uint32_t w[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          w[u] = __ballot_sync(0xffffffffu, live[u]);
+          const int64_t at = first + c + __popc(w[u] & lt);
+          if (live[u] && MODE == CWM_MARK16) static_cast<int16_t*>(mk.vals)[at] = static_cast<int16_t>(g[u]);
+          if (live[u] && MODE == CWM_MARK32) static_cast<int32_t*>(mk.vals)[at] = g[u];
+          c += __popc(w[u]);
+        }
+        if (lane == 0) reinterpret_cast<uint4*>(mk.bits)[r >> 7] = make_uint4(w[0], w[1], w[2], w[3]);
       } else {
         // two lanes' 4 rows make a byte of the bitmap (the chunk's holds
         // whole 128-item steps); the ids in row order
@@ -244,17 +265,17 @@ __device__ __forceinline__ void cwm_probe_rows(const DimSet& d, const unsigned c
   }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(1024, 1) cwm_probe_kernel(const DimSet d, int64_t n, int vec, int32_t tile,
-                                                            int64_t n_tiles, void* __restrict__ out, const Marks mk,
+template <int MODE, bool VEC>
+__global__ void __launch_bounds__(1024, 1) cwm_probe_kernel(const DimSet d, int64_t n, int32_t tile, int64_t n_tiles,
+                                                            void* __restrict__ out, const Marks mk,
                                                             unsigned long long* count, unsigned long long* range_err) {
   extern __shared__ __align__(16) unsigned char sdim[];
   bool late = false;
   const uint32_t staged = stage_dims(d, sdim, &late);
   unsigned int bad = 0;
   int64_t tot = 0;
-  if (late) cwm_probe_rows<MODE, true>(d, sdim, staged, n, vec, tile, n_tiles, out, mk, &tot, &bad);
-  else cwm_probe_rows<MODE, false>(d, sdim, staged, n, vec, tile, n_tiles, out, mk, &tot, &bad);
+  if (late) cwm_probe_rows<MODE, true, VEC>(d, sdim, staged, n, tile, n_tiles, out, mk, &tot, &bad);
+  else cwm_probe_rows<MODE, false, VEC>(d, sdim, staged, n, tile, n_tiles, out, mk, &tot, &bad);
   const unsigned int wbad = __reduce_add_sync(0xffffffffu, bad);
   if (MODE == CWM_SV32) tot = warp_sum_i64(tot);
   if ((threadIdx.x & 31) == 0) {
@@ -457,10 +478,10 @@ static int launch_probe(olap_ctx* ctx, const DimSet& d, int64_t n, int32_t tile,
   mark_grid(ctx, n_tiles, 1024, 1, &grid, &block);
   bool vec = aligned_to(out, MODE == CWM_SV16 ? 8 : 16);
   for (int j = 0; j < d.nd; ++j) vec &= aligned_to(d.fk[j], 16);
-  OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(cwm_probe_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kStageBytes));
-  cwm_probe_kernel<MODE><<<grid, block, static_cast<size_t>(d.smem), ctx->stream>>>(
-      d, n, vec, tile, n_tiles, out, mk, count, &ctx->counters->range_errors);
+  auto* const kernel = vec ? cwm_probe_kernel<MODE, true> : cwm_probe_kernel<MODE, false>;
+  OLAP_CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes));
+  kernel<<<grid, block, static_cast<size_t>(d.smem), ctx->stream>>>(d, n, tile, n_tiles, out, mk, count,
+                                                                  &ctx->counters->range_errors);
   OLAP_CUDA_TRY(ctx, cudaGetLastError());
   return OLAP_OK;
 }

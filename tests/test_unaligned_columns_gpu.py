@@ -26,3 +26,38 @@ def test_select_unaligned(ctx, n):
         full = np.zeros(32 * ((n + 31) // 32), bool)
         full[:n] = want
         assert np.array_equal(np.unpackbits(bits, bitorder="little").astype(bool), full)
+
+
+@pytest.mark.parametrize("moved", ["one key column", "output"])
+@pytest.mark.parametrize("n", [1, 31, 33, 127, 129, 1025, 700_001])
+def test_column_wise_probes_unaligned(ctx, n, moved):
+    import torch
+    from memory_database_b200 import olapcore, operators as ops
+    rng = np.random.default_rng(n)
+    lens, fk = (900, 40, 70_001, 7), []
+    vec = [rng.integers(0, 15, m).astype(np.int8) for m in lens]
+    for v in vec:
+        v[rng.random(len(v)) < 0.3] = 127
+    for m in lens:
+        k = rng.integers(0, m, n).astype(np.int32)
+        bad = rng.random(n) < 0.01
+        k[bad] = rng.choice([-1, m], bad.sum())
+        fk.append(k)
+    ok = np.all([(k >= 0) & (k < m) for k, m in zip(fk, lens)], axis=0)
+    codes = [v[np.where(ok, k, 0)].astype(np.int64) for v, k in zip(vec, fk)]
+    live = ok & np.all([c != 127 for c in codes], axis=0)
+    g = sum(c << s for c, s in zip(codes, (12, 8, 4, 0)))
+    dv = [torch.from_numpy(v).cuda() for v in vec]
+    dk = [shifted(k) if moved == "one key column" and j == 2 else torch.from_numpy(k).cuda() for j, k in enumerate(fk)]
+    pad = 1 if moved == "output" else 0
+    out = torch.empty(n + pad, dtype=torch.int32, device="cuda")[pad:]
+    assert ops.starjoinalgo_cwm_sv(n, *dv, *dk, out, ctx=ctx) == live.sum()
+    assert np.array_equal(out.cpu().numpy(), np.where(live, g, 32767))
+    k, pos, grp = ops.starjoinalgo_cwm_dv(n, *dv, *dk, ctx=ctx)
+    assert k == live.sum() and np.array_equal(pos.cpu().numpy(), np.flatnonzero(live))
+    assert np.array_equal(grp.cpu().numpy(), g[live])
+    gid = torch.empty(n + pad, dtype=torch.int16, device="cuda")[pad:]
+    olapcore.join_cwm_sv(dv, dk, [0, 1, 2, 3], 4, gid, [1, 2, 3, 4], n, ctx=ctx)
+    want = sum(c * f for c, f in zip(codes, (1, 2, 3, 4)))
+    assert np.array_equal(gid.cpu().numpy(), np.where(live, want, 32767).astype(np.int16))
+    assert ctx.take_range_errors() == 3 * (~ok).sum()
