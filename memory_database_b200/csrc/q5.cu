@@ -31,18 +31,20 @@ __device__ __forceinline__ bool nation_ok(uint64_t mask, int32_t n) {
 
 // What the supplier and order vectors hold for nation n: -1 when its region does
 // not pass, else its rank among the region's nations (equal ranks are equal
-// nations, and up to 15 of them fit 4 bits), or the nation itself in a region
-// of more than 15.
+// nations).  4 bits hold the rank modulo 15, and 15 for none: the rank itself in
+// a region of at most 15 nations, else a filter.
 constexpr int kQ5MaxCodes = 15;
-__device__ __forceinline__ int32_t q5_code(uint64_t mask, bool ranks, int32_t n) {
-  if (!nation_ok(mask, n)) return -1;
-  return ranks ? __popcll(mask & ((1ull << n) - 1ull)) : n;
+__device__ __forceinline__ int32_t q5_code(uint64_t mask, int32_t n) {
+  return nation_ok(mask, n) ? __popcll(mask & ((1ull << n) - 1ull)) : -1;
+}
+__device__ __forceinline__ uint32_t q5_low(int32_t code) {
+  return code < 0 ? 15u : static_cast<uint32_t>(code) % static_cast<uint32_t>(kQ5MaxCodes);
 }
 
 // Before the passes, in one launch: the region's nations as a bit mask
 // (set_bitmap, every block for itself, block 0 for the later kernels), the
-// supplier vector and its 4-bit codes (two suppliers per thread, 15 = none; of
-// use while the region has at most 15 nations), and zeroes in the sums.
+// supplier vector and its 4-bit codes (two suppliers per thread), and zeroes in
+// the sums.
 __global__ void __launch_bounds__(256) q5_prepare_kernel(const int32_t* __restrict__ r_regionkey, int64_t n_region,
                                                          const int32_t* __restrict__ n_regionkey, int64_t n_nation,
                                                          int32_t region, const int32_t* __restrict__ s_nationkey,
@@ -59,7 +61,6 @@ __global__ void __launch_bounds__(256) q5_prepare_kernel(const int32_t* __restri
   }
   __syncthreads();
   const uint64_t nmask = s_half[0] | (static_cast<uint64_t>(s_half[1]) << 32);
-  const bool ranks = __popcll(nmask) <= kQ5MaxCodes;
   if (blockIdx.x == 0) {
     if (n == 0) *d_mask = nmask;
     if (n < n_nation) sums[n] = 0;
@@ -67,11 +68,11 @@ __global__ void __launch_bounds__(256) q5_prepare_kernel(const int32_t* __restri
   const int64_t nbytes = (n_supp + 1) >> 1;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < nbytes; i += stride) {
-    const int32_t lo = q5_code(nmask, ranks, s_nationkey[2 * i]);
-    const int32_t hi = 2 * i + 1 < n_supp ? q5_code(nmask, ranks, s_nationkey[2 * i + 1]) : -1;
+    const int32_t lo = q5_code(nmask, s_nationkey[2 * i]);
+    const int32_t hi = 2 * i + 1 < n_supp ? q5_code(nmask, s_nationkey[2 * i + 1]) : -1;
     dim_s[2 * i] = static_cast<int8_t>(lo);
     if (2 * i + 1 < n_supp) dim_s[2 * i + 1] = static_cast<int8_t>(hi);
-    nib[i] = static_cast<uint8_t>((lo & 15) | (hi & 15) << 4);
+    nib[i] = static_cast<uint8_t>(q5_low(lo) | q5_low(hi) << 4);
   }
 }
 
@@ -82,8 +83,7 @@ __global__ void q5_orders_kernel(const int32_t* __restrict__ o_custkey, const in
   __shared__ int8_t s_code[kQ5MaxNations];  // by nation: 25 us per 15M orders; 34 us with the rank counted per order
   if (threadIdx.x < kQ5MaxNations) {
     const uint64_t nmask = *d_mask;
-    s_code[threadIdx.x] =
-        static_cast<int8_t>(q5_code(nmask, __popcll(nmask) <= kQ5MaxCodes, static_cast<int32_t>(threadIdx.x)));
+    s_code[threadIdx.x] = static_cast<int8_t>(q5_code(nmask, static_cast<int32_t>(threadIdx.x)));
   }
   __syncthreads();
   auto code = [&](int32_t n) -> int32_t { return static_cast<uint32_t>(n) < kQ5MaxNations ? s_code[n] : -1; };
@@ -132,54 +132,43 @@ __global__ void q5_orders_kernel(const int32_t* __restrict__ o_custkey, const in
 
 // Price and discount are read only for the lines that match (a fifth of the
 // suppliers, a seventh of the orders and equal nations leave about one in
-// 175): two thirds of their sectors are never read.
+// 175, so one in 22 of their sectors).
 // kStaged: the 4-bit supplier codes in shared memory (half the bytes of the
-// int8 vector, so four blocks fit an SM), unless the region has more than 15
-// nations; else the int8 vector through L1/L2.  Lines that drop out
-// are carried along without a branch, and codes are compared, not nations.
+// int8 vector, so four blocks fit an SM); in a region of more than 15 nations
+// they only filter, and the lines whose order passes and agrees in the 4 bits
+// look the code itself up.  Else the int8 vector through L1/L2.  Lines that drop
+// out are carried along without a branch, and codes are compared, not nations.
 // Bound by the order gathers' sectors and by instructions: 60M lines, 100,000
-// suppliers, 173 us (all four columns read, branches, nations) -> 151 us (late
-// reads) -> 115 us.
-template <bool kStaged>
-__global__ void __launch_bounds__(512, 4) q5_lines_kernel(
-    const int32_t* __restrict__ l_suppkey, const int32_t* __restrict__ l_order, const int32_t* __restrict__ price,
-    const int32_t* __restrict__ disc, int64_t n_lines, const int8_t* __restrict__ dim_s, int64_t n_supp,
-    const uint8_t* __restrict__ nib_s, const unsigned long long* __restrict__ d_mask,
-    const int8_t* __restrict__ dim_o, int64_t n_orders, unsigned long long* __restrict__ sums,
-    unsigned long long* range_err) {
-  extern __shared__ __align__(16) uint32_t s_nib[];  // kStaged: eight codes per word
-  __shared__ unsigned long long s_sum[kQ5MaxNations];  // by code
-  __shared__ int8_t s_nat[kQ5MaxNations];              // code -> nation
-  const int tid = threadIdx.x;
-  const uint64_t nmask = *d_mask;
-  const bool ranks = __popcll(nmask) <= kQ5MaxCodes;
-  const bool staged = kStaged && ranks;
-  for (int i = tid; i < kQ5MaxNations; i += blockDim.x) {
-    s_sum[i] = 0;
-    if (!ranks) s_nat[i] = static_cast<int8_t>(i);
-    else if (nation_ok(nmask, i)) s_nat[q5_code(nmask, true, i)] = static_cast<int8_t>(i);
-  }
-  if (staged) {
-    const int64_t nbytes = (n_supp + 1) >> 1;
-    for (int64_t i = tid; i < (nbytes >> 2); i += blockDim.x) s_nib[i] = __ldg(reinterpret_cast<const uint32_t*>(nib_s) + i);
-    for (int64_t i = (nbytes & ~int64_t(3)) + tid; i < nbytes; i += blockDim.x) reinterpret_cast<uint8_t*>(s_nib)[i] = nib_s[i];
-  }
-  __syncthreads();
-  // code of supplier row s (0-based): 15 or -1 when it is not in the region
+// suppliers, 5 nations of 25: 174 us with all four columns read, branches and
+// nations, 159 us so.  A region of all 25: 516 us so, 927 us with every
+// supplier's code through the little L1 that the staging leaves, 534 us with the
+// filter (16 of them: 451, 741 and 352 us).
+template <bool kStaged, bool kMany>
+__device__ __forceinline__ unsigned int q5_scan_lines(const int32_t* __restrict__ l_suppkey, const int32_t* __restrict__ l_order,
+                                              const int32_t* __restrict__ price, const int32_t* __restrict__ disc,
+                                              int64_t n_lines, const int8_t* __restrict__ dim_s, int64_t n_supp,
+                                              const uint32_t* s_nib, const int8_t* __restrict__ dim_o,
+                                              int64_t n_orders, unsigned long long* s_sum) {
+  unsigned int bad = 0;  // lines with a key out of range: the result
+  // what is known of supplier row s (0-based) before its order is: its 4 bits
+  // (15: not in the region), else its code (-1)
   auto scode = [&](uint32_t s) -> int32_t {
-    return staged ? static_cast<int32_t>(s_nib[s >> 3] >> ((s << 2) & 31u)) & 15 : __ldg(dim_s + s);
+    return kStaged ? static_cast<int32_t>(s_nib[s >> 3] >> ((s << 2) & 31u)) & 15 : __ldg(dim_s + s);
   };
-  const int32_t none = staged ? 15 : -1;
+  constexpr int32_t none = kStaged ? 15 : -1;
+  // the order's code agrees with it (kMany: in the 4 bits)
+  auto same = [&](int32_t c, int32_t o) -> bool {
+    return kMany ? o >= 0 && static_cast<uint32_t>(c) == q5_low(o) : c == o && c != none;
+  };
   const uint32_t n_s = static_cast<uint32_t>(n_supp < INT32_MAX ? n_supp : INT32_MAX);
   const uint32_t n_o = static_cast<uint32_t>(n_orders <= INT32_MAX ? n_orders : int64_t(INT32_MAX) + 1);
   const uint64_t pol = policy_evict_first();
   const uint64_t keep = policy_evict_last();
-  unsigned int bad = 0;
   auto add = [&](int32_t code, int64_t r) {
     smem_add_u64(&s_sum[code], static_cast<uint64_t>(static_cast<int64_t>(__ldg(price + r)) * (100 - __ldg(disc + r))));
   };
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + tid;
+  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool vec = ((reinterpret_cast<uintptr_t>(l_suppkey) | reinterpret_cast<uintptr_t>(l_order)) & 15) == 0;
   const int64_t n4 = vec && n_s && n_o ? n_lines >> 2 : 0;
   for (int64_t i = t0; i < n4; i += stride) {
@@ -204,9 +193,13 @@ __global__ void __launch_bounds__(512, 4) q5_lines_kernel(
     for (int e = 0; e < 4; ++e) cs[e] = scode(sk[e]);
 #pragma unroll
     for (int e = 0; e < 4; ++e) co[e] = static_cast<int8_t>(ld_probe_s8_if(cs[e] != none, dim_o + ok[e], keep, -2));
+    if (kMany) {  // the few lines that agree so far: their suppliers' codes, all of them in flight
+#pragma unroll
+      for (int e = 0; e < 4; ++e) cs[e] = same(cs[e], co[e]) ? __ldg(dim_s + sk[e]) : -1;
+    }
 #pragma unroll
     for (int e = 0; e < 4; ++e)
-      if (cs[e] == co[e] && cs[e] != none && !((out >> e) & 1u)) add(cs[e], 4 * i + e);
+      if (!((out >> e) & 1u) && (kMany ? cs[e] == co[e] && cs[e] >= 0 : same(cs[e], co[e]))) add(co[e], 4 * i + e);
   }
   for (int64_t r = 4 * n4 + t0; r < n_lines; r += stride) {
     const uint32_t sk = static_cast<uint32_t>(l_suppkey[r]) - 1u, ok = static_cast<uint32_t>(l_order[r]);
@@ -214,9 +207,41 @@ __global__ void __launch_bounds__(512, 4) q5_lines_kernel(
       ++bad;
       continue;
     }
-    const int32_t c = scode(sk);
-    if (c != none && dim_o[ok] == c) add(c, r);
+    const int32_t o = dim_o[ok];
+    if (same(scode(sk), o) && (!kMany || __ldg(dim_s + sk) == o)) add(o, r);
   }
+  return bad;
+}
+
+template <bool kStaged>
+__global__ void __launch_bounds__(512, 4) q5_lines_kernel(
+    const int32_t* __restrict__ l_suppkey, const int32_t* __restrict__ l_order, const int32_t* __restrict__ price,
+    const int32_t* __restrict__ disc, int64_t n_lines, const int8_t* __restrict__ dim_s, int64_t n_supp,
+    const uint8_t* __restrict__ nib_s, const unsigned long long* __restrict__ d_mask,
+    const int8_t* __restrict__ dim_o, int64_t n_orders, unsigned long long* __restrict__ sums,
+    unsigned long long* range_err) {
+  extern __shared__ __align__(16) uint32_t s_nib[];  // kStaged: eight codes per word
+  __shared__ unsigned long long s_sum[kQ5MaxNations];  // by code
+  __shared__ int8_t s_nat[kQ5MaxNations];              // code -> nation
+  const int tid = threadIdx.x;
+  const uint64_t nmask = *d_mask;
+  for (int i = tid; i < kQ5MaxNations; i += blockDim.x) {
+    s_sum[i] = 0;
+    if (nation_ok(nmask, i)) s_nat[q5_code(nmask, i)] = static_cast<int8_t>(i);
+  }
+  if (kStaged) {
+    const int64_t nbytes = (n_supp + 1) >> 1;
+    for (int64_t i = tid; i < (nbytes >> 2); i += blockDim.x) s_nib[i] = __ldg(reinterpret_cast<const uint32_t*>(nib_s) + i);
+    for (int64_t i = (nbytes & ~int64_t(3)) + tid; i < nbytes; i += blockDim.x) reinterpret_cast<uint8_t*>(s_nib)[i] = nib_s[i];
+  }
+  __syncthreads();
+  // (two instances: what a line costs more in a large region is not paid in others)
+  const unsigned int bad =
+      kStaged && __popcll(nmask) > kQ5MaxCodes
+          ? q5_scan_lines<kStaged, kStaged>(l_suppkey, l_order, price, disc, n_lines, dim_s, n_supp, s_nib, dim_o,
+                                            n_orders, s_sum)
+          : q5_scan_lines<kStaged, false>(l_suppkey, l_order, price, disc, n_lines, dim_s, n_supp, s_nib, dim_o,
+                                          n_orders, s_sum);
   const unsigned int wbad = __reduce_add_sync(0xffffffffu, bad);
   if ((tid & 31) == 0 && wbad) atomicAdd(range_err, static_cast<unsigned long long>(wbad));
   __syncthreads();
