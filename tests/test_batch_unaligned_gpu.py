@@ -18,14 +18,15 @@ def shifted(x, by):
 
 @pytest.mark.parametrize("agg", [olapcore.AGG_M1_PLUS_M2, olapcore.AGG_M2])
 @pytest.mark.parametrize("probe", [0, 1])
+@pytest.mark.parametrize("n_queries", [1, 2, 3, 16])
 @pytest.mark.parametrize("rows", [1, 4, 5, 131, 70_003])
-def test_shifted_columns(ctx, rows, probe, agg):
+def test_shifted_columns(ctx, rows, probe, agg, n_queries):
     rng = np.random.default_rng(rows)
     sizes, groups = (3000, 500, 800, 60), (5, 5, 4, 7)
     dims = batch.make_dim_tables(ctx, sizes, groups)
     fk = [rng.integers(0, n, rows).astype(np.int32) for n in sizes]
     m1, m2 = (rng.integers(-2**31, 2**31, rows).astype(np.int32) for _ in range(2))
-    qs = batch.random_queries(rng, 16, rows, groups, sel_range=(0.3, 1.0))
+    qs = batch.random_queries(rng, n_queries, rows, groups, sel_range=(0.3, 1.0))
     eng = batch.BatchEngine(ctx, dims)
     try:
         eng.tune(512, 4096, probe)
