@@ -770,17 +770,17 @@ __global__ void smem_region_taken_kernel(const uint64_t* __restrict__ taken, con
 
 // A bucket (four slots, 32 bytes) of the hash table, marked evict-last in L2:
 // every probe re-reads the table at random while the probe keys stream past
-// it once, so the part of the table that L2 holds should stay there.  The
-// 64-byte prefetch size asks L2 to fetch only the 64 bytes around the bucket
-// on a miss: 36 instead of 57 bytes of DRAM per probe (2^24 probes, 256 MB
-// table), for about 5 % more time per probe.  kWide: one 32-byte load (the
-// table is 32-byte aligned); a random load costs L1 a cycle per lane, so two
-// 16-byte ones cost twice that.  The address is always inside the table (the
+// it once, so the part of the table that L2 holds should stay there.  kWide: one
+// 32-byte load (the table is 32-byte aligned); a random load costs L1 a cycle
+// per lane, so two 16-byte ones cost twice that.  Those ask L2 to fetch 64 bytes
+// on a miss; the 32-byte one does without: 2^27 probes of a 256 MB table 1,243 us
+// with that hint and 1,207 us without where half of them match, 2,553 and
+// 2,445 us where all do.  The address is always inside the table (the
 // callers' guards may be moved past this load).
 template <bool kWide>
 __device__ __forceinline__ void ld_bucket(const uint64_t* p, uint64_t (&s)[4]) {
   if (kWide) {
-    asm("ld.global.nc.L2::cache_hint.L2::64B.v4.u64 {%0,%1,%2,%3}, [%4], %5;"
+    asm("ld.global.nc.L2::cache_hint.v4.u64 {%0,%1,%2,%3}, [%4], %5;"
         : "=l"(s[0]), "=l"(s[1]), "=l"(s[2]), "=l"(s[3])
         : "l"(p), "l"(policy_evict_last()));
   } else {
