@@ -682,7 +682,13 @@ __global__ void __launch_bounds__(V == 8 ? 512 : 1024, 1) starjoin_vec_kernel(co
 //    row, when few lanes of the warp had one in the step before (kLateLanes):
 //    at 1 % survivors that leaves 17 of the 24 bytes per row.  They arrive
 //    while the next step's rows are probed and are added up there, so no step
-//    waits for them; with more survivors they are read with the keys.
+//    waits for them; with more survivors they are read with the keys.  (60M
+//    rows of which 10 % survive, at 4, 7, 10, 14 and 20 lanes: 290, 289, 285,
+//    294 and 297 us with four dimensions, 356, 349, 327, 321 and 326 with two; at
+//    1 % and from 25 % on all the same.)  With one dimension they are always
+//    read with the keys: its scan is short enough that the second form costs
+//    more than the bytes it saves (a staged dimension that keeps 1 %: 130 us with
+//    it, 112 us without; one in L2 that keeps a fifth: 282 and 264 us).
 constexpr int kLateLanes = 10;
 
 template <int ND, int ACC, int AGGK>
@@ -891,7 +897,7 @@ __global__ void __launch_bounds__(1024, 1) starjoin_scan_kernel(const StarParams
         add_pending();
       }
     }
-    late = lanes <= kLateLanes;
+    late = ND > 1 && lanes <= kLateLanes;
   }
   if (pend) add_pending();
   if (bad & kMetOob) {  // rare: this thread's rows once more, for the range errors among them
