@@ -99,7 +99,9 @@ class Context:
         if self._fixed_stream:
             return
         torch = _torch()
-        raw = torch._C._cuda_getCurrentRawStream(self.device)  # current_stream() builds a Stream object: 1.5 us more
+        # current_stream() builds a Stream object: 1.5 us more than the raw handle, which no torch promises
+        raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        raw = raw_stream(self.device) if raw_stream else torch.cuda.current_stream(self.device).cuda_stream
         if raw != self._cur_stream:
             check(lib.olap_ctx_set_stream(self.handle, C.c_void_p(raw) if raw else None), self.handle)
             self._cur_stream = raw
