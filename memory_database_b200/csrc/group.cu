@@ -142,6 +142,7 @@ __device__ __forceinline__ void global_add(const HashAgg& t, int32_t k, uint64_t
 constexpr int kAggThreads = 1024;
 constexpr int kAggSlots = 8192;  // 16 B per slot: 128 KB of shared memory
 constexpr int kAggMaxSlots = 14336;  // 224 KB: the partitions' tables of many groups
+static_assert(kAggSlots % kAggThreads == 0 && kAggMaxSlots % kAggThreads == 0, "whole merge blocks");
 
 struct SmemAgg {
   int32_t* key;
@@ -1058,58 +1059,85 @@ __global__ void __launch_bounds__(kAggThreads) group_part_agg_kernel(
   append_groups(st, capacity, out_keys, out_sums, out_counts, d_groups, overflow);
 }
 
-// One block per split partition: adds up its slices' tables in a shared table
-// and appends the groups.
+// Adds up the tables of a split partition's slices and appends the groups.  A
+// block takes the keys of kMergeSlots slots' home buckets, so that a partition
+// is merged by slots / kMergeSlots blocks (one block for all of it took 886 us
+// for the 111 tables of a key that half of 2^26 rows have, 81 us so): in
+// each table those keys lie in these slots and in the full buckets that follow
+// (a run ends at a bucket with a free slot, and the tables have the same layout
+// and hash).
+constexpr uint32_t kMergeSlots = kAggThreads;
 __global__ void __launch_bounds__(kAggThreads) group_part_merge_kernel(
     const AggUnits* __restrict__ units, const int4* __restrict__ partials, uint32_t slots, int64_t capacity,
     int32_t* __restrict__ out_keys, int64_t* __restrict__ out_sums, int64_t* __restrict__ out_counts,
     unsigned long long* d_groups, unsigned long long* overflow, const unsigned long long* timeouts) {
   if (blockIdx.x == 0 && threadIdx.x == 0) overflow[1] = *timeouts;  // beside the overflow count, for the caller's one copy
-  if (static_cast<int>(blockIdx.x) >= units->n_merges) return;
-  const int2 m = units->merge[blockIdx.x];
   extern __shared__ __align__(16) unsigned char agg_smem[];
   const SmemAgg st = smem_agg(agg_smem, slots);
-  unsigned int lost = 0;
-  // the first table as it is (same layout and hash), then the slots of the
-  // others, four per thread with their key lookups in flight together
-  int4* dst = reinterpret_cast<int4*>(agg_smem);
-  for (uint32_t i = threadIdx.x; i < slots; i += blockDim.x) dst[i] = partials[static_cast<int64_t>(m.x) * slots + i];
-  __syncthreads();
-  for (int q = 1; q < m.y; ++q) {
-    const SmemAgg pt = smem_agg(reinterpret_cast<unsigned char*>(const_cast<int4*>(partials) +
-                                                                 static_cast<int64_t>(m.x + q) * slots),
-                                slots);
-    for (uint32_t i0 = 0; i0 < slots; i0 += 4 * kAggThreads) {
+  const int shares = static_cast<int>(slots / kMergeSlots), work = units->n_merges * shares;
+  for (int w = blockIdx.x; w < work; w += gridDim.x) {  // (usually none)
+    const int2 m = units->merge[w / shares];
+    smem_agg_clear(st);
+    __syncthreads();
+    const uint32_t first = static_cast<uint32_t>(w % shares) * kMergeSlots;  // slots [first, first + kMergeSlots)
+    auto table = [&](int q) {
+      return smem_agg(reinterpret_cast<unsigned char*>(const_cast<int4*>(partials) +
+                                                       static_cast<int64_t>(m.x + q) * slots),
+                      slots);
+    };
+    auto mine = [&](int32_t k) {
+      return k != kEmptyKey && 4 * st.home(k) - first < kMergeSlots;  // its home bucket lies in this block's slots
+    };
+    unsigned int lost = 0;
+    auto add = [&](int32_t k, uint32_t lo, uint32_t hi, uint32_t c) {
+      const int at = smem_find_insert(st, k, st.home(k));
+      if (at < 0) {
+        ++lost;
+        return;
+      }
+      const uint32_t old = atomicAdd(st.lo + at, lo);
+      const uint32_t h = hi + static_cast<uint32_t>(agg_high(old, static_cast<int32_t>(lo)));
+      if (h) atomicAdd(st.lo + slots + at, h);
+      atomicAdd(st.cnt + at, c);
+    };
+    // this block's slots, a thread each, four tables in flight
+    const uint32_t i = first + threadIdx.x;
+    for (int q0 = 0; q0 < m.y; q0 += 4) {
       int32_t k[4];
       uint32_t lo[4], hi[4], c[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const uint32_t i = i0 + u * kAggThreads + threadIdx.x;
-        const bool in = i < slots;
-        k[u] = in ? pt.key[i] : kEmptyKey;
-        lo[u] = in ? pt.lo[i] : 0u;
-        hi[u] = in ? pt.lo[slots + i] : 0u;
-        c[u] = in ? pt.cnt[i] : 0u;
+        const bool in = q0 + u < m.y;
+        const SmemAgg t = table(in ? q0 + u : q0);
+        k[u] = in ? t.key[i] : kEmptyKey;
+        lo[u] = t.lo[i];
+        hi[u] = t.lo[slots + i];
+        c[u] = t.cnt[i];
       }
-      int at[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) at[u] = k[u] != kEmptyKey ? smem_find_insert(st, k[u], st.home(k[u])) : -2;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (at[u] < 0) {
-          lost += at[u] == -1;
-          continue;
-        }
-        const uint32_t old = atomicAdd(st.lo + at[u], lo[u]);
-        const uint32_t h = hi[u] + static_cast<uint32_t>(agg_high(old, static_cast<int32_t>(lo[u])));
-        if (h) atomicAdd(st.lo + slots + at[u], h);
-        atomicAdd(st.cnt + at[u], c[u]);
+      for (int u = 0; u < 4; ++u)
+        if (mine(k[u])) add(k[u], lo[u], hi[u], c[u]);
+    }
+    // the full buckets behind them, a warp on a table, a lane per slot
+    const uint32_t lane = threadIdx.x & 31u;
+    for (int q = threadIdx.x >> 5; q < m.y; q += kAggThreads / 32) {
+      const SmemAgg t = table(q);
+      uint32_t b = (first + kMergeSlots) / 4 - 1;  // the last of its own buckets
+      for (uint32_t step = 0; step < t.nb; ++step) {
+        const int4 x = *reinterpret_cast<const int4*>(t.key + 4 * b);
+        if (x.x == kEmptyKey || x.y == kEmptyKey || x.z == kEmptyKey || x.w == kEmptyKey) break;
+        b = t.next(b);
+        if (b == first / 4) break;  // all the way round
+        if (lane < 4 && mine(t.key[4 * b + lane]))
+          add(t.key[4 * b + lane], t.lo[4 * b + lane], t.lo[slots + 4 * b + lane], t.cnt[4 * b + lane]);
+        __syncwarp();
       }
     }
+    if (lost) atomicAdd(overflow, static_cast<unsigned long long>(lost));
+    __syncthreads();
+    append_groups(st, capacity, out_keys, out_sums, out_counts, d_groups, overflow);
+    __syncthreads();  // the table is cleared next
   }
-  if (lost) atomicAdd(overflow, static_cast<unsigned long long>(lost));
-  __syncthreads();
-  append_groups(st, capacity, out_keys, out_sums, out_counts, d_groups, overflow);
 }
 
 // The global table of plan 1 empty, and the counters zero (one launch).
@@ -1500,7 +1528,7 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
       }
       // a split partition has at least two slices
       if (e == cudaSuccess)
-        olap::group_part_merge_kernel<<<olap::kMaxPartials / 2, olap::kAggThreads, asmem, ctx->stream>>>(
+        olap::group_part_merge_kernel<<<ctx->sm_count, olap::kAggThreads, asmem, ctx->stream>>>(
             d_units, d_partials, pp.slots, capacity, out_keys, out_sums, out_counts, d_groups_u, overflow,
             &ctx->counters->wait_timeouts);
       if (e == cudaSuccess) e = cudaGetLastError();
