@@ -1443,6 +1443,15 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
         break;
       }
     }
+    if (!tile_g) {
+      // The scatter keeps a cursor per partition only, and so many partitions
+      // have few rows each: clearing and emptying a table is what it costs.
+      // Small ones, as few as hold `capacity` distinct keys (7,650 of 8,192
+      // slots): 20M rows of 20M keys 600 us in the aggregation, 722 us with
+      // tables of 14,336 slots.
+      pp.slots = olap::kAggSlots;
+      waves = (capacity + 7650 * sms - 1) / (7650 * sms);
+    }
     pp.n_parts = static_cast<int32_t>(waves * sms);
     pp.n_blocks = ctx->sm_count * 2;
     pp.per = ((n + pp.n_blocks - 1) / pp.n_blocks + 3) & ~int64_t(3);

@@ -51,3 +51,20 @@ def test_hot_keys(ctx, max_groups, hot):
     keys = np.where(rng.random(n) < 0.97, rng.integers(0, hot, n), rng.integers(0, max_groups, n)).astype(np.int32)
     vals = rng.integers(-2**31, 2**31, n).astype(np.int32)
     check(ctx, keys, vals, None, max_groups)
+
+
+@pytest.mark.parametrize("share", [0.5, 1.0])
+def test_large_capacity_filled(ctx, share):
+    """More partitions than the tiled scatter keeps: as many distinct keys as asked for, and as the outputs hold."""
+    import torch
+    from memory_database_b200 import operators as ops
+    n = int((1 << 26) * share)
+    keys = torch.arange(n, dtype=torch.int32, device="cuda") * 63  # distinct modulo 2^32
+    keys = torch.where(keys == -2**31, torch.full_like(keys, -63), keys)  # the reserved key
+    k, s, c = ops.group_hash(keys, keys, max_groups=1 << 25, ctx=ctx)
+    want = torch.sort(torch.unique(keys))[0]
+    order = torch.argsort(k)
+    assert torch.equal(k[order], want)
+    assert int(c.sum()) == n and int(s.sum()) == int(keys.sum(dtype=torch.int64))
+    once = c[order] == 1
+    assert torch.equal(s[order][once], want[once].long())
