@@ -284,6 +284,45 @@ __global__ void __launch_bounds__(1024, 1) cwm_probe_kernel(const DimSet d, int6
   }
 }
 
+// The *_sv vectors of few rows: a thread per row and nothing staged, so a short
+// kernel.  Four dimensions, 10,000 rows: 3.0 us, cwm_probe_kernel 5.4; 500,000
+// rows 7.3 and 8.7 us, 1M rows 10.9 and 10.4, 2M rows 17.9 and 14.1.
+constexpr int64_t kFewRows = 1 << 20;
+template <int MODE>
+__global__ void __launch_bounds__(256) cwm_few_rows_kernel(const DimSet d, int64_t n, void* __restrict__ out,
+                                                           unsigned long long* count, unsigned long long* range_err) {
+  const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  uint32_t k[OLAP_MAX_DIMS];
+  bool ok = true, live = r < n;
+#pragma unroll
+  for (int j = 0; j < OLAP_MAX_DIMS; ++j) {
+    if (j >= d.nd) continue;
+    k[j] = live ? static_cast<uint32_t>(d.fk[j][r]) : 0u;
+    ok &= k[j] < d.len[j];
+  }
+  const bool bad = live && !ok;
+  live &= ok;
+  int32_t g = 0;
+#pragma unroll
+  for (int j = 0; j < OLAP_MAX_DIMS; ++j) {
+    if (j >= d.nd || !live) continue;
+    const int32_t c = __ldg(d.vec[j] + k[j]);
+    live = c != OLAP_DIM_NULL;
+    g += c * d.mul[j];
+  }
+  const int32_t v = live ? g : OLAP_GROUP_NULL;
+  if (r < n) {
+    if (MODE == CWM_SV16) static_cast<int16_t*>(out)[r] = static_cast<int16_t>(v);
+    else static_cast<int32_t*>(out)[r] = v;
+  }
+  const uint32_t wbad = __popc(__ballot_sync(0xffffffffu, bad));
+  const uint32_t some = MODE == CWM_SV32 ? __popc(__ballot_sync(0xffffffffu, v != OLAP_GROUP_NULL)) : 0u;
+  if ((threadIdx.x & 31) == 0) {
+    if (wbad) atomicAdd(range_err, static_cast<unsigned long long>(wbad));
+    if (some) atomicAdd(count, static_cast<unsigned long long>(some));
+  }
+}
+
 // The surviving rows of join_cwm_dv (int64 OID, int16 group) ...
 struct OidEmit {
   static constexpr bool kVals = true;
@@ -489,6 +528,12 @@ static int launch_probe(olap_ctx* ctx, const DimSet& d, int64_t n, int32_t tile,
 // One value per row (the *_sv vectors).
 template <int MODE>
 static int row_vector(olap_ctx* ctx, DimSet d, int64_t n, void* out, unsigned long long* count) {
+  if (n <= kFewRows) {
+    cwm_few_rows_kernel<MODE><<<static_cast<unsigned>((n + 255) / 256), 256, 0, ctx->stream>>>(
+        d, n, out, count, &ctx->counters->range_errors);
+    OLAP_CUDA_TRY(ctx, cudaGetLastError());
+    return OLAP_OK;
+  }
   stage_plan(&d, n);
   const int64_t tile = std::min<int64_t>(mark_tile(n, ctx->sm_count * int64_t(32)), 1 << 20);
   return launch_probe<MODE>(ctx, d, n, static_cast<int32_t>(tile), out, Marks{}, count);

@@ -61,3 +61,27 @@ def test_column_wise_probes_unaligned(ctx, n, moved):
     want = sum(c * f for c, f in zip(codes, (1, 2, 3, 4)))
     assert np.array_equal(gid.cpu().numpy(), np.where(live, want, 32767).astype(np.int16))
     assert ctx.take_range_errors() == 3 * (~ok).sum()
+
+
+@pytest.mark.parametrize("nd", [0, 1, 3])
+@pytest.mark.parametrize("n", [1, 255, 257, (1 << 20) - 1, 1 << 20, (1 << 20) + 1])
+def test_vector_of_few_rows(ctx, n, nd):
+    """Both sides of the size up to which the vector takes a thread per row."""
+    import torch
+    from memory_database_b200 import olapcore
+    rng = np.random.default_rng(n + nd)
+    lens, factor = (900, 40, 70_001)[:nd], [1, 7, 50][:nd]
+    vec = [np.where(rng.random(m) < 0.3, 127, rng.integers(-3, 15, m)).astype(np.int8) for m in lens]
+    fk = [np.where(rng.random(n) < 0.01, rng.choice([-1, m], n), rng.integers(0, m, n)).astype(np.int32) for m in lens]
+    ok, live, g = np.ones(n, bool), np.ones(n, bool), np.zeros(n, np.int64)
+    for v, k, f in zip(vec, fk, factor):
+        ok &= (k >= 0) & (k < len(v))
+    for v, k, f in zip(vec, fk, factor):
+        c = v[np.where(ok, k, 0)].astype(np.int64)
+        live &= c != 127
+        g += c * f
+    gid = torch.empty(n, dtype=torch.int16, device="cuda")
+    olapcore.join_cwm_sv([torch.from_numpy(v).cuda() for v in vec], [torch.from_numpy(k).cuda() for k in fk],
+                         list(range(nd)), nd, gid, factor, n, ctx=ctx)
+    assert np.array_equal(gid.cpu().numpy(), np.where(live & ok, g, 32767).astype(np.int16))
+    assert ctx.take_range_errors() == (~ok).sum()
