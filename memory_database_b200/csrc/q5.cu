@@ -199,7 +199,7 @@ __device__ __forceinline__ unsigned int q5_scan_lines(const int32_t* __restrict_
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e)
-      if (!((out >> e) & 1u) && (kMany ? cs[e] == co[e] && cs[e] >= 0 : same(cs[e], co[e]))) add(co[e], 4 * i + e);
+      if ((kMany ? cs[e] == co[e] && cs[e] >= 0 : same(cs[e], co[e])) && !((out >> e) & 1u)) add(cs[e], 4 * i + e);
   }
   for (int64_t r = 4 * n4 + t0; r < n_lines; r += stride) {
     const uint32_t sk = static_cast<uint32_t>(l_suppkey[r]) - 1u, ok = static_cast<uint32_t>(l_order[r]);
