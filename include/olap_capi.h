@@ -93,8 +93,9 @@ typedef struct olap_ctx olap_ctx;
 
 /* ---- context ---------------------------------------------------------------
  * A context binds one device, one stream (its own unless set), a device
- * scratch arena (scratch_bytes, 0 = 64 MiB) and a pinned host staging buffer
- * for the _host entry points.  Calls on one context are serialised by a
+ * scratch arena (scratch_bytes, 0 = 64 MiB; row lists longer than it has room
+ * for are made in chunks) and a pinned host staging buffer for the _host entry
+ * points.  Calls on one context are serialised by a
  * mutex; use one context per host thread for concurrent submission. */
 OLAP_API int olap_ctx_create(int device, size_t scratch_bytes, olap_ctx** out);
 OLAP_API int olap_ctx_destroy(olap_ctx* ctx);
@@ -492,7 +493,7 @@ typedef struct olap_batch_query {
 } olap_batch_query;
 
 /* A batch engine for up to max_queries (<= 64) queries per launch; holds the
- * packed attribute records of the dimensions and two staging slots (so one
+ * packed attributes of the dimensions and two staging slots (so one
  * batch can be prepared while the previous one runs). */
 OLAP_API int olap_batch_create(olap_ctx* ctx, int max_queries, olap_batch** out);
 OLAP_API int olap_batch_destroy(olap_batch* b);
@@ -521,9 +522,9 @@ OLAP_API int olap_batch_graph_captures(olap_batch* b, int64_t* captures);
 OLAP_API int olap_batch_tune(olap_batch* b, int block, int smem_slots);
 /* Probe order of the batched scan: 0 (the default) probes the tables one
  * after another, each only for rows that still have a live query using it;
- * 1 reads every table's query mask in one round trip, then the group
- * attributes of the tables a surviving query groups by (needs blocks of at
- * most 512 threads; with larger ones the first order runs).  The autotuner
+ * 1 reads every used table's record (16 bits: the filter attribute's interval
+ * and the group code) in one round trip (needs blocks of at most 512 threads;
+ * with larger ones the first order runs).  The autotuner
  * tries both.  olap_batch_get_tuning reports the shape in force. */
 OLAP_API int olap_batch_set_probe(olap_batch* b, int parallel_probe);
 OLAP_API int olap_batch_get_tuning(olap_batch* b, int* block, int* smem_slots, int* parallel_probe);

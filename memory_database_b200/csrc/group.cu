@@ -1421,6 +1421,9 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
     int64_t waves = need(olap::kAggSlots, 3);
     if (waves > 2) {
       pp.slots = olap::kAggMaxSlots;
+      // at least three: 2^27 rows, scatter and aggregation, 2^20 groups in two
+      // waves 593 + 596 us and in three 613 + 457, 2^19 groups in one wave 573 +
+      // 620 us and in three 612 + 394
       waves = std::max<int64_t>(3, need(olap::kAggMaxSlots, 4));
     }
     // The tiled scatter keeps some words per partition in shared memory: with
