@@ -132,8 +132,8 @@ class BatchEngine:
 
     def tune(self, block: int, smem_slots: int, parallel_probe: int | None = None) -> None:
         """Launch shape of the scan (threads per block, shared accumulators,
-        optionally the probe order: 1 reads every table's mask in one round
-        trip)."""
+        optionally the probe order: 1 reads every used table's record in one
+        round trip)."""
         check(lib.olap_batch_tune(self._h, int(block), int(smem_slots)), self.ctx.handle)
         if parallel_probe is not None:
             check(lib.olap_batch_set_probe(self._h, int(parallel_probe)), self.ctx.handle)

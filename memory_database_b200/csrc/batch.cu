@@ -581,7 +581,7 @@ struct olap_batch {
   int64_t attr_len[OLAP_MAX_DIMS] = {};
   int block = olap::kBatchThreads;        // scan kernel block size (olap_batch_tune / _autotune)
   int smem_slots = olap::kBatchSmemSlots; // per-block shared accumulators
-  int parallel_probe = 0;                 // 1: every table's mask in one round trip (block <= 512)
+  int parallel_probe = 0;                 // 1: every table's record in one round trip (block <= 512)
 };
 
 extern "C" {
