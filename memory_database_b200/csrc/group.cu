@@ -1448,12 +1448,10 @@ int olap_group_hash(olap_ctx* ctx, int64_t n, const int32_t* keys, int32_t key_o
     }
     if (!tile_g) {
       // The scatter keeps a cursor per partition only, and so many partitions
-      // have few rows each: clearing and emptying a table is what it costs.
-      // Small ones, as few as hold `capacity` distinct keys (7,650 of 8,192
-      // slots): 20M rows of 20M keys 600 us in the aggregation, 722 us with
-      // tables of 14,336 slots.
-      pp.slots = olap::kAggSlots;
-      waves = (capacity + 7650 * sms - 1) / (7650 * sms);
+      // have few rows each: clearing and emptying a table is what one costs.  As
+      // few as hold `capacity` distinct keys, then (20M rows of 20M keys, scatter
+      // and aggregation: 9,472 partitions 520 + 722 us, 5,032 486 + 476).
+      waves = (capacity + 13600 * sms - 1) / (13600 * sms);
     }
     pp.n_parts = static_cast<int32_t>(waves * sms);
     pp.n_blocks = ctx->sm_count * 2;
