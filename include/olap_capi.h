@@ -94,8 +94,9 @@ typedef struct olap_ctx olap_ctx;
 /* ---- context ---------------------------------------------------------------
  * A context binds one device, one stream (its own unless set), a device
  * scratch arena (scratch_bytes, 0 = 64 MiB; row lists longer than it has room
- * for are made in chunks) and a pinned host staging buffer for the _host entry
- * points.  Calls on one context are serialised by a
+ * for are made in chunks, or, from three chunks on and outside of graph capture,
+ * in up to 64 MiB of the context's growing buffer, see olap_group_hash) and a
+ * pinned host staging buffer for the _host entry points.  Calls on one context are serialised by a
  * mutex; use one context per host thread for concurrent submission. */
 OLAP_API int olap_ctx_create(int device, size_t scratch_bytes, olap_ctx** out);
 OLAP_API int olap_ctx_destroy(olap_ctx* ctx);

@@ -32,7 +32,7 @@ __global__ void max_i32_kernel(const int32_t* __restrict__ col, int64_t n, int* 
 
 // True while work on s goes into a graph instead of running (and where that
 // cannot be told because a capture is under way).
-static bool capturing(cudaStream_t s) {
+bool capturing(cudaStream_t s) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
     cudaGetLastError();

@@ -137,6 +137,8 @@ int stage_host_dims(olap_ctx* ctx, const olap_starjoin_query* q, Arena& ar, olap
 // stream is synchronised before a smaller buffer is replaced); null when the
 // allocation fails.  Used by calls whose scratch grows with their rows.
 char* big_scratch(olap_ctx* ctx, size_t bytes);
+// True while work on s is captured into a graph instead of running (ctx.cu).
+bool capturing(cudaStream_t s);
 // In-place scan of pinned host columns (dq: the query with its dimension
 // vectors staged in `ar`); *handled is false (and nothing ran) when a column
 // is not device-mapped, the columns' 16-byte phases differ, or the
